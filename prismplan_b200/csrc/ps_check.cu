@@ -1,5 +1,5 @@
-// ps_check.cu -- batched configuration check (one lane per configuration),
-// sphere FK diagnostics and the FP32 throughput probe.
+// ps_check.cu -- batched configuration check (1, 4 or 16 lanes per
+// configuration), sphere FK diagnostics and the FP32 throughput probe.
 //
 // Replaces check_collision_scene_kernel (code/gpu_planning/cpp/src/planning/
 // pRRTC.cu:2337-2389, one 4-thread block per configuration, 1/8 of a warp
@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "ps_internal.h"
+#include "ps_group.cuh"
 #include "ps_verdict.cuh"
 
 namespace ps {
@@ -37,6 +38,7 @@ __device__ __forceinline__ float sdf_from_min(const SceneSmem& sc, float px, flo
 // this block's configurations (c = block * threads + thread, grid-strided)
 // are reported in collision with a NaN clearance.
 __device__ __forceinline__ void configs_fail_closed(int n, int threads, uint8_t* hit_out, float* clr_out) {
+    if ((int)threadIdx.x >= threads) return;
     for (long long c = (long long)blockIdx.x * threads + threadIdx.x; c < n; c += (long long)gridDim.x * threads) {
         hit_out[c] = 1;
         if (clr_out) clr_out[c] = __int_as_float(0x7fc00000);
@@ -175,10 +177,11 @@ __device__ __noinline__ void sphere_tail(const SceneSmem& sc, const ps_scene_vie
     exact += st.v[ST_EXACT];
 }
 
-// Residency, measured: 6 blocks per SM with clearance (short per-sphere work,
-// latency-bound), 4 without (the early-exit loop wants its registers).
-template <bool kClr, bool kStats>
-__global__ void __launch_bounds__(kCfgThreads, kClr ? 6 : 4) check_configs_fast_kernel(ModelDev md, ps_scene_view sv,
+// Clearance in a scene with ESDF layers (every sphere then needs its lookups,
+// so there is little to cull; without layers configs_group_kernel runs).
+// Residency, measured: 6 blocks per SM (short per-sphere work, latency-bound).
+template <bool kStats>
+__global__ void __launch_bounds__(kCfgThreads, 6) check_configs_fast_kernel(ModelDev md, ps_scene_view sv,
                                                                         const float* __restrict__ q, int n,
                                                                         float margin, unsigned flags,
                                                                         uint8_t* __restrict__ hit_out,
@@ -204,14 +207,12 @@ __global__ void __launch_bounds__(kCfgThreads, kClr ? 6 : 4) check_configs_fast_
     ObbPair* pairs = reinterpret_cast<ObbPair*>(
         reinterpret_cast<unsigned char*>(qtile) + (((size_t)kCfgThreads * D * 4 + 15) & ~size_t(15)));
     const int n_pairs = (sc.n_obbs + 1) / 2;
-    if (kClr) {
-        __syncthreads();   // the staged boxes are visible
-        stage_obb_pairs(sc, pairs);
-        __syncthreads();
-    }
+    __syncthreads();   // the staged boxes are visible
+    stage_obb_pairs(sc, pairs);
+    __syncthreads();
     const bool no_gate = (flags & PS_NO_GATE) != 0;
-    const bool want_obb_clr = kClr && (flags & PS_CLEARANCE_OBB) != 0;
-    const bool want_esdf_clr = kClr && (flags & PS_CLEARANCE_ESDF) != 0;
+    const bool want_obb_clr = (flags & PS_CLEARANCE_OBB) != 0;
+    const bool want_esdf_clr = (flags & PS_CLEARANCE_ESDF) != 0;
     LaneStats st;
     st.zero();
 
@@ -255,11 +256,9 @@ __global__ void __launch_bounds__(kCfgThreads, kClr ? 6 : 4) check_configs_fast_
                 flagged = (sc.n_obbs && sphere_obb_any(sc, nullptr, 0, px, py, pz, sr, nullptr, st)) ||
                           (sc.n_layers && sphere_esdf_any(sc, sv, px, py, pz, sr, nullptr, st));
             }
-            if (!kClr && !(flagged && !hit)) continue;
             // ---- exact spheres: 4 per box load, then singles ----
             int k = jr.sph_beg;
             for (; k + 4 <= jr.sph_end; k += 4) {
-                if (!kClr && hit) break;
                 float px[4], py[4], pz[4], mn[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -268,8 +267,7 @@ __global__ void __launch_bounds__(kCfgThreads, kClr ? 6 : 4) check_configs_fast_
                 }
                 if (kStats) st.v[ST_SPHERES] += 4;
                 if (sc.n_obbs) {
-                    if (kClr) spheres_min_dsq_pairs<4>(pairs, n_pairs, px, py, pz, mn);
-                    else spheres_min_dsq<4>(sc, px, py, pz, mn);
+                    spheres_min_dsq_pairs<4>(pairs, n_pairs, px, py, pz, mn);
                     if (kStats) st.v[ST_PAIRS] += 4 * sc.n_obbs;
                 }
 #pragma unroll
@@ -278,7 +276,6 @@ __global__ void __launch_bounds__(kCfgThreads, kClr ? 6 : 4) check_configs_fast_
                                 want_esdf_clr, flagged, hit, clr, st.v[ST_EXACT]);
             }
             for (; k < jr.sph_end; ++k) {
-                if (!kClr && hit) break;
                 const float4 sp = M.S[k];
                 float px, py, pz;
                 sphere_world(T, sp.x, sp.y, sp.z, px, py, pz);
@@ -291,10 +288,67 @@ __global__ void __launch_bounds__(kCfgThreads, kClr ? 6 : 4) check_configs_fast_
                 }
                 sphere_tail(sc, sv, px, py, pz, sr, mn, want_obb_clr, want_esdf_clr, flagged, hit, clr, st.v[ST_EXACT]);
             }
-            if (!kClr && hit) break;
         }
         hit_out[c] = hit ? 1 : 0;
         if (clr_out) clr_out[c] = clr;
+    }
+    if (kStats) flush_stats(stats, st);
+}
+
+// The common configurations: see ps_group.cuh. A warp takes 32 / kSub
+// consecutive configurations at a time.
+template <int kSub, bool kClr, bool kEsdf, bool kStats>
+__global__ void __launch_bounds__(kCfgThreads, 5) configs_group_kernel(ModelDev md, ps_scene_view sv,
+                                                                       const float* __restrict__ q, int n,
+                                                                       float margin, unsigned flags,
+                                                                       uint8_t* __restrict__ hit_out,
+                                                                       float* __restrict__ clr_out,
+                                                                       unsigned long long* stats) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    ObbPrep* obbs = reinterpret_cast<ObbPrep*>(smem + md.bytes_core);
+    const int nob = max(sv.n_obbs, 1);
+    int* orig = reinterpret_cast<int*>(obbs + nob);
+    LayerPrep* layers = reinterpret_cast<LayerPrep*>(orig + ((nob + 3) & ~3));
+    float4* obs = reinterpret_cast<float4*>(layers + PS_MAX_LAYERS);
+    constexpr int kPer = 32 / kSub;                       // configurations per warp
+    constexpr int kTile = kCfgThreads / kSub;             // per block
+    if (!stage_model(md, smem, &mbar)) return configs_fail_closed(n, kTile, hit_out, clr_out);
+    SceneSmem sc;
+    stage_scene(sv, obbs, orig, layers, counters, &bmax, sc);
+    box_spheres(sc, obs);
+    __syncthreads();
+    box_limits(sc, obs);
+    __syncthreads();
+    const ModelSmem M = model_view(smem);
+    const int D = M.H->n_dof;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* wq = reinterpret_cast<float*>(obs + nob) + warp * kPer * D;
+    LaneStats st;
+    st.zero();
+    for (int base = (blockIdx.x * (kCfgThreads / 32) + warp) * kPer; base < n; base += gridDim.x * kTile) {
+        const int cnt = min(kPer, n - base);
+        __syncwarp();
+        for (int k = lane; k < cnt * D; k += 32) wq[k] = q[(size_t)base * D + k];
+        __syncwarp();
+        const int slot = lane / kSub;
+        const bool live = slot < cnt;   // a group past the end repeats the last configuration
+        bool hit;
+        float clr;
+        LaneStats ls;
+        ls.zero();
+        group_verdict<kSub, kClr, kEsdf, kStats>(M, sc, sv, obs, wq + min(slot, cnt - 1) * D, margin,
+                                                 (flags & PS_NO_GATE) != 0, hit, clr, ls);
+        if (live && (lane & (kSub - 1)) == 0) {
+            hit_out[base + slot] = hit ? 1 : 0;
+            if (clr_out) clr_out[base + slot] = clr;
+        }
+        if (kStats && live) {
+            if ((lane & (kSub - 1)) == 0) st.v[ST_SAMPLES] += 1;
+            for (int k = 0; k < ST_COUNT; ++k) st.v[k] += ls.v[k];
+        }
     }
     if (kStats) flush_stats(stats, st);
 }
@@ -427,6 +481,41 @@ extern "C" int ps_set_timing_events(void* start, void* stop) {
     return PS_OK;
 }
 
+namespace {
+
+using ConfigKernel = void (*)(ModelDev, ps_scene_view, const float*, int, float, unsigned, uint8_t*, float*,
+                              unsigned long long*);
+
+template <bool kClr, bool kEsdf, bool kStats>
+ConfigKernel pick_lanes(int sub) {
+    return sub == 1 ? configs_group_kernel<1, kClr, kEsdf, kStats>
+                    : (sub == 4 ? configs_group_kernel<4, kClr, kEsdf, kStats>
+                                : configs_group_kernel<16, kClr, kEsdf, kStats>);
+}
+
+ConfigKernel pick_group(int sub, bool clr, bool esdf, bool stats) {
+    if (clr) return stats ? pick_lanes<true, false, true>(sub) : pick_lanes<true, false, false>(sub);
+    if (esdf) return stats ? pick_lanes<false, true, true>(sub) : pick_lanes<false, true, false>(sub);
+    return stats ? pick_lanes<false, false, true>(sub) : pick_lanes<false, false, false>(sub);
+}
+
+// Lanes per configuration. Few configurations leave the chip idle one lane
+// each, and a configuration's chain of joints is serial, so its boxes and
+// spheres are split over 16 lanes while that makes at most 16 warps per SM,
+// over 4 while that makes at most 28; beyond, the split's repeated kinematics
+// cost more than the latency it hides. Measured (us, 1 / 4 / 16 lanes; 7
+// joints, 59 spheres, 16 boxes with clearance): 1024 configurations 35.2 /
+// 17.9 / 12.3, 4096 38.0 / 18.0 / 15.7, 8192 37.8 / 19.6 / 28.2, 32,768 41.1 /
+// 40.5 / 83.9, 131,072 92.7 / 132 / 302; the verdict on 14 joints, 128 boxes
+// and an ESDF crosses at the same counts.
+int config_lanes(int n) {
+    const long long per_warp = 32ll * sm_count();
+    if ((long long)n * 16 <= 16 * per_warp) return 16;
+    return (long long)n * 4 <= 28 * per_warp ? 4 : 1;
+}
+
+}  // namespace
+
 extern "C" int ps_check_configs(const ps_model* m, const ps_scene_view* scene, const float* q, int n,
                                 float margin, unsigned flags, uint8_t* hit, float* clearance, void* stream) {
     PS_NVTX("ps_check_configs");
@@ -438,19 +527,30 @@ extern "C" int ps_check_configs(const ps_model* m, const ps_scene_view* scene, c
     if (int rc = validate_scene(m, scene)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     // Without a clearance source the output (if any) is the 1000 sentinel.
-    const bool clr = clearance != nullptr && (flags & (PS_CLEARANCE_OBB | PS_CLEARANCE_ESDF));
-    size_t smem = (size_t)m->dev.bytes_core + scene_smem_bytes(scene) + (size_t)kCfgThreads * m->info.n_dof * 4;
-    smem = ((smem + 15) & ~size_t(15)) + (size_t)((scene->n_obbs + 1) / 2) * sizeof(ObbPair);   // box pairs
-    const int blocks_needed = (n + kCfgThreads - 1) / kCfgThreads;
-    const int per_sm = (flags >> 8) & 15u ? (int)((flags >> 8) & 15u) : 8;   // PS_CONFIG_BLOCKS_PER_SM
-    const int grid = std::max(1, std::min(blocks_needed, sm_count() * per_sm));
-    // (sphere_obb_acm_mask_approx changes no result: see the approximate gate)
+    const bool clr = clearance != nullptr &&
+                     ((flags & PS_CLEARANCE_OBB) || ((flags & PS_CLEARANCE_ESDF) && scene->n_voxel_layers > 0));
     const bool fast = m->root_slot_only && m->info.approx_shares_chain && !scene->sphere_obb_acm_mask &&
                       !scene->sphere_acm_mask;
-    auto k = fast ? (clr ? (g_stats ? check_configs_fast_kernel<true, true> : check_configs_fast_kernel<true, false>)
-                         : (g_stats ? check_configs_fast_kernel<false, true> : check_configs_fast_kernel<false, false>))
-                  : (clr ? (g_stats ? check_configs_kernel<true, true> : check_configs_kernel<true, false>)
-                         : (g_stats ? check_configs_kernel<false, true> : check_configs_kernel<false, false>));
+    void (*k)(ModelDev, ps_scene_view, const float*, int, float, unsigned, uint8_t*, float*, unsigned long long*);
+    const size_t tables = (size_t)m->dev.bytes_core + scene_smem_bytes(scene);
+    size_t smem;
+    int tile = kCfgThreads, per_sm = 8;
+    // (sphere_obb_acm_mask_approx changes no result: the approximate gate applies no mask)
+    if (fast && !(clr && scene->n_voxel_layers > 0)) {
+        const int sub = config_lanes(n);
+        k = pick_group(sub, clr, scene->n_voxel_layers > 0, g_stats != nullptr);
+        tile = kCfgThreads / sub;
+        smem = tables + (size_t)16 * std::max(scene->n_obbs, 1) + (size_t)tile * m->info.n_dof * 4;
+    } else {
+        smem = tables + (size_t)kCfgThreads * m->info.n_dof * 4;
+        smem = ((smem + 15) & ~size_t(15)) + (size_t)((scene->n_obbs + 1) / 2) * sizeof(ObbPair);   // box pairs
+        if (fast) k = g_stats ? check_configs_fast_kernel<true> : check_configs_fast_kernel<false>;
+        else k = clr ? (g_stats ? check_configs_kernel<true, true> : check_configs_kernel<true, false>)
+                     : (g_stats ? check_configs_kernel<false, true> : check_configs_kernel<false, false>);
+    }
+    if ((flags >> 8) & 15u) per_sm = (int)((flags >> 8) & 15u);   // PS_CONFIG_BLOCKS_PER_SM
+    const int blocks_needed = (n + tile - 1) / tile;
+    const int grid = std::max(1, std::min(blocks_needed, sm_count() * per_sm));
     PS_TRY_CUDA(allow_smem((const void*)k, smem));
     mark_start(s);
     k<<<grid, kCfgThreads, smem, s>>>(m->dev, *scene, q, n, margin, flags, hit, clearance, g_stats);

@@ -44,8 +44,15 @@ struct JointRec {
     float4 bound;            // link-frame point + radius enclosing every exact and
                              // approximate sphere of the joint (w < 0: none)
     int parent_pos;          // DFS position of the parent joint (root: 0)
-    int pad[3];
+    // World-frame bounds of the joint's spheres about its bound centre, for
+    // any model the library accepts (a fixed transform may stretch, a radius
+    // may be negative): reach >= |p_s - c| + |r_s| for every exact and
+    // approximate sphere s (< 0: none); for one exact sphere, near_d >=
+    // |p_s - c| and near_r = near_d - r_s, the least such value (PS_NO_NEAR: no
+    // exact sphere).
+    float reach, near_r, near_d;
 };
+#define PS_NO_NEAR 1.0e30f
 
 // Self pairs (global memory): packed (i | j << 16), reordered sphere indices.
 // The same pairs as runs: sruns[r] = (i | q << 9 | len << 14, j0) is sphere i

@@ -364,6 +364,10 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     int max_js = 0, max_ja = 0;
     auto fill_joints = [&](size_t at, const float* ftab, const int* ttab) {
         JointRec* J = reinterpret_cast<JointRec*>(host.data() + at);
+        // stretch[p]: bound on the spectral norm of joint p's world rotation
+        // part, the product of its ancestors' sqrt(|A^T A|_inf) (1 for rigid
+        // transforms up to the description's rounding)
+        std::vector<double> stretch(nj, 1.0);
         for (int p = 0; p < nj; ++p) {
             int i = dfs[p];
             for (int k = 0; k < 12; ++k) J[p].ft[k] = ftab[16 * i + k];
@@ -399,6 +403,39 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
             for (int k = sbeg[p]; k < send[p]; ++k) grow(d->spheres + 4 * sorder[k]);
             for (int k = abeg[p]; k < aend[p]; ++k) grow(d->approx_spheres + 4 * aorder[k]);
             J[p].bound = make_float4((float)cx, (float)cy, (float)cz, R < 0 ? -1.0f : (float)(R * (1.0 + 1e-6) + 1e-6));
+            if (p > 0) {
+                double norm = 0.0;
+                for (int a = 0; a < 3; ++a) {
+                    double row = 0.0;
+                    for (int b = 0; b < 3; ++b) {
+                        double v = 0.0;
+                        for (int r = 0; r < 3; ++r) v += (double)ftab[16 * i + 4 * r + a] * ftab[16 * i + 4 * r + b];
+                        row += std::fabs(v);
+                    }
+                    norm = std::max(norm, row);
+                }
+                stretch[p] = stretch[pos[parents[i]]] * std::sqrt(std::max(norm, 1.0)) * (1.0 + 4e-6);
+            }
+            double reach = -1.0, near_d = 0.0, near_r = PS_NO_NEAR;
+            auto far = [&](const float* s) {
+                const double dx = s[0] - cx, dy = s[1] - cy, dz = s[2] - cz;
+                const double dist = std::sqrt(dx * dx + dy * dy + dz * dz) * stretch[p] * (1.0 + 1e-5) + 1e-6;
+                const double r = dist + std::fabs((double)s[3]);
+                reach = std::max(reach, r < 1.0e30 ? r : 1.0e30);   // not finite: never culled
+                return dist;
+            };
+            for (int k = sbeg[p]; k < send[p]; ++k) {
+                const float* s = d->spheres + 4 * sorder[k];
+                const double dist = far(s);
+                if (dist - s[3] < near_r) {
+                    near_d = dist;
+                    near_r = dist - s[3];
+                }
+            }
+            for (int k = abeg[p]; k < aend[p]; ++k) far(d->approx_spheres + 4 * aorder[k]);
+            J[p].reach = (float)(reach * (1.0 + 1e-6));
+            J[p].near_r = (float)(near_r + std::fabs(near_r) * 1e-6);
+            J[p].near_d = (float)(near_d * (1.0 + 1e-6));
         }
     };
     fill_joints(h.off_joints, d->fixed_transforms, d->joint_types);
