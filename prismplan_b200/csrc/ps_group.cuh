@@ -216,9 +216,10 @@ __device__ __forceinline__ void group_verdict(const ModelSmem& M, const SceneSme
                 Rc2 = Rcl * Rcl;
             }
         };
-        if (kClr && slack > 2.0f) {
-            // no clearance known yet: the nearest box centre bounds it, so that
-            // the first joint does not take every box
+        if (kClr && (kSub > 1 ? __any_sync(kGrpFull, slack > 2.0f) : slack > 2.0f)) {
+            // no clearance known yet (on some group of the warp: the minimum
+            // below is warp-wide): the nearest box centre bounds it, so that the
+            // first joint does not take every box
             float dc = 3.0e38f;
             for (int o = u; o < sc.n_obbs; o += kSub) {
                 const float4 ob = obs[o];

@@ -63,3 +63,23 @@ def test_group_equals_generic(golden, n, robot, boxes, esdf):
             assert torch.equal(a[0], g[0])
             if clearance:
                 assert torch.equal(a[1].view(torch.int32), g[1].view(torch.int32))
+
+
+@pytest.mark.parametrize("n", [9, 1000, 4737])
+def test_clearances_on_both_sides_of_the_first_bound(golden, n):
+    """One box some 2 m from the arm: a warp's configurations disagree on
+    whether their clearance is known to be below the level at which the first
+    joints stop bounding it by the box centres (2 m)."""
+    import torch
+
+    from prismplan_b200 import api
+    from prismplan_b200.scene import SceneTensors, pack_obbs
+
+    b, asset = _robot("panda", golden)
+    d, p, e = pack_obbs(np.array([[0.2, 0.2, 0.2]]), np.array([[2.4, 0.0, 0.4]]), np.array([[1.0, 0.0, 0.0, 0.0]]))
+    ones = np.ones((len(b.sphere_to_joint), 1), np.uint8)
+    q = torch.from_numpy(workloads.uniform_configs(np.random.default_rng(n), asset, n)).cuda()
+    a = api.check_configs(b, SceneTensors(d, p, e), q, 0.0, "obb")
+    g = api.check_configs(b, SceneTensors(d, p, e, sphere_obb_acm_mask=ones), q, 0.0, "obb")
+    assert n < 100 or (float(g[1].min()) < 2.0 < float(g[1].max()))
+    assert torch.equal(a[0], g[0]) and torch.equal(a[1].view(torch.int32), g[1].view(torch.int32))
