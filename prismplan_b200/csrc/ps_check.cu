@@ -499,21 +499,6 @@ ConfigKernel pick_group(int sub, bool clr, bool esdf, bool stats) {
     return stats ? pick_lanes<false, false, true>(sub) : pick_lanes<false, false, false>(sub);
 }
 
-// Lanes per configuration. Few configurations leave the chip idle one lane
-// each, and a configuration's chain of joints is serial, so its boxes and
-// spheres are split over 16 lanes while that makes at most 16 warps per SM,
-// over 4 while that makes at most 28; beyond, the split's repeated kinematics
-// cost more than the latency it hides. Measured (us, 1 / 4 / 16 lanes; 7
-// joints, 59 spheres, 16 boxes with clearance): 1024 configurations 35.2 /
-// 17.9 / 12.3, 4096 38.0 / 18.0 / 15.7, 8192 37.8 / 19.6 / 28.2, 32,768 41.1 /
-// 40.5 / 83.9, 131,072 92.7 / 132 / 302; the verdict on 14 joints, 128 boxes
-// and an ESDF crosses at the same counts.
-int config_lanes(int n) {
-    const long long per_warp = 32ll * sm_count();
-    if ((long long)n * 16 <= 16 * per_warp) return 16;
-    return (long long)n * 4 <= 28 * per_warp ? 4 : 1;
-}
-
 }  // namespace
 
 extern "C" int ps_check_configs(const ps_model* m, const ps_scene_view* scene, const float* q, int n,

@@ -36,7 +36,7 @@ struct BlobHeader {          // 64 bytes
     int off_apx, off_apx_orig, bytes_core, bytes_total;
 };
 
-// One joint in DFS visit order (112 bytes).
+// One joint in DFS visit order (128 bytes).
 struct JointRec {
     float ft[12];            // rows 0..2 of the fixed transform, row-major
     int type, dof, parent_slot, slot;
@@ -51,6 +51,9 @@ struct JointRec {
     // |p_s - c| and near_r = near_d - r_s, the least such value (PS_NO_NEAR: no
     // exact sphere).
     float reach, near_r, near_d;
+    float link;              // length of the fixed transform's translation
+    float cen;               // |bound centre| in the joint's frame
+    int pad[2];
 };
 #define PS_NO_NEAR 1.0e30f
 

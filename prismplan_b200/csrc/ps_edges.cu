@@ -125,17 +125,22 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
     int* lst = split ? b.lst : nullptr;
     ProbePlan probe;
     if (int rc = plan_probe(m, scene, mode, g_stats != nullptr, 1.0f, n_edges, P->probe, probe)) return rc;
+    const bool coarse = coarse_path(m, P, mode, probe.kp != nullptr, n_edges, qgrid);
+    if (coarse) {
+        qk = g_stats ? edges_queue_kernel<3, true> : edges_queue_kernel<3, false>;   // same shared memory and residency
+        PS_TRY_CUDA(allow_smem((const void*)qk, smem));
+    }
     if (!probe.kp) {   // with the probe, its launch also prepares the edges
         const int pgrid = std::max(1, std::min((n_edges + 255) / 256, sm_count() * 4));
         edges_prep_kernel<<<pgrid, 256, 0, s>>>(*P, from, to, samples_per_edge, n_edges, D, b.hdr, b.G, b.len, b.bad,
-                                                b.clr, b.done, nullptr, lst);
+                                                b.clr, b.done, nullptr, lst, coarse);
         PS_TRY_CUDA(cudaGetLastError());
     }
     mark_start(s);
     if (probe.kp)
         probe.kp<<<probe.grid, kProbeThreads, probe.smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G,
                                                                 b.bad, g_stats, nullptr,
-                                                                PrepArgs{samples_per_edge, b.len, b.clr, b.done, lst});
+                                                                PrepArgs{samples_per_edge, b.len, b.clr, b.done, lst, coarse});
     qk<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
                                          g_stats, 0, nullptr, lst);
     if (split)
@@ -148,7 +153,7 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
         return rc;
     const int fgrid = std::max(1, std::min((n_edges + 255) / 256, sm_count() * 4));
     edges_finalize_kernel<<<fgrid, 256, 0, s>>>(n_edges, *P, b.bad, b.len, b.clr, b.done, b.G, b.hdr, valid, cost,
-                                                clearance);
+                                                clearance, nullptr, coarse);
     PS_TRY_CUDA(cudaGetLastError());
     return PS_OK;
 }

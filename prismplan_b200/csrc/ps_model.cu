@@ -433,6 +433,9 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
                 }
             }
             for (int k = abeg[p]; k < aend[p]; ++k) far(d->approx_spheres + 4 * aorder[k]);
+            const float* f = ftab + 16 * i;
+            J[p].link = (float)(std::sqrt((double)f[3] * f[3] + (double)f[7] * f[7] + (double)f[11] * f[11]) * (1.0 + 1e-6));
+            J[p].cen = (float)(std::sqrt(cx * cx + cy * cy + cz * cz) * (1.0 + 1e-6));
             J[p].reach = (float)(reach * (1.0 + 1e-6));
             J[p].near_r = (float)(near_r + std::fabs(near_r) * 1e-6);
             J[p].near_d = (float)(near_d * (1.0 + 1e-6));
@@ -492,6 +495,19 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     m->root_slot_only = tmem[dfs[0]] == 0;
     for (int p = 1; p < nj; ++p) m->root_slot_only = m->root_slot_only && tmem[dfs[p]] == 1;
     m->max_joint_approx = max_ja;
+    m->min_radius = ns + na > 0 ? 3.0e38f : 0.0f;
+    for (int s = 0; s < ns; ++s) m->min_radius = std::min(m->min_radius, d->spheres[4 * s + 3]);
+    for (int a = 0; a < na; ++a) m->min_radius = std::min(m->min_radius, d->approx_spheres[4 * a + 3]);
+    m->rigid = true;
+    for (int p = 1; p < nj; ++p) {
+        const float* f = d->fixed_transforms + 16 * dfs[p];
+        for (int a = 0; a < 3; ++a)
+            for (int b = 0; b < 3; ++b) {
+                double v = a == b ? -1.0 : 0.0;
+                for (int r = 0; r < 3; ++r) v += (double)f[4 * r + a] * f[4 * r + b];
+                m->rigid = m->rigid && std::fabs(v) <= 2e-5;
+            }
+    }
     m->sph_orig = sorder;
     int dev = 0;
     cudaGetDevice(&dev);
