@@ -76,6 +76,11 @@ struct ModelDev {
                                    // chain, whose centre is the joint's bound centre (the self check reads it there)
     const float* lower;            // device
     const float* upper;            // device
+    const float* lever;            // device [n_joints][n_joints], DFS positions: how far a point of joint j's spheres
+                                   // lies at most from joint k's origin, k an ancestor of j or j itself (1 for a
+                                   // sliding joint k: its motion is the same everywhere), sliding joints between
+                                   // them out by at most slide_max
+    float slide_max;
     int* status;                   // device error latch
     int bytes_core;
     int stage_polls;               // polls of the staging wait before a kernel gives up

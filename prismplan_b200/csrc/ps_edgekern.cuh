@@ -8,6 +8,7 @@
 
 #include "ps_internal.h"
 #include "ps_group.cuh"
+#include "ps_pathkern.cuh"
 #include "ps_verdict.cuh"
 
 namespace ps {
@@ -70,33 +71,6 @@ __device__ __forceinline__ int ordered_float(float f) {
     return i >= 0 ? i : (i ^ 0x7fffffff);
 }
 __device__ __forceinline__ float unordered_float(int i) { return __int_as_float(i >= 0 ? i : (i ^ 0x7fffffff)); }
-
-// Sample count of an edge (edge_eval.cuh:54-60 plus the L-inf rule).
-__device__ __forceinline__ int edge_samples(const ps_edge_params& P, const int* given, int e, const float* a,
-                                            const float* b, int D, float len) {
-    if (given) return given[e];
-    if (P.resolution > 0.0f) {
-        int g = (int)ceilf(__fdiv_rn(len, P.resolution));
-        return min(max(g, 2), 1024);
-    }
-    if (P.max_joint_step > 0.0f) {
-        float m = 0.0f;
-        for (int i = 0; i < D; ++i) m = fmaxf(m, fabsf(__fadd_rn(b[i], -a[i])));
-        int g = (int)ceilf(__fdiv_rn(m, P.max_joint_step));
-        const int cap = P.max_samples > 0 ? P.max_samples : 1024;
-        return min(max(g, 1), cap);
-    }
-    return P.granularity;
-}
-
-__device__ __forceinline__ float edge_length(const float* a, const float* b, int D) {
-    float len2 = 0.0f;   // edge_eval.cuh:104-106
-    for (int i = 0; i < D; ++i) {
-        float d = __fadd_rn(b[i], -a[i]);
-        len2 = __fmaf_rn(d, d, len2);
-    }
-    return sqrtf(len2);
-}
 
 struct WarpScratch {
     float* q;          // [32 * D]

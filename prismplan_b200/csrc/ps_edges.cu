@@ -99,6 +99,22 @@ EdgeBufs carve_workspace(void* ws, int n_edges) {
     return b;
 }
 
+// Whether a batch runs one block per edge (edges_path_kernel): small ones,
+// where the queue path waits on its launches and on single warps. Measured
+// (us, queue path / block per edge; 59-sphere arm, 64 small boxes, 0.02 rad
+// steps), with the self check 27 edges 164 / 95, 1009 223 / 163, 2048 247 /
+// 241, 4096 313 / 388; without 27 109 / 39, 1009 134 / 73, but among 64 large
+// boxes at 0.01 rad 512 69 / 68 and 1009 77 / 87; 16 samples an edge among 16
+// boxes with the self check 27 85 / 27, 2048 117 / 83, 4096 131 / 140. With an ESDF layer in reach few
+// intervals are shown clear: 27 edges 237 / 184, 512 471 / 896.
+bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, const int* given, int mode,
+                int n_edges) {
+    if (mode == 0 || !m->rigid || g_stats || P->time_budget_ms > 0.0f) return false;   // (the counters live in the queue path)
+    const bool few = !given && P->resolution <= 0.0f && P->max_joint_step <= 0.0f && P->granularity <= 32;
+    const int most = mode == 2 ? 64 : (P->check_self || few ? 2048 : 512);
+    return n_edges <= most && path_serves(m, scene, P->collision_margin, P->check_self != 0);
+}
+
 // memset header -> prep -> end-sample probe -> queue pass(es) -> self pass ->
 // finalize on stream s.
 int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* from, const float* to,
@@ -106,8 +122,20 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
                    float* clearance, const EdgeBufs& b, cudaStream_t s) {
     const int D = m->info.n_dof;
     PS_TRY_CUDA(cudaMemsetAsync(b.hdr, 0, sizeof(EdgeWs), s));   // queue heads, deadline, max rounds, timeout
-    const size_t smem = edge_smem_bytes(m, scene);
     const int mode = fast_path(m, scene, P);
+    if (path_edges(m, scene, P, samples_per_edge, mode, n_edges)) {
+        auto pk = mode == 2 ? edges_path_kernel<true> : edges_path_kernel<false>;
+        const size_t psmem = path_smem_bytes(m, scene, P->check_self != 0);
+        PS_TRY_CUDA(allow_smem((const void*)pk, psmem));
+        mark_start(s);
+        pk<<<std::min(n_edges, sm_count() * 16), kPathThreads, psmem, s>>>(m->dev, *scene, *P, from, to, samples_per_edge,
+                                                                          n_edges, valid, cost, clearance,
+                                                                          &b.hdr->timed_out);
+        mark_stop(s);
+        PS_TRY_CUDA(cudaGetLastError());
+        return PS_OK;
+    }
+    const size_t smem = edge_smem_bytes(m, scene);
     auto qk = pick(mode, g_stats != nullptr, edges_queue_kernel<0, false>, edges_queue_kernel<0, true>,
                    edges_queue_kernel<1, false>, edges_queue_kernel<1, true>, edges_queue_kernel<2, false>,
                    edges_queue_kernel<2, true>);

@@ -343,6 +343,8 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     off += align16(sizeof(float) * nd);
     const size_t off_upper = off;
     off += align16(sizeof(float) * nd);
+    const size_t off_lever = off;
+    off += align16(sizeof(float) * nj * nj);
     const size_t off_status = off;
     off += 16;
     const size_t total = align16(off);
@@ -464,6 +466,33 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     std::memcpy(host.data() + off_lower, d->joint_lower, sizeof(float) * nd);
     std::memcpy(host.data() + off_upper, d->joint_upper, sizeof(float) * nd);
 
+    // levers (ModelDev::lever), for rigid transforms
+    float slide_max = 1.0f;
+    {
+        auto dist = [](const float* v) {
+            return std::sqrt((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]);
+        };
+        for (int p = 1; p < nj; ++p) {
+            const int i = dfs[p];
+            if (d->joint_types[i] < PS_X_PRISM || d->joint_types[i] >= PS_X_ROT) continue;
+            slide_max = std::max(slide_max, std::max(std::fabs(d->joint_lower[id2dof[i]]), std::fabs(d->joint_upper[id2dof[i]])));
+        }
+        float* L = reinterpret_cast<float*>(host.data() + off_lever);
+        for (int p = 0; p < nj; ++p) {
+            double far = 0.0;   // from joint p's origin to its spheres
+            for (int k = sbeg[p]; k < send[p]; ++k) far = std::max(far, dist(d->spheres + 4 * sorder[k]));
+            for (int k = abeg[p]; k < aend[p]; ++k) far = std::max(far, dist(d->approx_spheres + 4 * aorder[k]));
+            for (int k = p; k > 0; k = pos[parents[dfs[k]]]) {
+                const int i = dfs[k];
+                const bool slides = d->joint_types[i] >= PS_X_PRISM && d->joint_types[i] < PS_X_ROT;
+                L[k * nj + p] = slides ? 1.0f : (float)(far * (1.0 + 1e-5) + 1e-6);
+                const float* f = d->fixed_transforms + 16 * i;
+                const float t[3] = {f[3], f[7], f[11]};
+                far += dist(t) + (slides ? slide_max : 0.0);   // from the parent's origin
+            }
+        }
+    }
+
     ps_model* m = new ps_model();
     cudaError_t e = cudaMalloc(&m->alloc, total);
     if (e != cudaSuccess) {
@@ -488,6 +517,8 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     m->dev.bound_from_apx = bound_from_apx ? 1 : 0;
     m->dev.lower = reinterpret_cast<const float*>(base + off_lower);
     m->dev.upper = reinterpret_cast<const float*>(base + off_upper);
+    m->dev.lever = reinterpret_cast<const float*>(base + off_lever);
+    m->dev.slide_max = slide_max;
     m->dev.status = reinterpret_cast<int*>(base + off_status);
     m->dev.bytes_core = (int)core;
     m->dev.stage_polls = PS_STAGE_POLLS;

@@ -1,0 +1,503 @@
+// ps_pathkern.cuh -- one block checks a short path: every sample of an edge
+// (small edge batches, ps_edges.cu) or the waypoints and densified segments of
+// a slice of a trajectory (the optimisers, ps_optloop.cuh), scene and self
+// collision, in one launch.
+//
+// A small batch is bound by latency and launches: the queue path runs one warp
+// per 32 samples through serial candidate loops, once for the scene and once
+// more, one thread per sample, for the self check, with a preparation, a
+// second queue pass and a finalize around them. Here a block of 32 groups of 4
+// lanes holds one path.
+//   1. Swept check: the path is cut into at most 32 intervals, one per group.
+//      From one kinematic pass at an interval's middle, with bounds on how far
+//      links move inside it, an interval is shown clear of every box (and out
+//      of reach of every ESDF layer) and of self collision, or not. Skipped
+//      when the samples themselves fit the groups.
+//   2. The samples of the other intervals are checked one by one, a group
+//      each (group_verdict, group_self_hit), until one hits.
+// The verdict is the OR over the samples' verdicts, and step 1 only leaves out
+// samples that cannot hit, so the result is the queue path's.
+#pragma once
+
+#include <cfloat>
+
+#include "ps_group.cuh"
+#include "ps_internal.h"
+#include "ps_verdict.cuh"
+
+namespace ps {
+namespace {
+
+constexpr int kPathThreads = 128;
+constexpr int kPathSub = kSelfSub;                       // lanes per group
+constexpr int kPathGroups = kPathThreads / kPathSub;     // intervals (or samples) at a time
+constexpr float kSweepMaxQ = 16.0f;                      // largest joint value that the swept check judges
+
+__device__ __forceinline__ float len_up(float x, float y, float z) {   // |(x, y, z)|, never below it
+    const float d2 = fmaxf(fmaf(z, z, fmaf(y, y, x * x)), 1.0e-30f);
+    return d2 * rsqrtf(d2) * (1.0f + 1.0e-6f);
+}
+
+// What a block of these kernels holds in shared memory.
+struct PathSmem {
+    ObbPrep* obbs;
+    int* orig;
+    LayerPrep* layers;
+    float4* obs;
+    float* q;        // [groups][2 D]: a group's configuration, and an interval's half width
+    SelfSmem self;   // positions of the groups' configurations
+};
+
+__host__ __device__ inline size_t path_tables(int n_obbs) {   // boxes, their indices, layers, spheres
+    const size_t n = n_obbs > 1 ? n_obbs : 1;
+    return n * sizeof(ObbPrep) + ((n + 3) & ~size_t(3)) * 4 + sizeof(LayerPrep) * PS_MAX_LAYERS + n * 16;
+}
+
+inline size_t path_smem_bytes(const ps_model* m, const ps_scene_view* sv, bool self) {
+    const int nc = m->dev.bound_from_apx ? 0 : m->info.n_joints;
+    return (size_t)m->dev.bytes_core + path_tables(sv->n_obbs) + (size_t)kPathGroups * 2 * m->info.n_dof * 4 +
+           (self ? (size_t)(m->info.n_spheres + m->info.n_approx_spheres + nc) * 3 * kPathGroups * 4 : 0) + 64;
+}
+
+// Models and calls these kernels serve; the rest takes the queue path. (A
+// negative effective radius would be decided by the guard band's lower edge,
+// which the two paths take from different bounds.)
+inline bool path_serves(const ps_model* m, const ps_scene_view* sv, float margin, bool self) {
+    return m->root_slot_only && m->info.approx_shares_chain && !sv->sphere_obb_acm_mask && !sv->sphere_acm_mask &&
+           m->min_radius + margin >= 0.0f && path_smem_bytes(m, sv, self) <= smem_optin() / 2;
+}
+
+__device__ __forceinline__ PathSmem path_carve(unsigned char* smem, const ModelDev& md, const ps_scene_view& sv) {
+    const BlobHeader* H = reinterpret_cast<const BlobHeader*>(md.blob);
+    const int nob = max(sv.n_obbs, 1);
+    PathSmem s;
+    s.obbs = reinterpret_cast<ObbPrep*>(smem + md.bytes_core);
+    s.orig = reinterpret_cast<int*>(s.obbs + nob);
+    s.layers = reinterpret_cast<LayerPrep*>(s.orig + ((nob + 3) & ~3));
+    s.obs = reinterpret_cast<float4*>(s.layers + PS_MAX_LAYERS);
+    s.q = reinterpret_cast<float*>(s.obs + nob);
+    s.self = carve_self<kPathGroups>(reinterpret_cast<unsigned char*>(s.q + kPathGroups * 2 * H->n_dof), H->n_spheres,
+                                     H->n_approx, H->n_joints, md.bound_from_apx != 0);
+    return s;
+}
+
+// Swept check of the group's segment qm + s d, s in [-1, 1]: bit 0 set when a
+// sphere may meet a box (or a layer's voxel box) somewhere on it, bit 1 when a
+// self pair may overlap (with kSelf). Zero means that no sample of the segment
+// can hit.
+//
+// One kinematic pass at the midpoint carries each joint frame's angular
+// velocity w and origin velocity v per unit s, and bounds W >= |w|, A >= |w'|
+// and Ao >= |v'| that hold on the whole segment, so a point at distance r from
+// the joint's origin moves at most |v + w x r| + (Ao + |r| (W^2 + A)) / 2. A
+// joint whose reach, widened by its centre's motion, meets no box is clear;
+// otherwise its spheres, each widened by its own motion, are tested against
+// the boxes met. The distance of two links changes only with the joints
+// between them, by at most sum |d_k| lever(k, link) (ModelDev::lever). The
+// guard band covers the rounding of the kinematics on either side (__sinf /
+// __cosf included, for |q| <= kSweepMaxQ).
+//
+// Every lane of the warp calls it (ok: the group's segment may be judged);
+// the result is the same on all lanes of a group.
+template <bool kEsdf>
+__device__ __forceinline__ unsigned path_sweep(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
+                                               const float4* __restrict__ obs, const float* qm, const float* dq,
+                                               float margin, bool ok, bool self, const SelfSmem& sm, int slot) {
+    constexpr int kSub = kPathSub;
+    const int u = (threadIdx.x & 31) & (kSub - 1);
+    const int NJ = M.H->n_joints;
+    const float am = fabsf(margin), G4 = 4.0f * PS_GUARD_K;
+    Affine T;
+    affine_identity(T);
+    float wx = 0.f, wy = 0.f, wz = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, W = 0.f, A = 0.f, Ao = 0.f;
+    bool clear = ok;
+    for (int p = 0; p < NJ; ++p) {
+        const JointRec& jr = M.J[p];
+        if (p > 0) {
+            const float qi = jr.dof >= 0 ? qm[jr.dof] : 0.0f;
+            const float di = jr.dof >= 0 && jr.type != PS_FIXED ? dq[jr.dof] : 0.0f;
+            float ox, oy, oz;   // the parent's origin
+            if (jr.parent_slot == 0) {
+                Affine I;
+                affine_identity(I);
+                joint_compose<true>(jr, qi, I, T);
+                ox = oy = oz = wx = wy = wz = vx = vy = vz = W = A = Ao = 0.0f;
+            } else {
+                ox = T.m[3], oy = T.m[7], oz = T.m[11];
+                joint_compose<true>(jr, qi, T, T);
+            }
+            const float ex = T.m[3] - ox, ey = T.m[7] - oy, ez = T.m[11] - oz;
+            vx += wy * ez - wz * ey;
+            vy += wz * ex - wx * ez;
+            vz += wx * ey - wy * ex;
+            const float ad = fabsf(di), el = len_up(ex, ey, ez) + ad;   // a sliding joint's offset grows by ad at most
+            Ao += el * fmaf(W, W, A);
+            const int ax = jr.type >= PS_X_ROT ? jr.type - PS_X_ROT : max(jr.type, 0);
+            const float ux = T.m[ax] * di, uy = T.m[4 + ax] * di, uz = T.m[8 + ax] * di;
+            if (jr.type >= PS_X_ROT) {
+                wx += ux;
+                wy += uy;
+                wz += uz;
+                A += ad * W;
+                W += ad;
+            } else {
+                vx += ux;
+                vy += uy;
+                vz += uz;
+                Ao += 2.0f * W * ad;
+                if (jr.type >= PS_X_PRISM) ok = ok && fabsf(qi) + ad <= md.slide_max;   // the levers' range
+            }
+        }
+        if (self) {
+            for (int k = jr.sph_beg + u; k < jr.sph_end; k += kSub) {
+                const float4 s = M.S[k];
+                float px, py, pz;
+                sphere_world(T, s.x, s.y, s.z, px, py, pz);
+                put3(sm.pos, k, kPathGroups, slot, px, py, pz);
+            }
+            for (int k = jr.apx_beg + u; k < jr.apx_end && md.bound_from_apx; k += kSub) {
+                const float4 s = M.A[k];
+                float px, py, pz;
+                sphere_world(T, s.x, s.y, s.z, px, py, pz);
+                put3(sm.apos, k, kPathGroups, slot, px, py, pz);
+            }
+        }
+        if (jr.reach < 0.0f) continue;   // uniform
+        float cx, cy, cz;
+        sphere_world(T, jr.bound.x, jr.bound.y, jr.bound.z, cx, cy, cz);
+        if (self && u == 0 && !md.bound_from_apx) put3(sm.cpos, p, kPathGroups, slot, cx, cy, cz);
+        if (sc.n_obbs == 0 && !kEsdf) continue;   // uniform
+        const float WA = 0.5f * fmaf(W, W, A), hAo = 0.5f * Ao;
+        // how far a point of this frame can move from its midpoint position
+        auto motion = [&](float x, float y, float z) {
+            const float rx = x - T.m[3], ry = y - T.m[7], rz = z - T.m[11];
+            const float sp = len_up(vx + wy * rz - wz * ry, vy + wz * rx - wx * rz, vz + wx * ry - wy * rx);
+            return (sp + hAo + len_up(rx, ry, rz) * WA) * 1.001f;   // a rigid transform's rounding
+        };
+        const float Sm = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz)));
+        const float R0 = jr.reach + am + motion(cx, cy, cz);
+        const float gq = (Sm + R0 + sc.Bmax + 1.0f) * G4;
+        const float Rc = R0 * (1.0f + G4) + gq;
+        const float Rcl = Rc * sc.Mscale;
+        float Rc2 = Rcl * Rcl;
+        const float Rj = (Rc * (1.0f + G4) + G4 * (Sm + 1.0f)) * (1.0f + 1.0e-6f);
+        bool near = kEsdf && esdf_reachable(sc, cx, cy, cz, Rc);
+        LaneStats st;
+#pragma unroll 1
+        for (int base = 0; base < sc.n_obbs; base += 32) {
+            const unsigned mask = reach_mask<kSub, false>(sc, obs, base, u, cx, cy, cz, Rj, Rc2, clear, [](float) {}, st);
+            if (!mask) continue;
+#pragma unroll 1
+            for (int k = jr.sph_beg + u; k < jr.sph_end && !near; k += kSub) {
+                const float4 s = M.S[k];
+                float px, py, pz;
+                sphere_world(T, s.x, s.y, s.z, px, py, pz);
+                const float lim = (fabsf(s.w) + am + motion(px, py, pz) + gq) * sc.Mscale;
+                const float lim2 = lim * lim;
+#pragma unroll 1
+                for (unsigned m = mask; m && !near; m &= m - 1) {
+                    float qx, qy, qz;
+                    near = !(fast_box_dsq(sc.obbs[base + __ffs(m) - 1], px, py, pz, qx, qy, qz) >= lim2);
+                }
+            }
+        }
+        const bool any_near = group_any<kSub>(near);   // every lane of the warp: the vote is warp-wide
+        clear = clear && !any_near;
+        if (!self && __all_sync(kGrpFull, !clear)) break;   // uniform
+    }
+    bool close = !ok;
+    if (self) {   // uniform
+        __syncwarp();   // the groups' positions are written
+        auto at = [&](const float* a, int k, int c) { return a[(k * 3 + c) * kPathGroups + slot]; };
+        auto bc = [&](int p, int c) { return md.bound_from_apx ? at(sm.apos, M.J[p].apx_beg, c) : at(sm.cpos, p, c); };
+        // the group's lanes test 4 joint pairs at a time, then share the runs of
+        // those that pass (the shuffles take the whole warp, so the loops over
+        // pairs are uniform)
+        for (int jp0 = 0; jp0 < md.n_sjp; jp0 += kSub) {
+            bool pass = false;
+            float wide = 0.0f;   // motion and guard
+            if (jp0 + u < md.n_sjp) {
+                const uint4 e = __ldg(md.sjp + jp0 + u);
+                const int a = (int)(e.x & 0xffffu), qj = (int)(e.x >> 16);
+                // how much the distance of a point of a and one of q can change
+                float m = 0.0f;
+                for (int x = qj, y = a; x != y;) {
+                    const bool up = x > y;
+                    const int k = up ? x : y;   // the later one in DFS order is not an ancestor of the other
+                    const JointRec& jk = M.J[k];
+                    if (jk.dof >= 0 && jk.type != PS_FIXED)
+                        m = fmaf(fabsf(dq[jk.dof]), __ldg(md.lever + k * NJ + (up ? qj : a)), m);
+                    if (up) x = jk.parent_pos;
+                    else y = jk.parent_pos;
+                }
+                m *= 1.001f;
+                const float ax = bc(a, 0), ay = bc(a, 1), az = bc(a, 2);
+                const float qx = bc(qj, 0), qy = bc(qj, 1), qz = bc(qj, 2);
+                const float dx = ax - qx, dy = ay - qy, dz = az - qz;
+                const float S = fmaxf(fmaxf(fabsf(ax), fmaxf(fabsf(ay), fabsf(az))),
+                                      fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz))));
+                const float R = M.J[a].reach + M.J[qj].reach;
+                wide = m + 4.0f * (S + R + m + 1.0f) * PS_GUARD_K;
+                const float lim = R + wide;
+                pass = !(fmaf(dz, dz, fmaf(dy, dy, dx * dx)) >= lim * lim);
+            }
+            const unsigned bal = group_bits<kSub>(__ballot_sync(kGrpFull, pass));
+            for (int v = 0; v < kSub && jp0 + v < md.n_sjp; ++v) {
+                const float wv = __shfl_sync(kGrpFull, wide, (threadIdx.x & 31 & ~(kSub - 1)) + v);
+                if (close || !((bal >> v) & 1u)) continue;   // no warp-wide call below
+                const uint4 e = __ldg(md.sjp + jp0 + v);
+                const int qj = (int)(e.x >> 16);
+                const float qx = bc(qj, 0), qy = bc(qj, 1), qz = bc(qj, 2), Rq = M.J[qj].reach;
+                for (int r = (int)e.y + u; r < (int)e.z && !close; r += kSub) {
+                    const uint2 run = __ldg(md.sruns + r);
+                    const int i = run.x & 0x1ff, len = run.x >> 14;
+                    const float px = at(sm.pos, i, 0), py = at(sm.pos, i, 1), pz = at(sm.pos, i, 2);
+                    const float ri = fabsf(M.S[i].w) + wv;
+                    const float ex = px - qx, ey = py - qy, ez = pz - qz;
+                    const float lim = ri + Rq;
+                    if (fmaf(ez, ez, fmaf(ey, ey, ex * ex)) >= lim * lim) continue;
+#pragma unroll 4
+                    for (int k = 0; k < len; ++k) {
+                        const int j = (int)run.y + k;
+                        const float fx = px - at(sm.pos, j, 0), fy = py - at(sm.pos, j, 1), fz = pz - at(sm.pos, j, 2);
+                        const float lj = ri + fabsf(M.S[j].w);
+                        close = close || !(fmaf(fz, fz, fmaf(fy, fy, fx * fx)) >= lj * lj);
+                    }
+                }
+            }
+        }
+        const bool any_close = group_any<kSub>(close);   // every lane of the warp
+        close = any_close;
+        __syncwarp();   // the positions' readers are done
+    }
+    return (clear ? 0u : 1u) | (self && close ? 2u : 0u);
+}
+
+// A list of intervals in shared memory: [lo, hi] and what to check them for
+// (path_sweep's bits).
+struct PathList {
+    int lo[4 * kPathGroups], hi[4 * kPathGroups];
+    unsigned char what[4 * kPathGroups];
+};
+struct PathBlock {
+    int hit;             // a sample collides
+    int n_list;          // intervals to check sample by sample
+    PathList list, cand; // those, and those to sweep
+};
+
+// Appends the groups' intervals whose bits are set to the list, in any order
+// (group leaders hold them; the caller has emptied the list, a barrier follows).
+__device__ __forceinline__ void path_collect(PathBlock& blk, unsigned bits, bool present, int lo, int hi) {
+    if ((threadIdx.x & (kPathSub - 1)) == 0 && present && bits) {
+        const int k = atomicAdd(&blk.n_list, 1);
+        blk.list.lo[k] = lo;
+        blk.list.hi[k] = hi;
+        blk.list.what[k] = (unsigned char)bits;
+    }
+}
+
+// Checks samples 0 .. per - 1 of the listed intervals, all groups at a time,
+// until one hits. place(x, s, i) gives DoF i of sample s of list entry x,
+// present(x, s) whether it exists. Every thread of the block calls it after a
+// block barrier; blk.hit holds the result after the barrier inside.
+template <bool kEsdf, class Place, class Present>
+__device__ __forceinline__ void path_samples(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
+                                             const ps_scene_view& sv, const PathSmem& ps, float margin, bool self,
+                                             PathBlock& blk, int per, Place&& place, Present&& present) {
+    constexpr int kSub = kPathSub;
+    const int D = M.H->n_dof;
+    const int lane = threadIdx.x & 31, slot = threadIdx.x / kSub, u = lane & (kSub - 1);
+    const int first = (threadIdx.x & ~31) / kSub;   // the warp's first group
+    float* qc = ps.q + slot * 2 * D;
+    volatile int* hit_flag = &blk.hit;
+    const int n = blk.n_list;
+    const long long total = (long long)per * n;
+    LaneStats st;
+    st.zero();
+    // task t: sample t / n of interval t % n, so that every interval is looked
+    // at before any is finished
+    for (long long t0 = first; t0 < total; t0 += kPathGroups) {
+        if (__any_sync(kGrpFull, *hit_flag != 0)) break;   // one decision for the warp
+        const long long t = min(t0 + (slot - first), total - 1);
+        const int x = (int)(t % n), s = (int)(t / n);
+        const unsigned what = blk.list.what[x];
+        const bool on = t0 + (slot - first) < total && present(x, s);
+        if (!__any_sync(kGrpFull, on)) continue;   // uniform
+        __syncwarp();
+        for (int i = u; i < D; i += kSub) qc[i] = on ? place(x, s, i) : 0.0f;
+        __syncwarp();
+        bool hit = false;
+        if (__any_sync(kGrpFull, on && (what & 1u))) {   // uniform
+            bool h;
+            float clr;
+            group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
+            hit = on && (what & 1u) && h;
+        }
+        if (self && on && (what & 2u) && !hit)   // uniform over the group
+            hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
+        if (hit && u == 0) *hit_flag = 1;
+        __syncwarp();
+    }
+    __syncthreads();
+}
+
+// Stages the model and the scene. False: the staging gave up (uniform).
+__device__ __forceinline__ bool path_stage(const ModelDev& md, const ps_scene_view& sv, unsigned char* smem,
+                                           uint64_t* mbar, int* counters, float* bmax, PathSmem& ps, SceneSmem& sc) {
+    if (!stage_model(md, smem, mbar)) return false;
+    ps = path_carve(smem, md, sv);
+    stage_scene(sv, ps.obbs, ps.orig, ps.layers, counters, bmax, sc);
+    box_spheres(sc, ps.obs);
+    __syncthreads();
+    box_limits(sc, ps.obs);
+    __syncthreads();
+    return true;
+}
+
+// Sample count of an edge (edge_eval.cuh:54-60 plus the L-inf rule).
+__device__ __forceinline__ int edge_samples(const ps_edge_params& P, const int* given, int e, const float* a,
+                                            const float* b, int D, float len) {
+    if (given) return given[e];
+    if (P.resolution > 0.0f) {
+        int g = (int)ceilf(__fdiv_rn(len, P.resolution));
+        return min(max(g, 2), 1024);
+    }
+    if (P.max_joint_step > 0.0f) {
+        float m = 0.0f;
+        for (int i = 0; i < D; ++i) m = fmaxf(m, fabsf(__fadd_rn(b[i], -a[i])));
+        int g = (int)ceilf(__fdiv_rn(m, P.max_joint_step));
+        const int cap = P.max_samples > 0 ? P.max_samples : 1024;
+        return min(max(g, 1), cap);
+    }
+    return P.granularity;
+}
+
+__device__ __forceinline__ float edge_length(const float* a, const float* b, int D) {
+    float len2 = 0.0f;   // edge_eval.cuh:104-106
+    for (int i = 0; i < D; ++i) {
+        float d = __fadd_rn(b[i], -a[i]);
+        len2 = __fmaf_rn(d, d, len2);
+    }
+    return sqrtf(len2);
+}
+
+// ---------------------------------------------------------------------------
+// Small edge batches: one block per edge
+// ---------------------------------------------------------------------------
+template <bool kEsdf>
+__global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md, ps_scene_view sv, ps_edge_params P,
+                                                                     const float* __restrict__ from,
+                                                                     const float* __restrict__ to,
+                                                                     const int* __restrict__ given, int n_edges,
+                                                                     uint8_t* __restrict__ valid,
+                                                                     float* __restrict__ cost,
+                                                                     float* __restrict__ clearance, int* timed_out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    __shared__ PathBlock blk;
+    PathSmem ps;
+    SceneSmem sc;
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, ps, sc)) {   // fail closed
+        if (threadIdx.x == 0) {
+            atomicExch(timed_out, 1);
+            for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
+                valid[e] = 0;
+                cost[e] = FLT_MAX;
+                if (clearance) clearance[e] = FLT_MAX;
+            }
+        }
+        return;
+    }
+    const ModelSmem M = model_view(smem);
+    const int D = M.H->n_dof;
+    const int slot = threadIdx.x / kPathSub, u = threadIdx.x & (kPathSub - 1);
+    const bool self = P.check_self != 0;
+    const float margin = P.collision_margin;
+    float* qm = ps.q + slot * 2 * D;
+    float* dq = qm + D;
+    for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
+        const float* a = from + (size_t)e * D;
+        const float* b = to + (size_t)e * D;
+        const float len = edge_length(a, b, D);
+        const int G = edge_samples(P, given, e, a, b, D, len);
+        const bool start = G > 0 && (G % 16) != 0;   // the start configuration belongs to the samples
+        // at most 32 intervals of m samples; when all samples fit the groups, one each and no swept check
+        const bool direct = G + (start ? 1 : 0) <= kPathGroups;
+        const int m = direct ? 1 : (G + kPathGroups - 1) / kPathGroups;
+        const int n = G > 0 ? (G + m - 1) / m : 0;
+        __syncthreads();   // the previous edge's readers of blk are done
+        if (threadIdx.x == 0) blk.hit = blk.n_list = 0;
+        if (threadIdx.x < kPathGroups) {
+            const int x = threadIdx.x;
+            blk.cand.lo[x] = !direct && x == 0 && start ? 0 : (x < n ? x * m + 1 : 0);   // direct: the start after the last
+            blk.cand.hi[x] = x < n ? min((x + 1) * m, G) : 0;
+            blk.cand.what[x] = self ? 3u : 1u;
+        }
+        __syncthreads();
+        int nc = direct && start ? n + 1 : n, per = direct ? 1 : m + 1;
+        for (bool quarters = false;; quarters = true) {
+            // ---- swept check of the candidates, a group each ----
+            for (int k0 = 0; k0 < nc; k0 += kPathGroups) {
+                const int k = min(k0 + slot, nc - 1);   // a group past the end repeats the last one
+                const int lo = blk.cand.lo[k], hi = blk.cand.hi[k];
+                unsigned bits = blk.cand.what[k];
+                if (!direct) {   // uniform
+                    const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
+                                th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
+                    bool ok = true;
+                    __syncwarp();
+                    for (int i = 0; i < D; ++i) {
+                        const float ai = __ldg(a + i), bi = __ldg(b + i);
+                        ok = ok && fabsf(ai) <= kSweepMaxQ && fabsf(bi) <= kSweepMaxQ;
+                        if ((i & (kPathSub - 1)) == u) {
+                            qm[i] = fmaf(tm, bi - ai, ai);
+                            dq[i] = th * (bi - ai);
+                        }
+                    }
+                    __syncwarp();
+                    bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qm, dq, margin, ok, self, ps.self, slot);
+                }
+                path_collect(blk, bits, k0 + slot < nc && lo <= hi, lo, hi);
+            }
+            __syncthreads();
+            // ---- samples of the intervals left: all of them if they are few,
+            //      else the middle ones, and the intervals once more in quarters ----
+            const int left = blk.n_list;
+            const bool all = direct || quarters || (long long)left * per <= 2 * kPathGroups;
+            path_samples<kEsdf>(
+                M, md, sc, sv, ps, margin, self, blk, all ? per : 1,
+                [&](int x, int s, int i) {
+                    const int lo = blk.list.lo[x], cnt = blk.list.hi[x] - lo + 1;
+                    const int j = lo + (s + cnt / 2) % cnt;   // from the middle on
+                    const float t = __fdiv_rn((float)j, (float)G);
+                    const float ai = __ldg(a + i), bi = __ldg(b + i);
+                    return __fmaf_rn(t, __fadd_rn(bi, -ai), ai);
+                },
+                [&](int x, int s) { return s <= blk.list.hi[x] - blk.list.lo[x]; });
+            if (all || blk.hit) break;   // uniform
+            if (threadIdx.x < left)
+                for (int k = 0; k < 4; ++k) {
+                    const int lo = blk.list.lo[threadIdx.x], cnt = blk.list.hi[threadIdx.x] - lo + 1;
+                    blk.cand.lo[4 * threadIdx.x + k] = lo + (int)((long long)cnt * k / 4);
+                    blk.cand.hi[4 * threadIdx.x + k] = lo + (int)((long long)cnt * (k + 1) / 4) - 1;
+                    blk.cand.what[4 * threadIdx.x + k] = blk.list.what[threadIdx.x];
+                }
+            __syncthreads();   // the list's readers are done
+            if (threadIdx.x == 0) blk.n_list = 0;
+            __syncthreads();
+            nc = 4 * left;
+            per = (per + 3) / 4 + 1;
+        }
+        if (threadIdx.x == 0) {
+            const bool bad = blk.hit != 0;
+            valid[e] = bad ? 0 : 1;
+            cost[e] = bad ? FLT_MAX : len;
+            if (clearance) clearance[e] = FLT_MAX;
+        }
+    }
+}
+
+}  // namespace
+}  // namespace ps
