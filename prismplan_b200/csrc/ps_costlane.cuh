@@ -416,7 +416,7 @@ __device__ float lane_cost(const ModelSmem& M, const ModelDev& md, const SceneSm
                 lane_group<1, kGrad>(M, T, k0, jr.sph_end, sc, ws.cand, ncand, px, py, pz, rr, key, arg, kk, val);
             else {
                 lane_group<1, kGrad>(M, T, k0, jr.sph_end, sc, ws.cand, 0, px, py, pz, rr, key, arg, kk, val);
-                if (ncand > 0)
+                if (ncand > 0 && val[0])   // a lane past the joint's spheres has no mask row
                     lane_key_masked(sc, ws.cand, ncand, px[0], py[0], pz[0],
                                     sv.sphere_obb_acm_mask + (size_t)M.SO[kk[0]] * sv.n_obbs, key[0], arg[0]);
             }
