@@ -36,19 +36,19 @@ namespace {
 // waypoint costs + lambda theta^T R theta, the same traj_smooth_block as
 // ps_traj_cost, so the same bits), then the shared bookkeeping.
 __global__ void chomp_bookkeep_kernel(const float* __restrict__ theta, const float* __restrict__ wp_cost,
-                                      const uint8_t* __restrict__ seg_valid, const uint8_t* __restrict__ wp_hit,
-                                      int T, int D, ps_cost_params P, int n_iter, float conv_eps,
+                                      OptVerdict v, int T, int D, ps_cost_params P, int n_iter, float conv_eps,
                                       float time_limit_ms, const unsigned long long* __restrict__ t0,
                                       OptState* __restrict__ state, uint8_t* __restrict__ done,
                                       float* __restrict__ best, int* __restrict__ n_done) {
     extern __shared__ float sh[];   // traj_smooth_block: 2 (T + 12) + blockDim
     const int b = blockIdx.x;
+    if (b == 0 && threadIdx.x == 0) *v.n_list = 0;
     if (done[b]) return;   // uniform over the block
     const float* th = theta + (size_t)b * T * D;
     const float total = traj_smooth_block([&](int t, int d) { return th[(size_t)t * D + d]; },
                                           [&](int, int, float) {},
                                           [&](int t) { return wp_cost[(size_t)b * T + t]; }, T, D, P, false, sh);
-    opt_bookkeep_block(b, th, total, seg_valid, wp_hit, T, D, n_iter, conv_eps, time_limit_ms, t0, state, done, best,
+    opt_bookkeep_block(b, th, total, v, T, D, n_iter, conv_eps, time_limit_ms, t0, state, done, best,
                        n_done);
 }
 
@@ -167,7 +167,8 @@ extern "C" int ps_chomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     cp_total.smoothness_weight = P->smoothness_weight;
 
     opt_band_kernel<<<1, 1, 0, s>>>(T, P->delta_t, o.band);
-    opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0);
+    opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0, o.hit_step,
+                                                  o.n_list);
     PS_TRY_CUDA(cudaGetLastError());
     const int bk_threads = 128;
     const size_t bk_smem = (size_t)(2 * (T + 12) + bk_threads) * sizeof(float);
@@ -183,10 +184,11 @@ extern "C" int ps_chomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     // lives in the device state, so every iteration enqueues the same work.
     auto iteration = [&](cudaStream_t q, int) -> int {
         if (int rc = traj_cost_launch(m, scene, theta, B, T, &cp, w.wp, nullptr, w.grad, o.done, q)) return rc;
+        OptVerdict v;
         if (int rc = opt_validity(m, scene, theta, B, T, D, P->collision_margin, P->check_self,
-                                  P->collision_check_step, o, q))
+                                  P->collision_check_step, o, v, q))
             return rc;
-        chomp_bookkeep_kernel<<<B, bk_threads, bk_smem, q>>>(theta, w.wp, o.evalid, o.hit, T, D, cp_total,
+        chomp_bookkeep_kernel<<<B, bk_threads, bk_smem, q>>>(theta, w.wp, v, T, D, cp_total,
                                                              P->num_iterations, P->convergence_eps, P->time_limit_ms,
                                                              o.t0, o.state, o.done, best, o.n_done);
         PS_TRY_CUDA(cudaGetLastError());

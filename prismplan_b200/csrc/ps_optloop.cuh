@@ -16,6 +16,7 @@
 #include <cmath>
 
 #include "ps_internal.h"
+#include "ps_pathkern.cuh"
 
 namespace ps {
 namespace {
@@ -117,10 +118,12 @@ __device__ __forceinline__ void band_solve(const double* Ls, double* x, int T) {
 }
 
 __global__ void opt_init_kernel(OptState* __restrict__ st, uint8_t* __restrict__ done, int B, int polish,
-                                int* __restrict__ n_done, unsigned long long* __restrict__ t0) {
+                                int* __restrict__ n_done, unsigned long long* __restrict__ t0,
+                                int* __restrict__ hit_step, int* __restrict__ n_list) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b == 0) {
         *n_done = 0;
+        *n_list = 0;
         *t0 = now_ns();
     }
     if (b >= B) return;
@@ -136,6 +139,7 @@ __global__ void opt_init_kernel(OptState* __restrict__ st, uint8_t* __restrict__
     s.step = 0;
     st[b] = s;
     done[b] = 0;
+    hit_step[b] = 0;
 }
 
 // One block per request: its segments (theta_t -> theta_t+1) as edges with
@@ -181,6 +185,149 @@ __global__ void opt_segments_kernel(const float* __restrict__ theta, int T, int 
     for (int t = threadIdx.x; t < T - 1; t += blockDim.x) G[e0 + t] = g;
 }
 
+// Validity of the iterates in one launch (opt_validity's usual path): a block
+// takes a slice of 32 consecutive segments of a request, a group each. The
+// swept check shows most segments clear, ends included; the waypoints and
+// waypoints of the others are checked, and their densified samples when they
+// are few; else the segments go on a list for opt_refine_kernel, a block each
+// (an iterate far from its goal has some 90 samples on each of 63 segments).
+// All that stops when one of the request's slices has a
+// hit: hit_step[b] = the request's step + 1 (so that nothing needs clearing
+// between iterations). Together the same points as the waypoint
+// and segment checks below (a waypoint is the start of its segment; the last
+// one belongs to the last slice), so the request's validity is the same.
+// Finished requests are skipped.
+//
+// Those checks took eight launches (scene and self check of the waypoints,
+// segments, header, preparation, two queue passes, self pass, finalize) and
+// 141 us of a 256-request CHOMP iteration; this kernel takes 46 us and
+// opt_refine_kernel 38 us. With the refining inside this kernel (one launch)
+// the few requests without a colliding waypoint held it for 112 us.
+template <bool kEsdf>
+__global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md, ps_scene_view sv,
+                                                                    const float* __restrict__ theta, int T,
+                                                                    float check_step, float margin, int check_self,
+                                                                    const uint8_t* __restrict__ done,
+                                                                    const OptState* __restrict__ state,
+                                                                    int* hit_step, int2* __restrict__ list,
+                                                                    int* n_list) {
+    const int b = blockIdx.y;
+    if (done[b]) return;   // uniform over the block
+    const int now = state[b].step + 1;
+    volatile int* hit_at = hit_step + b;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    __shared__ PathBlock blk;
+    __shared__ int max_seg_bits;
+    PathSmem ps;
+    SceneSmem sc;
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, ps, sc)) {   // fail closed
+        if (threadIdx.x == 0) *hit_at = now;
+        return;
+    }
+    const ModelSmem M = model_view(smem);
+    const int D = M.H->n_dof;
+    const bool self = check_self != 0;
+    const float* th = theta + (size_t)b * T * D;
+    if (threadIdx.x == 0) blk.hit = max_seg_bits = 0;
+    __syncthreads();
+    // n_sub of the whole request, as opt_segments_kernel computes it
+    float mx = 0.0f;
+    for (int t = threadIdx.x; t < T - 1; t += blockDim.x) {
+        float d2 = 0.0f;
+        for (int d = 0; d < D; ++d) {
+            const float df = __fsub_rn(th[(t + 1) * D + d], th[t * D + d]);
+            d2 = __fadd_rn(d2, __fmul_rn(df, df));
+        }
+        mx = fmaxf(mx, __fsqrt_rn(d2));
+    }
+    atomicMax(&max_seg_bits, __float_as_int(mx));   // non-negative floats order as ints
+    __syncthreads();
+    const float max_seg = __int_as_float(max_seg_bits);
+    int G = 1;   // n_sub, capped so that the cast stays defined
+    if (check_step > 0.0f && max_seg > check_step)
+        G = (int)fminf(ceilf(__fdiv_rn(max_seg, check_step)), 1048576.0f);
+    // the slice's segments: the waypoint, samples 1 .. G, and after the last one its end
+    const int seg0 = blockIdx.x * kPathGroups, n = min(kPathGroups, T - 1 - seg0);
+    if (threadIdx.x < n)
+        blk.stack[threadIdx.x] =
+            PathItem{seg0 + (int)threadIdx.x, 0, seg0 + (int)threadIdx.x == T - 2 ? G + 1 : G, self ? 3 : 1};
+    if (threadIdx.x == 0) blk.n_stack = n;
+    __syncthreads();
+    path_run<kEsdf, true>(
+        M, md, sc, sv, ps, margin, self, blk, G, true,
+        [&](int sg, int i, float& a, float& b) {
+            a = th[sg * D + i];
+            b = th[(sg + 1) * D + i];
+        },
+        [&]() { return *hit_at == now; },
+        [&](const PathItem& x) { list[atomicAdd(n_list, 1)] = make_int2(b * (T - 1) + x.seg, G << 2 | x.what); });
+    if (threadIdx.x == 0 && blk.hit) *hit_at = now;
+}
+
+// The segments that opt_check_kernel put on the list, a block each.
+template <bool kEsdf>
+__global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md, ps_scene_view sv,
+                                                                     const float* __restrict__ theta, int T,
+                                                                     float margin, int check_self,
+                                                                     const OptState* __restrict__ state,
+                                                                     int* hit_step, const int2* __restrict__ list,
+                                                                     const int* __restrict__ n_list) {
+    const int total = *n_list;
+    if ((int)blockIdx.x >= total) return;   // uniform over the block
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    __shared__ PathBlock blk;
+    PathSmem ps;
+    SceneSmem sc;
+    const bool staged = path_stage(md, sv, smem, &mbar, counters, &bmax, ps, sc);
+    const ModelSmem M = model_view(smem);
+    const bool self = check_self != 0;
+    for (int k = blockIdx.x; k < total; k += gridDim.x) {
+        const int2 item = list[k];
+        const int b = item.x / (T - 1), sg = item.x - b * (T - 1), G = item.y >> 2;
+        const int now = state[b].step + 1;
+        volatile int* hit_at = hit_step + b;
+        if (!staged) {   // fail closed
+            if (threadIdx.x == 0) *hit_at = now;
+            continue;
+        }
+        if (__syncthreads_or(*hit_at == now)) continue;   // the request is known to collide (also: blk's readers are done)
+        const float* a = theta + ((size_t)b * T + sg) * M.H->n_dof;
+        const float* c = a + M.H->n_dof;
+        // samples 1 .. G, and the trajectory's end on its last segment, in up to 32 intervals
+        const int hi = sg == T - 2 ? G + 1 : G, m = (hi + kPathGroups - 1) / kPathGroups, n = (hi + m - 1) / m;
+        if (threadIdx.x == 0) {
+            blk.hit = 0;
+            blk.n_stack = n;
+        }
+        if (threadIdx.x < n)
+            blk.stack[threadIdx.x] =
+                PathItem{sg, (int)threadIdx.x * m + 1, min(((int)threadIdx.x + 1) * m, hi), item.y & 3};
+        __syncthreads();
+        path_run<kEsdf, false>(
+            M, md, sc, sv, ps, margin, self, blk, G, false,
+            [&](int, int i, float& x, float& y) {
+                x = a[i];
+                y = c[i];
+            },
+            [&]() { return *hit_at == now; }, [](const PathItem&) {});
+        if (threadIdx.x == 0 && blk.hit) *hit_at = now;
+    }
+}
+
+// What opt_bookkeep_block reads an iterate's validity from: hit_step
+// (opt_check_kernel) when given, else the segments' and waypoints' verdicts.
+struct OptVerdict {
+    const uint8_t *seg_valid, *wp_hit;
+    const int* hit_step;
+    int* n_list;   // opt_check_kernel's list, emptied for the next iteration
+};
+
 // Block-level part of the bookkeeping for request b (call from every thread
 // of a one-block-per-request kernel; `total` valid in thread 0): validity =
 // every segment and every waypoint free; then the reference's state machine
@@ -189,15 +336,18 @@ __global__ void opt_segments_kernel(const float* __restrict__ theta, int T, int 
 // copied into best when it improved. The reference checks its stop
 // conditions at the top of the next iteration; here they are checked at the
 // end of this one, which stops at the same iterate.
-__device__ void opt_bookkeep_block(int b, const float* __restrict__ th, float total, const uint8_t* __restrict__ seg_valid,
-                                   const uint8_t* __restrict__ wp_hit, int T, int D, int n_iter, float conv_eps,
+__device__ void opt_bookkeep_block(int b, const float* __restrict__ th, float total, const OptVerdict v, int T, int D, int n_iter, float conv_eps,
                                    float time_limit_ms, const unsigned long long* __restrict__ t0,
                                    OptState* __restrict__ state, uint8_t* __restrict__ done, float* __restrict__ best,
                                    int* __restrict__ n_done) {
     __shared__ int s_improved;
     bool bad = false;
-    for (int t = threadIdx.x; t < T - 1; t += blockDim.x) bad |= seg_valid[(size_t)b * (T - 1) + t] == 0;
-    for (int t = threadIdx.x; t < T; t += blockDim.x) bad |= wp_hit[(size_t)b * T + t] != 0;
+    if (v.hit_step) {
+        bad = v.hit_step[b] == state[b].step + 1;   // every thread, before thread 0 advances the step
+    } else {
+        for (int t = threadIdx.x; t < T - 1; t += blockDim.x) bad |= v.seg_valid[(size_t)b * (T - 1) + t] == 0;
+        for (int t = threadIdx.x; t < T; t += blockDim.x) bad |= v.wp_hit[(size_t)b * T + t] != 0;
+    }
     const bool valid = __syncthreads_or(bad) == 0;
     if (threadIdx.x == 0) {
         OptState s = state[b];
@@ -275,7 +425,8 @@ struct Carver {
 struct OptBufs {
     OptState* state;
     uint8_t *done, *evalid, *hit;
-    int *G, *n_done;
+    int *G, *n_done, *hit_step, *n_list;
+    int2* list;
     unsigned long long* t0;
     float *from, *to, *ecost;
     double* band;   // 5 T, opt_band_kernel
@@ -291,6 +442,9 @@ inline void opt_carve(Carver& c, int B, int T, int D, OptBufs& o) {
     o.hit = c.take<uint8_t>(BT);
     o.G = c.take<int>(4 * E);
     o.n_done = c.take<int>(sizeof(int));
+    o.hit_step = c.take<int>(4 * Bq);
+    o.n_list = c.take<int>(sizeof(int));
+    o.list = c.take<int2>(8 * E);
     o.t0 = c.take<unsigned long long>(sizeof(unsigned long long));
     o.from = c.take<float>(4 * E * D);
     o.to = c.take<float>(4 * E * D);
@@ -300,11 +454,29 @@ inline void opt_carve(Carver& c, int B, int T, int D, OptBufs& o) {
     o.ews = c.take<unsigned char>(o.ews_bytes);
 }
 
-// Densified validity of the B iterates theta [B][T][D]: every waypoint
-// (configuration kernel) and every segment sample (persistent edge kernel,
-// G = n_sub), self check as asked. Results in o.hit / o.evalid.
+// Densified validity of the B iterates theta [B][T][D]: every waypoint and
+// every segment sample (G = n_sub), self check as asked; `v` says where the
+// bookkeeping finds it. Models and scenes that opt_check_kernel does not serve
+// go through the configuration kernel and the persistent edge kernel.
 inline int opt_validity(const ps_model* m, const ps_scene_view* scene, const float* theta, int B, int T, int D,
-                        float collision_margin, int check_self, float check_step, const OptBufs& o, cudaStream_t q) {
+                        float collision_margin, int check_self, float check_step, const OptBufs& o, OptVerdict& v,
+                        cudaStream_t q) {
+    const int slices = (T - 1 + kPathGroups - 1) / kPathGroups;
+    v = OptVerdict{o.evalid, o.hit, nullptr, o.n_list};
+    if (m->rigid && !g_stats && B <= 65535 && path_serves(m, scene, collision_margin, check_self != 0)) {
+        auto k = scene->n_voxel_layers > 0 ? opt_check_kernel<true> : opt_check_kernel<false>;
+        const size_t smem = path_smem_bytes(m, scene, check_self != 0);
+        PS_TRY_CUDA(allow_smem((const void*)k, smem));
+        auto k2 = scene->n_voxel_layers > 0 ? opt_refine_kernel<true> : opt_refine_kernel<false>;
+        PS_TRY_CUDA(allow_smem((const void*)k2, smem));
+        v = OptVerdict{nullptr, nullptr, o.hit_step, o.n_list};
+        k<<<dim3(slices, B), kPathThreads, smem, q>>>(m->dev, *scene, theta, T, check_step, collision_margin, check_self,
+                                                      o.done, o.state, o.hit_step, o.list, o.n_list);
+        k2<<<(unsigned)std::min<long long>((long long)B * (T - 1), sm_count() * 4ll), kPathThreads, smem, q>>>(
+            m->dev, *scene, theta, T, collision_margin, check_self, o.state, o.hit_step, o.list, o.n_list);
+        PS_TRY_CUDA(cudaGetLastError());
+        return PS_OK;
+    }
     ps_edge_params ep{};
     ep.granularity = 1;
     ep.collision_margin = collision_margin;

@@ -8,13 +8,14 @@
 // more, one thread per sample, for the self check, with a preparation, a
 // second queue pass and a finalize around them. Here a block of 32 groups of 4
 // lanes holds one path.
-//   1. Swept check: the path is cut into at most 32 intervals, one per group.
+//   1. Swept check: the path is cut into intervals of samples, one per group.
 //      From one kinematic pass at an interval's middle, with bounds on how far
 //      links move inside it, an interval is shown clear of every box (and out
 //      of reach of every ESDF layer) and of self collision, or not. Skipped
 //      when the samples themselves fit the groups.
 //   2. The samples of the other intervals are checked one by one, a group
-//      each (group_verdict, group_self_hit), until one hits.
+//      each (group_verdict, group_self_hit), until one hits; when there are
+//      many, only their middles, and step 1 goes over their quarters.
 // The verdict is the OR over the samples' verdicts, and step 1 only leaves out
 // samples that cannot hit, so the result is the queue path's.
 #pragma once
@@ -273,70 +274,130 @@ __device__ __forceinline__ unsigned path_sweep(const ModelSmem& M, const ModelDe
     return (clear ? 0u : 1u) | (self && close ? 2u : 0u);
 }
 
-// A list of intervals in shared memory: [lo, hi] and what to check them for
+// An interval of a segment's samples, lo .. hi, and what to check it for
 // (path_sweep's bits).
-struct PathList {
-    int lo[4 * kPathGroups], hi[4 * kPathGroups];
-    unsigned char what[4 * kPathGroups];
+struct PathItem {
+    int seg, lo, hi, what;
 };
+constexpr int kPathStack = 256;
 struct PathBlock {
-    int hit;             // a sample collides
-    int n_list;          // intervals to check sample by sample
-    PathList list, cand; // those, and those to sweep
+    int hit;          // a sample collides
+    int n_stack;      // intervals still to sweep
+    int n_list;       // intervals of this pass that the swept check left
+    int n_samples;    // samples they hold (saturated)
+    PathItem list[kPathGroups], stack[kPathStack];
 };
 
-// Appends the groups' intervals whose bits are set to the list, in any order
-// (group leaders hold them; the caller has emptied the list, a barrier follows).
-__device__ __forceinline__ void path_collect(PathBlock& blk, unsigned bits, bool present, int lo, int hi) {
-    if ((threadIdx.x & (kPathSub - 1)) == 0 && present && bits) {
-        const int k = atomicAdd(&blk.n_list, 1);
-        blk.list.lo[k] = lo;
-        blk.list.hi[k] = hi;
-        blk.list.what[k] = (unsigned char)bits;
-    }
-}
-
-// Checks samples 0 .. per - 1 of the listed intervals, all groups at a time,
-// until one hits. place(x, s, i) gives DoF i of sample s of list entry x,
-// present(x, s) whether it exists. Every thread of the block calls it after a
-// block barrier; blk.hit holds the result after the barrier inside.
-template <bool kEsdf, class Place, class Present>
-__device__ __forceinline__ void path_samples(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
-                                             const ps_scene_view& sv, const PathSmem& ps, float margin, bool self,
-                                             PathBlock& blk, int per, Place&& place, Present&& present) {
+// Works through the intervals on blk.stack, 32 at a time from the top, until
+// one sample hits, stop() says that the answer no longer matters, or nothing
+// is left: the swept check (skipped for single samples), then for the
+// intervals that it leaves every sample if they are few, else the middle ones
+// (on the first pass the first ones, when `ends`) and the intervals once more
+// in quarters (with kDefer they go to defer(), a thread each, instead).
+//
+// point(seg, i, a, b): DoF i of a segment's ends; sample j is a + (j / G)
+// (b - a), rounded as the edge kernels round it, and j = G + 1 is b itself.
+// Every thread of the block calls it after a block barrier; blk.hit holds the
+// result after the barrier inside.
+template <bool kEsdf, bool kDefer, class Point, class Stop, class Defer>
+__device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
+                                         const ps_scene_view& sv, const PathSmem& ps, float margin, bool self,
+                                         PathBlock& blk, int G, bool ends, Point&& point, Stop&& stop,
+                                         Defer&& defer) {
     constexpr int kSub = kPathSub;
     const int D = M.H->n_dof;
     const int lane = threadIdx.x & 31, slot = threadIdx.x / kSub, u = lane & (kSub - 1);
     const int first = (threadIdx.x & ~31) / kSub;   // the warp's first group
     float* qc = ps.q + slot * 2 * D;
+    float* dq = qc + D;
     volatile int* hit_flag = &blk.hit;
-    const int n = blk.n_list;
-    const long long total = (long long)per * n;
     LaneStats st;
     st.zero();
-    // task t: sample t / n of interval t % n, so that every interval is looked
-    // at before any is finished
-    for (long long t0 = first; t0 < total; t0 += kPathGroups) {
-        if (__any_sync(kGrpFull, *hit_flag != 0)) break;   // one decision for the warp
-        const long long t = min(t0 + (slot - first), total - 1);
-        const int x = (int)(t % n), s = (int)(t / n);
-        const unsigned what = blk.list.what[x];
-        const bool on = t0 + (slot - first) < total && present(x, s);
-        if (!__any_sync(kGrpFull, on)) continue;   // uniform
-        __syncwarp();
-        for (int i = u; i < D; i += kSub) qc[i] = on ? place(x, s, i) : 0.0f;
-        __syncwarp();
-        bool hit = false;
-        if (__any_sync(kGrpFull, on && (what & 1u))) {   // uniform
-            bool h;
-            float clr;
-            group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
-            hit = on && (what & 1u) && h;
+    for (bool begin = true;; begin = false) {
+        const int ns = blk.n_stack, nc = min(ns, kPathGroups);
+        if (nc == 0) break;   // uniform
+        // ---- swept check of the top intervals, a group each ----
+        const PathItem it = blk.stack[ns - 1 - min(slot, nc - 1)];   // a group past the end repeats the last one
+        const bool single = it.lo == it.hi;
+        __syncthreads();   // the stack's and the last pass' readers are done
+        if (threadIdx.x == 0) {
+            blk.n_stack = ns - nc;
+            blk.n_list = blk.n_samples = 0;
         }
-        if (self && on && (what & 2u) && !hit)   // uniform over the group
-            hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
-        if (hit && u == 0) *hit_flag = 1;
-        __syncwarp();
+        unsigned bits = (unsigned)it.what;
+        if (!__all_sync(kGrpFull, single)) {   // uniform
+            const int lo = min(it.lo, G), hi = min(it.hi, G);
+            const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
+                        th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
+            bool ok = !single;   // a single sample is checked itself
+            __syncwarp();
+            for (int i = 0; i < D; ++i) {
+                float a, b;
+                point(it.seg, i, a, b);
+                ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
+                if ((i & (kSub - 1)) == u) {
+                    qc[i] = fmaf(tm, b - a, a);
+                    dq[i] = th * (b - a);
+                }
+            }
+            __syncwarp();
+            bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
+        }
+        __syncthreads();   // the list is empty
+        if (u == 0 && slot < nc && bits) {   // in any order
+            const int k = atomicAdd(&blk.n_list, 1);
+            blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
+            atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
+        }
+        __syncthreads();
+        const int n = blk.n_list;
+        const bool all = blk.n_samples <= 2 * kPathGroups || blk.n_stack + 4 * n > kPathStack;
+        int per = 1;
+        if (all)
+            for (int k = 0; k < n; ++k) per = max(per, blk.list[k].hi - blk.list[k].lo + 1);
+        // ---- samples: task t is sample t / n of interval t % n, so that every
+        //      interval is looked at before any is finished ----
+        const long long total = (long long)per * n;
+        for (long long t0 = first; t0 < total; t0 += kPathGroups) {
+            if (__any_sync(kGrpFull, *hit_flag != 0 || stop())) break;   // one decision for the warp
+            const long long t = min(t0 + (slot - first), total - 1);
+            const PathItem x = blk.list[(int)(t % n)];
+            const int s = (int)(t / n), cnt = x.hi - x.lo + 1;
+            const bool on = t0 + (slot - first) < total && s < cnt;
+            if (!__any_sync(kGrpFull, on)) continue;   // uniform
+            const int j = x.lo + (begin && ends ? s : (s + cnt / 2) % cnt);   // from the middle on
+            const float tj = __fdiv_rn((float)j, (float)G);
+            __syncwarp();
+            for (int i = u; i < D; i += kSub) {
+                float a, b;
+                point(x.seg, i, a, b);
+                qc[i] = j > G ? b : __fmaf_rn(tj, __fadd_rn(b, -a), a);
+            }
+            __syncwarp();
+            bool hit = false;
+            if (__any_sync(kGrpFull, on && (x.what & 1))) {   // uniform
+                bool h;
+                float clr;
+                group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
+                hit = on && (x.what & 1) && h;
+            }
+            if (self && on && (x.what & 2) && !hit)   // uniform over the group
+                hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
+            if (hit && u == 0) *hit_flag = 1;
+            __syncwarp();
+        }
+        __syncthreads();
+        if (__syncthreads_or(*hit_flag != 0 || stop())) break;   // one decision for the block
+        if (!all && threadIdx.x < n) {
+            const PathItem x = blk.list[threadIdx.x];
+            const long long cnt = x.hi - x.lo + 1;
+            if (kDefer) defer(x);
+            for (int k = 0; k < 4 && cnt > 1 && !kDefer; ++k) {
+                const int lo = x.lo + (int)(cnt * k / 4), hi = x.lo + (int)(cnt * (k + 1) / 4) - 1;
+                if (lo <= hi) blk.stack[atomicAdd(&blk.n_stack, 1)] = PathItem{x.seg, lo, hi, x.what};
+            }
+        }
+        __syncthreads();
     }
     __syncthreads();
 }
@@ -412,84 +473,35 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md
     }
     const ModelSmem M = model_view(smem);
     const int D = M.H->n_dof;
-    const int slot = threadIdx.x / kPathSub, u = threadIdx.x & (kPathSub - 1);
     const bool self = P.check_self != 0;
     const float margin = P.collision_margin;
-    float* qm = ps.q + slot * 2 * D;
-    float* dq = qm + D;
     for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
         const float* a = from + (size_t)e * D;
         const float* b = to + (size_t)e * D;
         const float len = edge_length(a, b, D);
         const int G = edge_samples(P, given, e, a, b, D, len);
         const bool start = G > 0 && (G % 16) != 0;   // the start configuration belongs to the samples
-        // at most 32 intervals of m samples; when all samples fit the groups, one each and no swept check
-        const bool direct = G + (start ? 1 : 0) <= kPathGroups;
-        const int m = direct ? 1 : (G + kPathGroups - 1) / kPathGroups;
+        // at most 32 intervals (33 with the start by itself); single samples when they fit the groups
+        const int m = max(1, (G + kPathGroups - 1) / kPathGroups);
         const int n = G > 0 ? (G + m - 1) / m : 0;
         __syncthreads();   // the previous edge's readers of blk are done
-        if (threadIdx.x == 0) blk.hit = blk.n_list = 0;
-        if (threadIdx.x < kPathGroups) {
-            const int x = threadIdx.x;
-            blk.cand.lo[x] = !direct && x == 0 && start ? 0 : (x < n ? x * m + 1 : 0);   // direct: the start after the last
-            blk.cand.hi[x] = x < n ? min((x + 1) * m, G) : 0;
-            blk.cand.what[x] = self ? 3u : 1u;
+        if (threadIdx.x == 0) {
+            blk.hit = 0;
+            blk.n_stack = n + (start && m == 1 ? 1 : 0);
+        }
+        if (threadIdx.x <= n && G > 0) {
+            const int x = threadIdx.x;   // x = n: the start configuration
+            blk.stack[x] = PathItem{0, x == n || (x == 0 && start && m > 1) ? 0 : x * m + 1,
+                                    x == n ? 0 : min((x + 1) * m, G), self ? 3 : 1};
         }
         __syncthreads();
-        int nc = direct && start ? n + 1 : n, per = direct ? 1 : m + 1;
-        for (bool quarters = false;; quarters = true) {
-            // ---- swept check of the candidates, a group each ----
-            for (int k0 = 0; k0 < nc; k0 += kPathGroups) {
-                const int k = min(k0 + slot, nc - 1);   // a group past the end repeats the last one
-                const int lo = blk.cand.lo[k], hi = blk.cand.hi[k];
-                unsigned bits = blk.cand.what[k];
-                if (!direct) {   // uniform
-                    const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
-                                th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
-                    bool ok = true;
-                    __syncwarp();
-                    for (int i = 0; i < D; ++i) {
-                        const float ai = __ldg(a + i), bi = __ldg(b + i);
-                        ok = ok && fabsf(ai) <= kSweepMaxQ && fabsf(bi) <= kSweepMaxQ;
-                        if ((i & (kPathSub - 1)) == u) {
-                            qm[i] = fmaf(tm, bi - ai, ai);
-                            dq[i] = th * (bi - ai);
-                        }
-                    }
-                    __syncwarp();
-                    bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qm, dq, margin, ok, self, ps.self, slot);
-                }
-                path_collect(blk, bits, k0 + slot < nc && lo <= hi, lo, hi);
-            }
-            __syncthreads();
-            // ---- samples of the intervals left: all of them if they are few,
-            //      else the middle ones, and the intervals once more in quarters ----
-            const int left = blk.n_list;
-            const bool all = direct || quarters || (long long)left * per <= 2 * kPathGroups;
-            path_samples<kEsdf>(
-                M, md, sc, sv, ps, margin, self, blk, all ? per : 1,
-                [&](int x, int s, int i) {
-                    const int lo = blk.list.lo[x], cnt = blk.list.hi[x] - lo + 1;
-                    const int j = lo + (s + cnt / 2) % cnt;   // from the middle on
-                    const float t = __fdiv_rn((float)j, (float)G);
-                    const float ai = __ldg(a + i), bi = __ldg(b + i);
-                    return __fmaf_rn(t, __fadd_rn(bi, -ai), ai);
-                },
-                [&](int x, int s) { return s <= blk.list.hi[x] - blk.list.lo[x]; });
-            if (all || blk.hit) break;   // uniform
-            if (threadIdx.x < left)
-                for (int k = 0; k < 4; ++k) {
-                    const int lo = blk.list.lo[threadIdx.x], cnt = blk.list.hi[threadIdx.x] - lo + 1;
-                    blk.cand.lo[4 * threadIdx.x + k] = lo + (int)((long long)cnt * k / 4);
-                    blk.cand.hi[4 * threadIdx.x + k] = lo + (int)((long long)cnt * (k + 1) / 4) - 1;
-                    blk.cand.what[4 * threadIdx.x + k] = blk.list.what[threadIdx.x];
-                }
-            __syncthreads();   // the list's readers are done
-            if (threadIdx.x == 0) blk.n_list = 0;
-            __syncthreads();
-            nc = 4 * left;
-            per = (per + 3) / 4 + 1;
-        }
+        path_run<kEsdf, false>(
+            M, md, sc, sv, ps, margin, self, blk, G, false,
+            [&](int, int i, float& ai, float& bi) {
+                ai = __ldg(a + i);
+                bi = __ldg(b + i);
+            },
+            []() { return false; }, [](const PathItem&) {});
         if (threadIdx.x == 0) {
             const bool bad = blk.hit != 0;
             valid[e] = bad ? 0 : 1;

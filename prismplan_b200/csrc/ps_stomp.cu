@@ -380,19 +380,19 @@ __global__ void stomp_project_kernel(float* __restrict__ theta, const float* __r
 // w_c sum_d theta_d^T R theta_d (stomp.cu:466-500), then the shared
 // bookkeeping.
 __global__ void stomp_bookkeep_kernel(const float* __restrict__ theta, const float* __restrict__ opt_sc,
-                                      const uint8_t* __restrict__ seg_valid, const uint8_t* __restrict__ wp_hit,
-                                      int T, int D, ps_cost_params P, int n_iter, float conv_eps,
+                                      OptVerdict v, int T, int D, ps_cost_params P, int n_iter, float conv_eps,
                                       float time_limit_ms, const unsigned long long* __restrict__ t0,
                                       OptState* __restrict__ state, uint8_t* __restrict__ done,
                                       float* __restrict__ best, int* __restrict__ n_done) {
     extern __shared__ float sh[];   // traj_smooth_block: 2 (T + 12) + blockDim
     const int b = blockIdx.x;
+    if (b == 0 && threadIdx.x == 0) *v.n_list = 0;
     if (done[b]) return;
     const float* th = theta + (size_t)b * T * D;
     const float total = traj_smooth_block([&](int t, int d) { return th[(size_t)t * D + d]; },
                                           [&](int, int, float) {},
                                           [&](int t) { return opt_sc[(size_t)b * T + t]; }, T, D, P, false, sh);
-    opt_bookkeep_block(b, th, total, seg_valid, wp_hit, T, D, n_iter, conv_eps, time_limit_ms, t0, state, done, best,
+    opt_bookkeep_block(b, th, total, v, T, D, n_iter, conv_eps, time_limit_ms, t0, state, done, best,
                        n_done);
 }
 
@@ -517,7 +517,8 @@ extern "C" int ps_stomp_optimize(const ps_model* m, const ps_scene_view* scene, 
 
     opt_band_kernel<<<1, 1, 0, s>>>(T, P->delta_t, o.band);
     stomp_setup_kernel<<<1, 256, 0, s>>>(T, o.band, w.scratch, w.colscale, w.amp, P->noise_scale);
-    opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0);
+    opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0, o.hit_step,
+                                                  o.n_list);
     PS_TRY_CUDA(cudaGetLastError());
 
     // rollouts per block of the rollouts kernel: up to 8, within 96 KiB of
@@ -567,10 +568,11 @@ extern "C" int ps_stomp_optimize(const ps_model* m, const ps_scene_view* scene, 
         stomp_project_kernel<<<B * D, 64, pj_smem, q>>>(theta, w.delta, o.band, w.colscale, B, T, D, o.state, o.done);
         PS_TRY_CUDA(cudaGetLastError());
         if (int rc = traj_cost_launch(m, scene, theta, B, T, &cp, w.opt_sc, nullptr, nullptr, o.done, q)) return rc;
+        OptVerdict v;
         if (int rc = opt_validity(m, scene, theta, B, T, D, P->collision_margin, P->check_self,
-                                  P->collision_check_step, o, q))
+                                  P->collision_check_step, o, v, q))
             return rc;
-        stomp_bookkeep_kernel<<<B, bk_threads, bk_smem, q>>>(theta, w.opt_sc, o.evalid, o.hit, T, D, cp_total,
+        stomp_bookkeep_kernel<<<B, bk_threads, bk_smem, q>>>(theta, w.opt_sc, v, T, D, cp_total,
                                                              P->num_iterations, P->convergence_eps, P->time_limit_ms,
                                                              o.t0, o.state, o.done, best, o.n_done);
         PS_TRY_CUDA(cudaGetLastError());
