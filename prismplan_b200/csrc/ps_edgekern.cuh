@@ -28,8 +28,9 @@ struct EdgeWs {                         // header of the persistent workspace (6
     int self_edges;                     // edges with at least one sample
     int self_next;                      // next window of the self pass
     int wp_next;                        // next waypoint group (the batch's work-queue kernel)
-    int n_long;                         // edges with more than one chunk round (the long list)
-    int pad[2];
+    int n_long;                         // edges with more than one chunk round (the long list); without the
+                                        // list, the most rounds of any edge when long ones go by units
+    int probed, probed_hit;             // long edges probed, and those that the probe retired
 };
 static_assert(sizeof(EdgeWs) == 64, "the workspace header is 64 B");
 
@@ -58,13 +59,9 @@ struct ChunkOrder {
     __device__ __forceinline__ int chunk(int k) const { return (k % m) * s + k / m; }
 };
 
-// Samples per work unit of an edge with G samples: one chunk, or (coarse, see
-// process_coarse) the four chunks that one coarse pass covers.
 constexpr int kStride = 4;                    // samples per lane of a coarse pass
+constexpr int kCoarseUnit = 32 * kStride;     // samples of a coarse unit
 constexpr int kCoarseMin = 256;               // fewest samples of an edge in coarse units
-__device__ __forceinline__ int edge_unit(int G, bool coarse) {
-    return coarse && G >= kCoarseMin ? 32 * kStride : 32;
-}
 
 __device__ __forceinline__ int ordered_float(float f) {
     int i = __float_as_int(f);
@@ -463,9 +460,9 @@ __device__ bool process_chunk_fast(const ModelSmem& M, const SceneSmem& sc, cons
 // lane whose widened spheres meet nothing has shown its samples free; the
 // chunks of the other lanes are checked sample by sample (process_chunk_fast),
 // so no verdict changes. One pass costs about as much as one chunk and covers
-// four. Most of what it costs beyond a chunk is the wider candidate lists:
-// with 8 samples per lane the same batch (65,536 edges, 47 % free) took 654 us
-// instead of 525.
+// four: 65,536 uneven edges among 64 boxes, 71 % of them free, 932 -> 548 us.
+// Most of what it costs beyond a chunk is the wider candidate lists: with 8
+// samples per lane a batch with 47 % free edges took 654 us instead of 525.
 //
 // The motion bound, per node spacing (kStride samples): the joint's bound
 // centre c moves d = |c - c of the next lane| between nodes (the previous one
@@ -477,7 +474,7 @@ __device__ bool process_chunk_fast(const ModelSmem& M, const SceneSmem& sc, cons
 // on either side (__sinf / __cosf included, for |q| <= kCoarseMaxQ).
 constexpr float kCoarseMaxQ = 16.0f;
 
-// Returns the lanes (bit i: samples unit * 128 + 4 i + 1 .. + 4) that were not
+// Returns the lanes (bit i: samples unit * kCoarseUnit + 4 i + 1 .. + 4) that were not
 // shown free. Lane 0 of unit 0 also stands for the start configuration when
 // G % 16 != 0. Every lane of the warp calls it.
 template <bool kStats>
@@ -486,7 +483,7 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
                                    int unit, WarpScratch ws, LaneStats& st) {
     const int lane = threadIdx.x & 31;
     const int D = M.H->n_dof, NJ = M.H->n_joints;
-    const int j0 = unit * 32 * kStride;
+    const int j0 = unit * kCoarseUnit;
     const int nv = min(32, (G - j0 + kStride - 1) / kStride);   // lanes with samples
     const unsigned valid = nv >= 32 ? kFull : (1u << nv) - 1u;
     const int node = min(lane, nv - 1);   // a lane past the end repeats the last node
@@ -637,7 +634,8 @@ __device__ __forceinline__ bool process_unit(const ModelSmem& M, const SceneSmem
     unsigned chunks = 1u;   // chunks of the unit to check sample by sample
     int first = unit;
     bool last = false;      // the start configuration, which rides with the edge's last chunk
-    if (edge_unit(G, true) > 32) {
+    if (unit < 0) {   // ~unit of a long edge; else a chunk
+        unit = ~unit;
         left = process_coarse<kStats>(M, sc, P, from, to, e, G, unit, ws, st);
         if (!left) return false;
         first = unit * kStride;
@@ -778,12 +776,12 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode ? 6 : 3) edges_plain_kerne
 __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float* __restrict__ from,
                                            const float* __restrict__ to, const int* __restrict__ given,
                                            int n_edges, int D, EdgeWs* hdr, int* G_out, float* len_out, int* bad,
-                                           int* clr, int* done, int* lst, bool coarse) {
+                                           int* clr, int* done, int* lst) {
     if (blockIdx.x == 0 && threadIdx.x == 0)
         hdr->deadline = P.time_budget_ms > 0.0f
                             ? global_ns() + (unsigned long long)((double)P.time_budget_ms * 1.0e6) + 1ull
                             : 0ull;
-    int local_max = 0, local_ne = 0;
+    int local_max = 0, local_ne = 0, local_units = 0;
     unsigned long long local_ns = 0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x) {
         const float* a = from + (size_t)e * D;
@@ -795,8 +793,9 @@ __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float*
         bad[e] = 0;
         clr[e] = ordered_float(FLT_MAX);
         done[e] = 0;
-        const int rounds = ChunkOrder(G, edge_unit(G, coarse)).rounds();
+        const int rounds = ChunkOrder(G).rounds();
         local_max = max(local_max, rounds);
+        if (!lst) local_units = max(local_units, G >= kCoarseMin ? ChunkOrder(G, kCoarseUnit).rounds() : rounds);
         local_ns += (unsigned long long)(G + ((G % 16) != 0 ? 1 : 0));
         local_ne += G > 0;
         if (lst) {   // one atomic per group of converged lanes
@@ -816,6 +815,10 @@ __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float*
         local_ne += __shfl_xor_sync(kFull, local_ne, o);
     }
     if ((threadIdx.x & 31) == 0 && local_max > 0) atomicMax(&hdr->max_rounds, local_max);
+    if (!lst) {
+        local_units = __reduce_max_sync(kFull, local_units);
+        if ((threadIdx.x & 31) == 0 && local_units > 0) atomicMax(&hdr->n_long, local_units);
+    }
     if ((threadIdx.x & 31) == 0 && P.check_self && local_ns > 0) {
         atomicAdd(&hdr->self_samples, local_ns);
         atomicAdd(&hdr->self_edges, local_ne);
@@ -825,9 +828,9 @@ __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float*
 __global__ void edges_prep_kernel(ps_edge_params P, const float* __restrict__ from, const float* __restrict__ to,
                                   const int* __restrict__ given, int n_edges, int D, EdgeWs* hdr, int* G_out,
                                   float* len_out, int* bad, int* clr, int* done, const int* n_dev = nullptr,
-                                  int* lst = nullptr, bool coarse = false) {
+                                  int* lst = nullptr) {
     if (n_dev) n_edges = *n_dev;
-    prep_edges(P, from, to, given, n_edges, D, hdr, G_out, len_out, bad, clr, done, lst, coarse);
+    prep_edges(P, from, to, given, n_edges, D, hdr, G_out, len_out, bad, clr, done, lst);
 }
 
 // ---------------------------------------------------------------------------
@@ -968,7 +971,6 @@ struct PrepArgs {
     int* clr;
     int* done;
     int* lst;   // the long list, or nullptr
-    bool coarse;
 };
 
 template <bool kStats, bool kPrep>
@@ -983,7 +985,7 @@ __global__ void __launch_bounds__(kProbeThreads, 4) edges_probe_kernel(ModelDev 
     if (n_edges <= 0) return;
     if (kPrep) {
         const int D = reinterpret_cast<const BlobHeader*>(md.blob)->n_dof;
-        prep_edges(P, from, to, pa.given, n_edges, D, hdr, Gs, pa.len, bad, pa.clr, pa.done, pa.lst, pa.coarse);
+        prep_edges(P, from, to, pa.given, n_edges, D, hdr, Gs, pa.len, bad, pa.clr, pa.done, pa.lst);
     }
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
@@ -1009,6 +1011,7 @@ __global__ void __launch_bounds__(kProbeThreads, 4) edges_probe_kernel(ModelDev 
     const unsigned long long deadline = *((volatile unsigned long long*)&hdr->deadline);
     LaneStats st;
     st.zero();
+    int n_long = 0, n_hit = 0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x) {
         const int G = Gs[e];
         if (G <= 0) continue;
@@ -1021,7 +1024,18 @@ __global__ void __launch_bounds__(kProbeThreads, 4) edges_probe_kernel(ModelDev 
             qc[i] = __fmaf_rn(t, __fadd_rn(bi, -ai), ai);
         }
         if (kStats) st.v[ST_SAMPLES] += 1;
-        if (lane_probe_hit<kStats>(M, sc, obs, cand, qc, P.collision_margin, st)) bad[e] = 1;
+        const bool hit = lane_probe_hit<kStats>(M, sc, obs, cand, qc, P.collision_margin, st);
+        if (hit) bad[e] = 1;
+        n_long += G >= kCoarseMin;
+        n_hit += hit && G >= kCoarseMin;
+    }
+    if (kPrep) {   // see coarse_now
+        n_long = __reduce_add_sync(kFull, n_long);
+        n_hit = __reduce_add_sync(kFull, n_hit);
+        if ((threadIdx.x & 31) == 0 && n_long) {
+            atomicAdd(&hdr->probed, n_long);
+            atomicAdd(&hdr->probed_hit, n_hit);
+        }
     }
     flush_stats(stats, st);
 }
@@ -1065,6 +1079,16 @@ int plan_probe(const ps_model* m, const ps_scene_view* sv, int mode, bool stats,
 
 // kMode: 0 generic, 1 boxes only, 2 boxes and ESDF layers, 3 boxes only with
 // the coarse pass over long edges.
+// Whether the long edges of a batch that may be passed coarsely (coarse_path)
+// are. The pass costs an edge that collides more than chunks do, so it depends
+// on how many long edges the end-sample probe retired: with 11, 16, 23 and 27 %
+// of them the queue took 0.65, 0.67, 0.80 and 0.88 of its time without the
+// pass, with 37, 48, 49 and 59 % 1.08, 1.36, 1.25 and 1.43.
+__device__ __forceinline__ bool coarse_now(const EdgeWs* hdr) {
+    const volatile EdgeWs* h = hdr;
+    return 10ll * h->probed_hit < 3ll * h->probed;
+}
+
 // Residency per variant, measured: the boxes-only fast path runs fastest
 // with 5 blocks per SM (room for 96 registers), the ESDF variant with 6.
 template <int kMode, bool kStats>
@@ -1074,14 +1098,17 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
                                                                   EdgeWs* hdr, const int* __restrict__ Gs, int* bad,
                                                                   int* clr, int* done, unsigned long long* stats,
                                                                   int pass, const int* n_dev = nullptr,
-                                                                  const int* __restrict__ lst = nullptr) {
+                                                                  const int* __restrict__ lst = nullptr,
+                                                                  bool either = false) {
     if (n_dev) n_edges = *n_dev;
+    // either: a launch of mode 1 and one of mode 3, of which one runs
+    if (either && (kMode == 3) != coarse_now(hdr)) return;
     // Rounds of this launch. With many edges per resident warp (>= 8) one
     // launch (pass 0) runs every round and pass 1 returns at once. With fewer,
     // round 1 would start while much of round 0 is still in flight and check
     // chunks of edges that round 0 retires, so pass 0 runs round 0 only and
     // the second launch (pass 1) the rest.
-    const int max_rounds = *((volatile int*)&hdr->max_rounds);
+    const int max_rounds = kMode == 3 ? *((volatile int*)&hdr->n_long) : *((volatile int*)&hdr->max_rounds);
     const bool split = (long long)n_edges < 8ll * gridDim.x * kWarps;
     const int r_lo = pass == 0 ? 0 : (split ? 1 : max_rounds);
     const int r_hi = pass == 0 ? (split ? min(max_rounds, 1) : max_rounds) : max_rounds;
@@ -1161,12 +1188,14 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
                 e = lst ? __ldg(lst + idx) : idx;
             }
             G = __ldg(Gs + e);
-            const ChunkOrder ord(G, edge_unit(G, kMode == 3));
+            const bool units = kMode == 3 && G >= kCoarseMin;   // held as ~unit
+            const ChunkOrder ord(G, units ? kCoarseUnit : 32);
             if (k < ord.rounds()) {
                 k = ord.chunk(k);   // round -> chunk (or unit) index
                 // a retired edge's remaining chunks still count toward the
                 // clearance, which covers every sample (edge_eval.cuh:133-153)
                 live = k < ord.nc && (P.compute_clearance || vbad[e] == 0);
+                if (units) k = ~k;
             }
         }
         unsigned todo = __ballot_sync(kFull, live);
@@ -1342,13 +1371,12 @@ __global__ void edges_finalize_kernel(int n_edges, const ps_edge_params P, const
                                       const float* __restrict__ len, const int* __restrict__ clr,
                                       const int* __restrict__ done, const int* __restrict__ Gs, const EdgeWs* hdr,
                                       uint8_t* __restrict__ valid, float* __restrict__ cost,
-                                      float* __restrict__ clearance, const int* n_dev = nullptr,
-                                      bool coarse = false) {
+                                      float* __restrict__ clearance, const int* n_dev = nullptr) {
     if (n_dev) n_edges = *n_dev;
     const bool timed_out = hdr->timed_out != 0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x) {
         const int bv = bad[e];
-        const bool b = (P.check_self ? bv != 2 : bv != 0) || (timed_out && done[e] < ChunkOrder(Gs[e], edge_unit(Gs[e], coarse)).nc);
+        const bool b = (P.check_self ? bv != 2 : bv != 0) || (timed_out && done[e] < ChunkOrder(Gs[e]).nc);
         valid[e] = b ? 0 : 1;
         cost[e] = b ? FLT_MAX : len[e];
         if (clearance) clearance[e] = P.compute_clearance ? unordered_float(clr[e]) : FLT_MAX;
@@ -1388,16 +1416,23 @@ int fast_path(const ps_model* m, const ps_scene_view* sv, const ps_edge_params* 
     return fast ? (sv->n_voxel_layers > 0 ? 2 : 1) : 0;
 }
 
-// Whether units of long edges are passed coarsely first: rigid models, boxes
-// only, no negative effective radius, and a probe that has left mostly free
-// edges, enough of them to fill the chip with units four chunks long (the
-// queue's one-pass rule). Measured (us, without / with): 65,536 uneven edges
-// among 64 boxes 633 / 525 (47 % free) and 932 / 548 (71 %), among 16 596 /
-// 430 and 985 / 450; 32,768 (no probe, a quarter free) 259 / 411; 30,000
-// two-arm edges by an ESDF 865 / 1529.
-bool coarse_path(const ps_model* m, const ps_edge_params* P, int mode, bool probed, int n_edges, int qgrid) {
-    return mode == 1 && probed && m->rigid && m->min_radius + P->collision_margin >= 0.0f &&
-           (long long)n_edges >= 8ll * qgrid * kWarps;
+// Whether units of long edges may be passed coarsely first (coarse_now decides
+// from the probe): rigid models, boxes only, no time budget (its progress
+// counts chunks), no negative effective radius, the probe, enough edges to fill
+// the chip with units four chunks long (the queue's one-pass rule), and edges
+// that can be long (twice kCoarseMin on the widest joint range). 32,768 edges
+// (no probe, a quarter free) took 411 us with the pass and 259 without, 30,000
+// two-arm edges by an ESDF 1529 and 865.
+bool coarse_path(const ps_model* m, const ps_edge_params* P, const int* given, int mode, bool probed, int n_edges,
+                 int qgrid) {
+    if (mode != 1 || !probed || !m->rigid || P->time_budget_ms > 0.0f || m->min_radius + P->collision_margin < 0.0f)
+        return false;
+    if (!given) {
+        const float step = P->resolution > 0.0f ? P->resolution : P->max_joint_step;
+        const float longest = step > 0.0f ? m->widest / step : (float)P->granularity;
+        if (longest < 2.0f * kCoarseMin) return false;
+    }
+    return (long long)n_edges >= 8ll * qgrid * kWarps;
 }
 
 template <typename K>

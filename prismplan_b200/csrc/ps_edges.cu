@@ -150,30 +150,31 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
     // rounds (a CHOMP loop's 16 K short segments: 34.7 -> 29.9 ms per call).
     // With many, one pass runs every round over every edge, as before.
     const bool split = (long long)n_edges < 8ll * qgrid * kEdgeThreads / 32;   // the kernel's own split rule
-    int* lst = split ? b.lst : nullptr;
     ProbePlan probe;
     if (int rc = plan_probe(m, scene, mode, g_stats != nullptr, 1.0f, n_edges, P->probe, probe)) return rc;
-    const bool coarse = coarse_path(m, P, mode, probe.kp != nullptr, n_edges, qgrid);
-    if (coarse) {
-        qk = g_stats ? edges_queue_kernel<3, true> : edges_queue_kernel<3, false>;   // same shared memory and residency
-        PS_TRY_CUDA(allow_smem((const void*)qk, smem));
-    }
+    const bool coarse = coarse_path(m, P, samples_per_edge, mode, probe.kp != nullptr, n_edges, qgrid);
+    auto qk3 = g_stats ? edges_queue_kernel<3, true> : edges_queue_kernel<3, false>;   // shared memory and residency as qk
+    if (coarse) PS_TRY_CUDA(allow_smem((const void*)qk3, smem));
+    int* lst = split ? b.lst : nullptr;
     if (!probe.kp) {   // with the probe, its launch also prepares the edges
         const int pgrid = std::max(1, std::min((n_edges + 255) / 256, sm_count() * 4));
         edges_prep_kernel<<<pgrid, 256, 0, s>>>(*P, from, to, samples_per_edge, n_edges, D, b.hdr, b.G, b.len, b.bad,
-                                                b.clr, b.done, nullptr, lst, coarse);
+                                                b.clr, b.done, nullptr, lst);
         PS_TRY_CUDA(cudaGetLastError());
     }
     mark_start(s);
     if (probe.kp)
         probe.kp<<<probe.grid, kProbeThreads, probe.smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G,
                                                                 b.bad, g_stats, nullptr,
-                                                                PrepArgs{samples_per_edge, b.len, b.clr, b.done, lst, coarse});
+                                                                PrepArgs{samples_per_edge, b.len, b.clr, b.done, lst});
     qk<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
-                                         g_stats, 0, nullptr, lst);
+                                         g_stats, 0, nullptr, lst, coarse);
+    if (coarse)   // one pass (not split); the probe's counts say which of the two runs
+        qk3<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
+                                              g_stats, 0, nullptr, lst, true);
     if (split)
         qk<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
-                                             g_stats, 1, nullptr, lst);
+                                             g_stats, 1, nullptr, lst, false);
     mark_stop(s);
     PS_TRY_CUDA(cudaGetLastError());
     if (int rc = launch_edges_self(m, P, from, to, samples_per_edge, n_edges, b.G, b.bad, nullptr, nullptr, b.hdr,
@@ -181,7 +182,7 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
         return rc;
     const int fgrid = std::max(1, std::min((n_edges + 255) / 256, sm_count() * 4));
     edges_finalize_kernel<<<fgrid, 256, 0, s>>>(n_edges, *P, b.bad, b.len, b.clr, b.done, b.G, b.hdr, valid, cost,
-                                                clearance, nullptr, coarse);
+                                                clearance);
     PS_TRY_CUDA(cudaGetLastError());
     return PS_OK;
 }

@@ -17,6 +17,7 @@ struct ps_model {
     int max_joint_spheres = 0;  // most exact spheres on one joint
     bool root_slot_only = false; // slot 0 holds only the root (identity) frame
     bool rigid = false;         // every fixed transform is a rotation and a translation (to 2e-5)
+    float widest = 0.0f;        // widest joint range (upper - lower) at creation
     float min_radius = 0.0f;    // least radius of the exact and approximate spheres
     int max_joint_approx = 0;
     std::vector<int> sph_orig;  // reordered -> descriptor index (host copy)

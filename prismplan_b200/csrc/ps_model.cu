@@ -529,6 +529,7 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     m->min_radius = ns + na > 0 ? 3.0e38f : 0.0f;
     for (int s = 0; s < ns; ++s) m->min_radius = std::min(m->min_radius, d->spheres[4 * s + 3]);
     for (int a = 0; a < na; ++a) m->min_radius = std::min(m->min_radius, d->approx_spheres[4 * a + 3]);
+    for (int k = 0; k < nd; ++k) m->widest = std::max(m->widest, d->joint_upper[k] - d->joint_lower[k]);
     m->rigid = true;
     for (int p = 1; p < nj; ++p) {
         const float* f = d->fixed_transforms + 16 * dfs[p];

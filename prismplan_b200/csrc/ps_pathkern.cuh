@@ -279,16 +279,17 @@ __device__ __forceinline__ unsigned path_sweep(const ModelSmem& M, const ModelDe
 struct PathItem {
     int seg, lo, hi, what;
 };
-constexpr int kPathStack = 256;
+constexpr int kPathBatch = 4 * kPathGroups;   // intervals swept before the samples of those left
+constexpr int kPathStack = 512;
 struct PathBlock {
     int hit;          // a sample collides
     int n_stack;      // intervals still to sweep
     int n_list;       // intervals of this pass that the swept check left
     int n_samples;    // samples they hold (saturated)
-    PathItem list[kPathGroups], stack[kPathStack];
+    PathItem list[kPathBatch], stack[kPathStack];
 };
 
-// Works through the intervals on blk.stack, 32 at a time from the top, until
+// Works through the intervals on blk.stack, up to 128 at a time from the top, until
 // one sample hits, stop() says that the answer no longer matters, or nothing
 // is left: the swept check (skipped for single samples), then for the
 // intervals that it leaves every sample if they are few, else the middle ones
@@ -314,40 +315,42 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
     LaneStats st;
     st.zero();
     for (bool begin = true;; begin = false) {
-        const int ns = blk.n_stack, nc = min(ns, kPathGroups);
+        const int ns = blk.n_stack, nc = min(ns, kPathBatch);
         if (nc == 0) break;   // uniform
-        // ---- swept check of the top intervals, a group each ----
-        const PathItem it = blk.stack[ns - 1 - min(slot, nc - 1)];   // a group past the end repeats the last one
-        const bool single = it.lo == it.hi;
-        __syncthreads();   // the stack's and the last pass' readers are done
+        __syncthreads();      // n_stack's and the last pass' readers are done
         if (threadIdx.x == 0) {
             blk.n_stack = ns - nc;
             blk.n_list = blk.n_samples = 0;
         }
-        unsigned bits = (unsigned)it.what;
-        if (!__all_sync(kGrpFull, single)) {   // uniform
-            const int lo = min(it.lo, G), hi = min(it.hi, G);
-            const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
-                        th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
-            bool ok = !single;   // a single sample is checked itself
-            __syncwarp();
-            for (int i = 0; i < D; ++i) {
-                float a, b;
-                point(it.seg, i, a, b);
-                ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
-                if ((i & (kSub - 1)) == u) {
-                    qc[i] = fmaf(tm, b - a, a);
-                    dq[i] = th * (b - a);
+        __syncthreads();
+        // ---- swept check of the top intervals, a group each ----
+        for (int k0 = 0; k0 < nc; k0 += kPathGroups) {
+            const PathItem it = blk.stack[ns - 1 - min(k0 + slot, nc - 1)];   // a group past the end repeats the last one
+            const bool single = it.lo == it.hi;
+            unsigned bits = (unsigned)it.what;
+            if (!__all_sync(kGrpFull, single)) {   // uniform
+                const int lo = min(it.lo, G), hi = min(it.hi, G);
+                const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
+                            th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
+                bool ok = !single;   // a single sample is checked itself
+                __syncwarp();
+                for (int i = 0; i < D; ++i) {
+                    float a, b;
+                    point(it.seg, i, a, b);
+                    ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
+                    if ((i & (kSub - 1)) == u) {
+                        qc[i] = fmaf(tm, b - a, a);
+                        dq[i] = th * (b - a);
+                    }
                 }
+                __syncwarp();
+                bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
             }
-            __syncwarp();
-            bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
-        }
-        __syncthreads();   // the list is empty
-        if (u == 0 && slot < nc && bits) {   // in any order
-            const int k = atomicAdd(&blk.n_list, 1);
-            blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
-            atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
+            if (u == 0 && k0 + slot < nc && bits) {   // in any order
+                const int k = atomicAdd(&blk.n_list, 1);
+                blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
+                atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
+            }
         }
         __syncthreads();
         const int n = blk.n_list;
