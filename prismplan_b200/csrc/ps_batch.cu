@@ -61,14 +61,15 @@ __global__ void batch_gather_edges(const EdgeReq* __restrict__ req, const Counts
                                    ps_edge_params P, int D, float* __restrict__ from, float* __restrict__ to,
                                    int* __restrict__ G) {
     const int nreq = cnt->n_edge_req;
+    const int lo = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;   // slices of a request
     for (int r = blockIdx.x; r < nreq; r += gridDim.x) {
         const EdgeReq q = req[r];
         const size_t base = (size_t)q.offset * D;
-        for (int i = threadIdx.x; i < q.n * D; i += blockDim.x) {
+        for (int i = lo; i < q.n * D; i += step) {
             from[base + i] = q.from[i];
             to[base + i] = q.to[i];
         }
-        for (int i = threadIdx.x; i < q.n; i += blockDim.x) {
+        for (int i = lo; i < q.n; i += step) {
             const float* a = q.from + (size_t)i * D;
             const float* b = q.to + (size_t)i * D;
             G[q.offset + i] = edge_samples(P, q.samples, i, a, b, D, edge_length(a, b, D));
@@ -93,14 +94,15 @@ __global__ void batch_scatter_edges(const EdgeReq* __restrict__ req, const Count
 __global__ void batch_gather_traj(const TrajReq* __restrict__ req, const Counts* __restrict__ cnt, int D,
                                   float* __restrict__ q) {
     const int nreq = cnt->n_traj_req;
+    const int lo = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;   // slices of a request
     for (int r = blockIdx.x; r < nreq; r += gridDim.x) {
         const TrajReq t = req[r];
         const size_t base = (size_t)t.offset * D;
         if (!t.rollouts) {
-            for (int i = threadIdx.x; i < t.T * D; i += blockDim.x) q[base + i] = t.q[i];
+            for (int i = lo; i < t.T * D; i += step) q[base + i] = t.q[i];
         } else {
             const long long n = (long long)t.rows * t.T * D;
-            for (long long i = threadIdx.x; i < n; i += blockDim.x) {   // i over the packed rows
+            for (long long i = lo; i < n; i += step) {   // i over the packed rows
                 const int d = (int)(i % D);
                 const long long w = i / D;
                 const int row = (int)(w / t.T), tt = (int)(w - (long long)row * t.T);
@@ -467,8 +469,16 @@ struct LaunchPlan {
                  EdgeWs*, const int*, int*, int*, int*, const float*, float*, float*, int, int, int) = nullptr;
     size_t qsmem = 0, wsmem = 0, fsmem = 0, ssmem = 0, ksmem = 0;
     int qgrid = 1, wgrid = 1, req_grid_e = 1, req_grid_t = 1, pgrid = 1, sgrid = 1, kgrid = 1;
+    int slices_e = 1, slices_t = 1;   // blocks a request in the gathers
     ProbePlan probe;
 };
+
+// Blocks that share a request in the gathers, which wait for each thread's
+// serial loads: a batch of few requests spreads each over up to 16 blocks
+// (four rollout requests of 640 waypoints by 14 joints and eight trajectories
+// of 80: 32.5 us with a block each, 4.4 us; twelve edge requests 6.8 and
+// 2.9 us), and one of more than 296 fills the device with a block each.
+int request_slices(int grid) { return std::max(1, std::min(16, 4 * sm_count() / std::max(grid, 1))); }
 
 using WorkKernel = decltype(LaunchPlan::work);
 
@@ -503,6 +513,7 @@ int plan_launch(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep, 
         if (int rc = plan_probe(m, sv, L.mode, false, b->edge_share, b->lim.max_edges, ep->probe, L.probe)) return rc;
         L.pgrid = std::max(1, std::min((b->lim.max_edges + 255) / 256, sms * 4));
         L.req_grid_e = std::max(1, std::min(b->lim.max_edge_requests, sms * 8));
+        L.slices_e = request_slices(L.req_grid_e);
         if (ep->check_self) {
             if (int rc = check_self_fits(m)) return rc;
             L.ssmem = self_lane_smem_bytes(m);
@@ -529,6 +540,7 @@ int plan_launch(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep, 
         if (L.fsmem > 48 * 1024)
             PS_TRY_CUDA(allow_smem((const void*)batch_traj_finish, L.fsmem));
         L.req_grid_t = std::max(1, std::min(b->lim.max_traj_requests, sms * 8));
+        L.slices_t = request_slices(L.req_grid_t);
     }
     if (b->layout == 1) {   // one work-queue kernel for edge chunks and waypoint groups
         const int mode = b->lim.max_edges > 0 ? L.mode : 1;
@@ -557,7 +569,8 @@ void record_work_graph(ps_batch* b, const ps_scene_view* sv, const ps_edge_param
     const bool edges = b->lim.max_edges > 0, trajs = b->lim.max_waypoints > 0;
     cudaMemsetAsync(b->d_hdr, 0, sizeof(EdgeWs), s0);
     if (edges) {
-        batch_gather_edges<<<L.req_grid_e, 128, 0, s0>>>(b->d_ereq, b->d_cnt, *ep, D, b->d_from, b->d_to, b->d_given);
+        batch_gather_edges<<<dim3(L.req_grid_e, L.slices_e), 128, 0, s0>>>(b->d_ereq, b->d_cnt, *ep, D, b->d_from, b->d_to,
+                                                                        b->d_given);
         edges_prep_kernel<<<L.pgrid, 256, 0, s0>>>(*ep, b->d_from, b->d_to, b->d_given, b->lim.max_edges, D, b->d_hdr,
                                                    b->d_G, b->d_len, b->d_bad, b->d_clr, b->d_done, n_dev);
         if (L.probe.k)
@@ -565,7 +578,7 @@ void record_work_graph(ps_batch* b, const ps_scene_view* sv, const ps_edge_param
                                                                           b->lim.max_edges, b->d_hdr, b->d_G,
                                                                           b->d_bad, nullptr, n_dev, PrepArgs{});
     }
-    if (trajs) batch_gather_traj<<<L.req_grid_t, 128, 0, s0>>>(b->d_treq, b->d_cnt, D, b->d_q);
+    if (trajs) batch_gather_traj<<<dim3(L.req_grid_t, L.slices_t), 128, 0, s0>>>(b->d_treq, b->d_cnt, D, b->d_q);
     for (int pass = 0; pass < 2; ++pass)
         L.work<<<L.kgrid, b->work_threads, L.ksmem, s0>>>(m->dev, *sv, *ep, *cp, b->d_cnt, b->d_from, b->d_to,
                                                           b->d_hdr, b->d_G, b->d_bad, b->d_clr, b->d_done, b->d_q,
@@ -604,7 +617,8 @@ void record_graph(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep
     if (b->lim.max_edges > 0) {   // edge branch on s0
         const int* n_dev = &b->d_cnt->n_edges;
         cudaMemsetAsync(b->d_hdr, 0, sizeof(EdgeWs), s0);
-        batch_gather_edges<<<L.req_grid_e, 128, 0, s0>>>(b->d_ereq, b->d_cnt, *ep, D, b->d_from, b->d_to, b->d_given);
+        batch_gather_edges<<<dim3(L.req_grid_e, L.slices_e), 128, 0, s0>>>(b->d_ereq, b->d_cnt, *ep, D, b->d_from, b->d_to,
+                                                                        b->d_given);
         edges_prep_kernel<<<L.pgrid, 256, 0, s0>>>(*ep, b->d_from, b->d_to, b->d_given, b->lim.max_edges, D, b->d_hdr,
                                                    b->d_G, b->d_len, b->d_bad, b->d_clr, b->d_done, n_dev);
         if (L.probe.k)
@@ -626,7 +640,7 @@ void record_graph(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep
         batch_scatter_edges<<<L.req_grid_e, 128, 0, s0>>>(b->d_ereq, b->d_cnt, b->d_valid, b->d_cost);
     }
     if (b->lim.max_waypoints > 0) {   // trajectory branch on s1
-        batch_gather_traj<<<L.req_grid_t, 128, 0, s1>>>(b->d_treq, b->d_cnt, D, b->d_q);
+        batch_gather_traj<<<dim3(L.req_grid_t, L.slices_t), 128, 0, s1>>>(b->d_treq, b->d_cnt, D, b->d_q);
         L.wk<<<L.wgrid, b->traj_threads, L.wsmem, s1>>>(m->dev, *sv, *cp, b->d_cnt, b->d_q, b->d_wp_cost, b->d_grad,
                                                         b->lim.max_waypoints);
         batch_traj_finish<<<L.req_grid_t, kFinishThreads, L.fsmem, s1>>>(b->d_treq, b->d_cnt, D, *cp, b->d_q,
