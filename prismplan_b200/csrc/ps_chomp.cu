@@ -166,7 +166,7 @@ extern "C" int ps_chomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     ps_cost_params cp_total = cp;
     cp_total.smoothness_weight = P->smoothness_weight;
 
-    opt_band_kernel<<<1, 1, 0, s>>>(T, P->delta_t, o.band);
+    opt_band_kernel<<<1, kBandThreads, 0, s>>>(T, P->delta_t, o.band);
     opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0, o.hit_step,
                                                   o.n_list);
     PS_TRY_CUDA(cudaGetLastError());

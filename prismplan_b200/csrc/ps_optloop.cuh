@@ -38,9 +38,13 @@ __device__ __forceinline__ unsigned long long now_ns() {
 // R (central T x T block of dt A^T A over the 6-padded 5-point acceleration
 // stencil, chomp_precompute.cpp:20-37, stomp_precompute.cpp:24-42) + 1e-8 I,
 // factored as L L^T with L lower-banded: L[i * 5 + k] = L(i, i - k) for
-// k = 1..4 and L[i * 5] = 1 / L(i, i). FP64, one thread.
-__global__ void opt_band_kernel(int T, float dt_f, double* __restrict__ L) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+// k = 1..4 and L[i * 5] = 1 / L(i, i). FP64. One block: its threads compute
+// the entries of R, kBandRows rows at a time in shared memory, and thread 0
+// factors them with the last kBand rows of L in registers (T = 64: 127 us in
+// one thread over global memory, now 13 us).
+constexpr int kBandThreads = 128, kBandRows = 64;
+__global__ void __launch_bounds__(kBandThreads) opt_band_kernel(int T, float dt_f, double* __restrict__ L) {
+    __shared__ double rows[kBandRows * 5];
     const double dt = dt_f, inv_dt2 = 1.0 / (dt * dt);
     const double coeff[7] = {0.0, -1.0 / 12.0, 16.0 / 12.0, -30.0 / 12.0, 16.0 / 12.0, -1.0 / 12.0, 0.0};
     const int pad = 6, Np = T + 12;
@@ -54,13 +58,38 @@ __global__ void opt_band_kernel(int T, float dt_f, double* __restrict__ L) {
         for (int r = max(max(ci, cj) - 3, 0); r <= min(min(ci, cj) + 3, Np - 1); ++r) s += A(r, ci) * A(r, cj);
         return dt * s + (i == j ? 1.0e-8 : 0.0);
     };
-    for (int i = 0; i < T; ++i) {
-        for (int j = max(0, i - kBand); j <= i; ++j) {
-            double s = R(i, j);
-            for (int k = max(0, i - kBand); k < j; ++k) s -= L[i * 5 + (i - k)] * L[j * 5 + (j - k)];
-            if (i == j) L[i * 5] = 1.0 / sqrt(s > 0.0 ? s : 1.0e-300);
-            else L[i * 5 + (i - j)] = s * L[j * 5];
+    double w[kBand][5] = {};   // w[m]: row i - 1 - m of L (zero above the matrix)
+    for (int i0 = 0; i0 < T; i0 += kBandRows) {
+        const int n = min(kBandRows, T - i0);
+        for (int e = threadIdx.x; e < n * 5; e += blockDim.x) {
+            const int i = i0 + e / 5, k = e % 5;
+            rows[e] = k <= i ? R(i, i - k) : 0.0;
         }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = 0; i < n; ++i) {
+                double c[5];   // L(i, i - k), k = 1..4, then 1 / L(i, i)
+#pragma unroll
+                for (int k = kBand; k >= 0; --k) {
+                    double s = rows[i * 5 + k];
+#pragma unroll
+                    for (int m = kBand; m > k; --m) s -= c[m] * (k ? w[k - 1][m - k] : c[m]);
+                    c[k] = k ? s * w[k - 1][0] : 1.0 / sqrt(s > 0.0 ? s : 1.0e-300);
+                }
+#pragma unroll
+                for (int m = kBand - 1; m > 0; --m)
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) w[m][k] = w[m - 1][k];
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    w[0][k] = c[k];
+                    rows[i * 5 + k] = c[k];
+                }
+            }
+        __syncthreads();
+        for (int e = threadIdx.x; e < n * 5; e += blockDim.x)
+            if (e % 5 <= i0 + e / 5) L[(size_t)i0 * 5 + e] = rows[e];
+        __syncthreads();
     }
 }
 

@@ -74,13 +74,17 @@ __device__ __forceinline__ void band_back(const double* Ls, double* x, int T) { 
 // Column scales of M and the noise amplitude (stomp_precompute.cpp:46-94):
 // with Rinv = (R + 1e-8 I)^-1, s_j = (1/T) / max_i Rinv(i, j) and
 // sqrt_c = noise_scale * sqrt((1/T) / max_ij Rinv(i, j)). One thread per
-// column of Rinv (a banded solve of e_j into scratch [T][T]). FP64.
+// column of Rinv (a banded solve of e_j), in shared memory at an odd stride
+// while the columns fit there (T = 51: 40 us over rows of scratch [T][T] in
+// global memory, 12.9 us). FP64.
 __global__ void stomp_setup_kernel(int T, const double* __restrict__ band, double* __restrict__ scratch,
-                                   double* __restrict__ colscale, double* __restrict__ amp, float noise_scale) {
+                                   double* __restrict__ colscale, double* __restrict__ amp, float noise_scale,
+                                   bool shared) {
+    extern __shared__ double cols[];
     __shared__ double red[256];
     double gmax = -INFINITY;
     for (int j = threadIdx.x; j < T; j += blockDim.x) {
-        double* x = scratch + (size_t)j * T;
+        double* x = shared ? cols + (size_t)j * (T | 1) : scratch + (size_t)j * T;
         for (int i = 0; i < T; ++i) x[i] = (i == j) ? 1.0 : 0.0;
         band_solve(band, x, T);
         double mx = -INFINITY;
@@ -106,8 +110,11 @@ __device__ __forceinline__ bool stomp_active(const OptState* state, const uint8_
 
 // Per request: the num_rollouts_old lowest row totals of the previous
 // iteration, by the reference's selection (stomp.cu:133-152: repeated
-// first-minimum scan, each pick masked with 3e38). Thread 0; the totals
-// staged in shared memory.
+// first-minimum scan, each pick masked with 3e38). Each thread ranks its
+// totals by (value, place), which is the scan's order as long as it finds
+// enough totals below the mask and entry 0, where it starts, is a number;
+// otherwise thread 0 scans (20 of 51: 8.6 us by the scan, 2.9 us by ranks).
+constexpr int kTopkThreads = 128;
 __global__ void stomp_topk_kernel(const float* __restrict__ tot_prev, int* __restrict__ topk, int R, int Ro, int B,
                                   const OptState* __restrict__ state, const uint8_t* __restrict__ done) {
     extern __shared__ float cc[];   // [R]
@@ -115,6 +122,19 @@ __global__ void stomp_topk_kernel(const float* __restrict__ tot_prev, int* __res
     if (Ro == 0 || !stomp_active(state, done, b) || state[b].step == 1) return;
     for (int r = threadIdx.x; r < R; r += blockDim.x) cc[r] = tot_prev[(size_t)r * B + b];
     __syncthreads();
+    int below = 0;   // totals below the mask
+#pragma unroll 4
+    for (int i = 0; i < R; ++i) below += cc[i] < 3.0e38f;
+    if (below >= Ro && cc[0] == cc[0]) {   // the same in every thread
+        for (int r = threadIdx.x; r < R; r += blockDim.x) {
+            const float v = cc[r];
+            int rank = 0;
+#pragma unroll 4
+            for (int i = 0; i < R; ++i) rank += cc[i] < v || (cc[i] == v && i < r);
+            if (v < 3.0e38f && rank < Ro) topk[(size_t)b * Ro + rank] = r;
+        }
+        return;
+    }
     if (threadIdx.x != 0) return;
     for (int k = 0; k < Ro; ++k) {
         int bi = 0;
@@ -278,75 +298,82 @@ __global__ void stomp_row_totals_kernel(const float* __restrict__ roll_cur, cons
     if (threadIdx.x == 0) tot_cur[row] = red[0];
 }
 
-// One thread per (request, t, d): over the R rollouts, cost
+// One block per 32 entries (t, d) of a request: over the R rollouts, cost
 // c_r = state_r,t + control_r,t,d, weights p_r = exp(-h (c_r - min) /
 // max(max - min, 1e-8)) / max(sum, 1e-12) (stomp.cu:314-355), and the
 // weighted noise delta = sum_r p_r noise_r, 0 at the endpoints
-// (stomp.cu:360-385).
-__global__ void stomp_weights_kernel(const float* __restrict__ sc_cur, const float* __restrict__ ctrl,
-                                     const float* __restrict__ noise, float* __restrict__ delta, int B, int T, int D,
-                                     int R, float h, const OptState* __restrict__ state,
-                                     const uint8_t* __restrict__ done) {
-    const long long n = (long long)B * T * D;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(idx / ((long long)T * D));
-        const int rem = (int)(idx - (long long)b * T * D);
-        const int t = rem / D;
-        if (!stomp_active(state, done, b)) continue;
+// (stomp.cu:360-385). Lanes are entries; the block's warps share the rollouts
+// for the loads, exponentials and quotients, kWeightRolls at a time through
+// shared memory, and warp 0 adds each entry's terms in rollout order. With one
+// thread an entry, a call of 16 requests, 51 waypoints by 7 joints and 51
+// rollouts had 179 warps on the device, each through three serial passes:
+// 22.4 us, now 5.5 us.
+constexpr int kWeightWarps = 8, kWeightRolls = 64;
+__global__ void __launch_bounds__(kWeightWarps * 32) stomp_weights_kernel(
+    const float* __restrict__ sc_cur, const float* __restrict__ ctrl, const float* __restrict__ noise,
+    float* __restrict__ delta, int B, int T, int D, int R, float h, const OptState* __restrict__ state,
+    const uint8_t* __restrict__ done) {
+    __shared__ float cs[kWeightRolls][32], zs[kWeightRolls][32], lo[kWeightWarps][32], hi[kWeightWarps][32], tot[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int TD = T * D, tiles = (TD + 31) / 32;
+    const bool once = R <= kWeightRolls;   // every rollout's terms stay in shared memory
+    for (int item = blockIdx.x; item < B * tiles; item += gridDim.x) {
+        const int b = item / tiles, e = (item - b * tiles) * 32 + lane;
+        if (!stomp_active(state, done, b)) continue;   // uniform over the block
+        const int rem = min(e, TD - 1), t = rem / D;
         auto cost = [&](int r) {
             const size_t row = (size_t)r * B + b;
-            return sc_cur[row * T + t] + ctrl[row * T * D + rem];
+            return sc_cur[row * T + t] + ctrl[row * TD + rem];
         };
-        // the rollouts go in batches of 8 whose loads are all issued before
-        // their values are used, so that each thread keeps 16 or 24 loads in
-        // flight (the kernel waited on one load at a time); the min/max, the
-        // sum and the weighted noise still run in rollout order
-        constexpr int kB = 8;
-        float mn = cost(0), mx = mn;
-        int r = 1;
-        for (; r + kB <= R; r += kB) {
-            float c[kB];
-#pragma unroll
-            for (int k = 0; k < kB; ++k) c[k] = cost(r + k);
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                mn = fminf(mn, c[k]);
-                mx = fmaxf(mx, c[k]);
-            }
-        }
-        for (; r < R; ++r) {
+        auto noise_at = [&](int r) { return noise[((size_t)r * B + b) * TD + rem]; };
+        float mn = __int_as_float(0x7fffffff), mx = mn;   // a NaN: fminf and fmaxf drop it
+#pragma unroll 4
+        for (int r = warp; r < R; r += kWeightWarps) {
             const float c = cost(r);
             mn = fminf(mn, c);
             mx = fmaxf(mx, c);
+            if (once) {
+                cs[r][lane] = c;
+                zs[r][lane] = noise_at(r);
+            }
+        }
+        lo[warp][lane] = mn;
+        hi[warp][lane] = mx;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kWeightWarps; ++k) {
+            mn = fminf(mn, lo[k][lane]);
+            mx = fmaxf(mx, hi[k][lane]);
         }
         const float denom = fmaxf(mx - mn, 1.0e-8f);
         float sum = 0.0f;
-        for (r = 0; r + kB <= R; r += kB) {
-            float c[kB];
-#pragma unroll
-            for (int k = 0; k < kB; ++k) c[k] = cost(r + k);
-#pragma unroll
-            for (int k = 0; k < kB; ++k) sum += expf(-h * (c[k] - mn) / denom);
+        for (int r0 = 0; r0 < R; r0 += kWeightRolls) {
+            const int n = min(kWeightRolls, R - r0);
+            for (int r = warp; r < n; r += kWeightWarps)
+                cs[r][lane] = expf(-h * ((once ? cs[r][lane] : cost(r0 + r)) - mn) / denom);
+            __syncthreads();
+            if (warp == 0)
+#pragma unroll 8
+                for (int r = 0; r < n; ++r) sum += cs[r][lane];
+            if (!once) __syncthreads();
         }
-        for (; r < R; ++r) sum += expf(-h * (cost(r) - mn) / denom);
-        sum = fmaxf(sum, 1.0e-12f);
+        if (warp == 0) tot[lane] = fmaxf(sum, 1.0e-12f);
+        __syncthreads();
+        sum = tot[lane];
         float acc = 0.0f;
-        for (r = 0; r + kB <= R; r += kB) {
-            float c[kB], z[kB];
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                c[k] = cost(r + k);
-                z[k] = noise[((size_t)(r + k) * B + b) * T * D + rem];
+        for (int r0 = 0; r0 < R; r0 += kWeightRolls) {
+            const int n = min(kWeightRolls, R - r0);
+            for (int r = warp; r < n; r += kWeightWarps) {
+                if (!once) zs[r][lane] = noise_at(r0 + r);
+                cs[r][lane] = (once ? cs[r][lane] : expf(-h * (cost(r0 + r) - mn) / denom)) / sum;
             }
-#pragma unroll
-            for (int k = 0; k < kB; ++k) acc += z[k] * (expf(-h * (c[k] - mn) / denom) / sum);
+            __syncthreads();
+            if (warp == 0)
+#pragma unroll 8
+                for (int r = 0; r < n; ++r) acc += zs[r][lane] * cs[r][lane];
+            __syncthreads();
         }
-        for (; r < R; ++r) {
-            const float p = expf(-h * (cost(r) - mn) / denom) / sum;
-            acc += noise[((size_t)r * B + b) * T * D + rem] * p;
-        }
-        delta[idx] = (t == 0 || t == T - 1) ? 0.0f : acc;
+        if (warp == 0 && e < TD) delta[(size_t)b * TD + e] = (t == 0 || t == T - 1) ? 0.0f : acc;
     }
 }
 
@@ -515,8 +542,13 @@ extern "C" int ps_stomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     cp_total.smoothness_weight = P->control_cost_weight;
     const uint32_t key0 = (uint32_t)(P->seed & 0xffffffffull), key1 = (uint32_t)(P->seed >> 32);
 
-    opt_band_kernel<<<1, 1, 0, s>>>(T, P->delta_t, o.band);
-    stomp_setup_kernel<<<1, 256, 0, s>>>(T, o.band, w.scratch, w.colscale, w.amp, P->noise_scale);
+    opt_band_kernel<<<1, kBandThreads, 0, s>>>(T, P->delta_t, o.band);
+    const size_t setup_smem = sizeof(double) * (size_t)T * (T | 1);
+    const bool setup_shared = setup_smem <= 160 * 1024;   // within the limit beside the reduction's scratch
+    if (setup_shared && setup_smem > 40 * 1024)
+        PS_TRY_CUDA(allow_smem((const void*)stomp_setup_kernel, setup_smem));
+    stomp_setup_kernel<<<1, 256, setup_shared ? setup_smem : 0, s>>>(T, o.band, w.scratch, w.colscale, w.amp,
+                                                                     P->noise_scale, setup_shared);
     opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0, o.hit_step,
                                                   o.n_list);
     PS_TRY_CUDA(cudaGetLastError());
@@ -542,15 +574,14 @@ extern "C" int ps_stomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     if (int rc = big(stomp_project_kernel, pj_smem)) return rc;
     if (int rc = big(stomp_bookkeep_kernel, bk_smem)) return rc;
     if (int rc = big(stomp_topk_kernel, sizeof(float) * (size_t)R)) return rc;
-    const long long n_w = (long long)B * T * D;
-    const int w_grid = (int)std::min<long long>((n_w + 255) / 256, (long long)sm_count() * 16);
+    const int w_grid = (int)std::min<long long>((long long)B * ((T * D + 31) / 32), (long long)sm_count() * 8);
 
     // One iteration at chunk position i (parity i & 1; a chunk has an even
     // length, so the parity is the iteration's own): a request at step 0 is
     // only evaluated (the seed); from step 1 on it is updated first.
     auto iteration = [&](cudaStream_t q, int i) -> int {
         const int cur = i & 1, prev = cur ^ 1;
-        stomp_topk_kernel<<<B, 32, sizeof(float) * R, q>>>(w.tot[prev], w.topk, R, Ro, B, o.state, o.done);
+        stomp_topk_kernel<<<B, kTopkThreads, sizeof(float) * R, q>>>(w.tot[prev], w.topk, R, Ro, B, o.state, o.done);
         stomp_rollouts_kernel<<<dim3((R + ro_kg - 1) / ro_kg, B), 128, ro_smem, q>>>(theta, B, T, D, Rn, Ro, ro_kg,
                                                               o.band, w.amp, key0, key1,
                                                               m->dev.lower, m->dev.upper, w.roll[cur], w.roll[prev],
@@ -563,7 +594,7 @@ extern "C" int ps_stomp_optimize(const ps_model* m, const ps_scene_view* scene, 
         stomp_row_totals_kernel<<<dim3(R, B), tot_threads, tot_smem, q>>>(w.roll[cur], w.sc[cur], w.ctrl, w.tot[cur],
                                                                          B, T, D, P->control_cost_weight, P->delta_t,
                                                                          o.state, o.done);
-        stomp_weights_kernel<<<w_grid, 256, 0, q>>>(w.sc[cur], w.ctrl, w.noise, w.delta, B, T, D, R,
+        stomp_weights_kernel<<<w_grid, kWeightWarps * 32, 0, q>>>(w.sc[cur], w.ctrl, w.noise, w.delta, B, T, D, R,
                                                     P->exponentiated_cost_sensitivity, o.state, o.done);
         stomp_project_kernel<<<B * D, 64, pj_smem, q>>>(theta, w.delta, o.band, w.colscale, B, T, D, o.state, o.done);
         PS_TRY_CUDA(cudaGetLastError());
