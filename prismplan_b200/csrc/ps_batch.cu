@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) batch_waypoint_kerne
     const int n_wp = cnt->n_wp, n_roll = cnt->n_roll;
     const int chunks_a = (n_wp + kCostSlots - 1) / kCostSlots, chunks = chunks_a + (n_roll + kCostSlots - 1) / kCostSlots;
     if (blockIdx.x * kWarps >= chunks) return;   // nothing for this block: skip staging
-    if (P.include_self) warm_self_tables(md);
+    if (P.include_self) warm_self_tables<false>(md);
     if (!stage_model(md, smem, &mbar)) {   // fail closed: NaN costs and gradient rows
         const float nan = __int_as_float(0x7fc00000);
         cost_fail_closed(md, n_wp, kWarps * kCostSlots, [&](long long k, int D) {

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kLaneCostWarps * 32, 2) waypoint_cost_kernel(
     __shared__ int counters[4];
     __shared__ float bmax;
     const bool bdt = P.layout == PS_LAYOUT_BDT;
-    if (P.include_self) warm_self_tables(md);
+    if (P.include_self) warm_self_tables<false>(md);
     if (!stage_model(md, smem, &mbar)) {
         const float nan = __int_as_float(0x7fc00000);
         cost_fail_closed(md, (long long)n_rows * T, kLaneCostWarps * kCostSlots, [&](long long idx, int D) {

@@ -152,19 +152,6 @@ __device__ __forceinline__ void lane_fold(const ModelSmem& M, const LaneScratch&
     }
 }
 
-// Reads the self pass's tables once into L1, at the start of a block while the
-// model and the scene are staged: the pass meets them one entry after the
-// other, an L2 trip each.
-__device__ __forceinline__ void warm_self_tables(const ModelDev& md) {
-    constexpr int kLine = 128;
-    const char* t[2] = {reinterpret_cast<const char*>(md.sjp), reinterpret_cast<const char*>(md.sruns)};
-    const int n[2] = {md.n_sjp * (int)sizeof(uint4), md.n_sruns * (int)sizeof(uint2)};
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        for (int i = threadIdx.x * kLine; i < n[k]; i += blockDim.x * kLine)
-            asm volatile("{ .reg .u32 t; ld.global.nc.u32 t, [%0]; }" ::"l"(t[k] + i));
-}
-
 // Sum over the kCostSub lanes of a waypoint's group (fixed xor order).
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll

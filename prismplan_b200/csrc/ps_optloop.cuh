@@ -229,8 +229,8 @@ __global__ void opt_segments_kernel(const float* __restrict__ theta, int T, int 
 //
 // Those checks took eight launches (scene and self check of the waypoints,
 // segments, header, preparation, two queue passes, self pass, finalize) and
-// 141 us of a 256-request CHOMP iteration; this kernel takes 46 us and
-// opt_refine_kernel 38 us. With the refining inside this kernel (one launch)
+// 141 us of a 256-request CHOMP iteration; this kernel takes 42 us and
+// opt_refine_kernel 36 us. With the refining inside this kernel (one launch)
 // the few requests without a colliding waypoint held it for 112 us.
 template <bool kEsdf>
 __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md, ps_scene_view sv,
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md,
     __shared__ int max_seg_bits;
     PathSmem ps;
     SceneSmem sc;
-    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, ps, sc)) {   // fail closed
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, ps, sc)) {   // fail closed
         if (threadIdx.x == 0) *hit_at = now;
         return;
     }
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md
     __shared__ PathBlock blk;
     PathSmem ps;
     SceneSmem sc;
-    const bool staged = path_stage(md, sv, smem, &mbar, counters, &bmax, ps, sc);
+    const bool staged = path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, ps, sc);
     const ModelSmem M = model_view(smem);
     const bool self = check_self != 0;
     for (int k = blockIdx.x; k < total; k += gridDim.x) {

@@ -257,13 +257,15 @@ __device__ __forceinline__ unsigned path_sweep(const ModelSmem& M, const ModelDe
                     const float ex = px - qx, ey = py - qy, ez = pz - qz;
                     const float lim = ri + Rq;
                     if (fmaf(ez, ez, fmaf(ey, ey, ex * ex)) >= lim * lim) continue;
+                    bool any = false;   // no branch in the loop: its loads go out together
 #pragma unroll 4
                     for (int k = 0; k < len; ++k) {
                         const int j = (int)run.y + k;
                         const float fx = px - at(sm.pos, j, 0), fy = py - at(sm.pos, j, 1), fz = pz - at(sm.pos, j, 2);
                         const float lj = ri + fabsf(M.S[j].w);
-                        close = close || !(fmaf(fz, fz, fmaf(fy, fy, fx * fx)) >= lj * lj);
+                        any |= !(fmaf(fz, fz, fmaf(fy, fy, fx * fx)) >= lj * lj);
                     }
+                    close = any;
                 }
             }
         }
@@ -407,8 +409,10 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
 
 // Stages the model and the scene. False: the staging gave up (uniform).
 __device__ __forceinline__ bool path_stage(const ModelDev& md, const ps_scene_view& sv, unsigned char* smem,
-                                           uint64_t* mbar, int* counters, float* bmax, PathSmem& ps, SceneSmem& sc) {
+                                           uint64_t* mbar, int* counters, float* bmax, bool self, PathSmem& ps,
+                                           SceneSmem& sc) {
     if (!stage_model(md, smem, mbar)) return false;
+    if (self) warm_self_tables<true>(md, reinterpret_cast<const BlobHeader*>(smem)->n_joints);
     ps = path_carve(smem, md, sv);
     stage_scene(sv, ps.obbs, ps.orig, ps.layers, counters, bmax, sc);
     box_spheres(sc, ps.obs);
@@ -463,7 +467,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md
     __shared__ PathBlock blk;
     PathSmem ps;
     SceneSmem sc;
-    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, ps, sc)) {   // fail closed
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, ps, sc)) {   // fail closed
         if (threadIdx.x == 0) {
             atomicExch(timed_out, 1);
             for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {

@@ -22,6 +22,22 @@ __device__ __forceinline__ ObbPrep prep_box(float4 dm, float4 pa, float4 pb) {
     return p;
 }
 
+// Reads the self pairs' tables once into L1, at the start of a block while the
+// model and the scene are staged: the passes over them meet one entry after
+// the other, an L2 trip each. With kLever the levers too.
+template <bool kLever>
+__device__ __forceinline__ void warm_self_tables(const ModelDev& md, int n_joints = 0) {
+    constexpr int kLine = 128;
+    const char* t[3] = {reinterpret_cast<const char*>(md.sjp), reinterpret_cast<const char*>(md.sruns),
+                        reinterpret_cast<const char*>(md.lever)};
+    const int n[3] = {md.n_sjp * (int)sizeof(uint4), md.n_sruns * (int)sizeof(uint2),
+                      n_joints * n_joints * (int)sizeof(float)};
+#pragma unroll
+    for (int k = 0; k < (kLever ? 3 : 2); ++k)
+        for (int i = threadIdx.x * kLine; i < n[k]; i += blockDim.x * kLine)
+            asm volatile("{ .reg .u32 t; ld.global.nc.u32 t, [%0]; }" ::"l"(t[k] + i));
+}
+
 // Builds the prepared box table (compacted enabled boxes, 3x3 maps, exact
 // half extents) and the ESDF layer headers from the caller's
 // SceneCollisionData arrays. Call with all threads; ends with __syncthreads().

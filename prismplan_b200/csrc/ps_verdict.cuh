@@ -594,11 +594,13 @@ __device__ bool lane_self_hit(const ModelSmem& M, const ModelDev& md, const floa
 // lanes then split the approximate pairs and, per joint pair that passes its
 // bound test, the runs, each lane to its own first hit, with one group ballot
 // per phase (the verdict is an OR, so the split changes the work, not the
-// result). The check of a few
-// thousand configurations is latency-bound: one lane per configuration left
+// result). The check of a few thousand configurations is latency-bound: one lane per configuration left
 // 3 warps per SM for the same shared memory (16,384 CHOMP waypoints: 49.6 ->
-// 26.5 us with a ballot after every round, 24.0 us with one per phase). The edge self pass keeps lane_self_hit: its windows of samples
-// ran slower with groups of 2 or 4 lanes (107 -> 135 and 124 us).
+// 26.5 us with a ballot after every round, 24.0 us with one per phase). With
+// the joint pairs' bounds split over the lanes and four pairs at a time
+// 20,011 configurations of a two-arm robot take 44.5 us (55 before). The edge
+// self pass keeps lane_self_hit: its windows of samples ran slower with groups
+// of 2 or 4 lanes (107 -> 135 and 124 us).
 constexpr int kSelfSub = 4;
 constexpr int kSelfBlock = kSelfThreads * kSelfSub;   // threads of a self-check block
 
@@ -654,25 +656,32 @@ __device__ bool group_self_hit(const ModelSmem& M, const ModelDev& md, const flo
     auto at = [&](const float* a, int k, int c) { return a[(k * 3 + c) * kSlots + slot]; };
     // a joint's world bound centre (its first approximate sphere's when the model says so)
     auto bc = [&](int p, int c) { return md.bound_from_apx ? at(apos, M.J[p].apx_beg, c) : at(cpos, p, c); };
-    // each lane runs its share to its own first hit; the group ballots once
-    // per phase (the verdict is an OR, so a lane's early stop changes nothing)
+    // each lane runs its share, four pairs at a time (loads that wait for each
+    // other otherwise), to its own first hit; the group ballots once per phase
+    // or batch of joint pairs (the verdict is an OR, so a lane's early stop
+    // changes nothing)
     bool need = false;
-    for (int k = u; k < M.H->n_apx_self_pairs && !need; k += kSelfSub) {
-        const uint32_t pr = __ldg(md.apx_self_pairs + k);
-        const int i = pr & 0xffff, j = pr >> 16;
-        st.v[ST_SELF] += 1;
-        need = ref_self_hit(at(apos, i, 0), at(apos, i, 1), at(apos, i, 2), M.A[i].w, at(apos, j, 0), at(apos, j, 1),
-                            at(apos, j, 2), M.A[j].w);
+    const int na = M.H->n_apx_self_pairs;
+    for (int k0 = u; k0 < na && !need; k0 += 4 * kSelfSub) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const uint32_t pr = __ldg(md.apx_self_pairs + min(k0 + v * kSelfSub, na - 1));
+            const int i = pr & 0xffff, j = pr >> 16;
+            need |= ref_self_hit(at(apos, i, 0), at(apos, i, 1), at(apos, i, 2), M.A[i].w, at(apos, j, 0),
+                                 at(apos, j, 1), at(apos, j, 2), M.A[j].w);
+        }
+        st.v[ST_SELF] += 4;
     }
     if (!__ballot_sync(gmask, need)) return false;
-    bool hit = false;
-    // joint pairs (a, q), nearest in DFS order first: a pair whose bound
-    // spheres are apart (|c_a - c_q| >= R_a + R_q plus the guard band) holds
-    // no pair that can pass the float test, so its runs are skipped
-    for (int jp = 0; jp < md.n_sjp && !hit; ++jp) {
-        const uint4 e = __ldg(md.sjp + jp);
-        const int a = (int)(e.x & 0xffffu), qj = (int)(e.x >> 16);
-        {
+    // joint pairs (a, q), nearest in DFS order first, one per lane: a pair
+    // whose bound spheres are apart (|c_a - c_q| >= R_a + R_q plus the guard
+    // band) holds no pair that can pass the float test, so its runs are
+    // skipped; the lanes share the runs of the others
+    for (int jp0 = 0; jp0 < md.n_sjp; jp0 += kSelfSub) {
+        bool pass = false;
+        if (jp0 + u < md.n_sjp) {
+            const uint4 e = __ldg(md.sjp + jp0 + u);
+            const int a = (int)(e.x & 0xffffu), qj = (int)(e.x >> 16);
             const float ax = bc(a, 0), ay = bc(a, 1), az = bc(a, 2);
             const float bx = bc(qj, 0), by = bc(qj, 1), bz = bc(qj, 2);
             const float dx = ax - bx, dy = ay - by, dz = az - bz;
@@ -680,30 +689,40 @@ __device__ bool group_self_hit(const ModelSmem& M, const ModelDev& md, const flo
                                   fmaxf(fabsf(bx), fmaxf(fabsf(by), fabsf(bz))));
             float lim = M.J[a].bound.w + M.J[qj].bound.w;
             lim += 4.0f * (S + lim + 1.0f) * PS_GUARD_K;
-            if (u == 0) st.v[ST_SELF] += 1;
-            if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) >= lim * lim * (1.0f + 1.0e-6f)) continue;
-        }
-        const float4 bq = M.J[qj].bound;
-        const float cx = bc(qj, 0), cy = bc(qj, 1), cz = bc(qj, 2);
-        for (int r = (int)e.y + u; r < (int)e.z && !hit; r += kSelfSub) {
-            const uint2 run = __ldg(md.sruns + r);
-            const int i = run.x & 0x1ff, len = run.x >> 14;
-            const float px = at(pos, i, 0), py = at(pos, i, 1), pz = at(pos, i, 2), ri = M.S[i].w;
-            const float dx = px - cx, dy = py - cy, dz = pz - cz;
-            const float S = fmaxf(fmaxf(fabsf(px), fmaxf(fabsf(py), fabsf(pz))),
-                                  fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))));
-            float lim = ri + bq.w;
-            lim += 4.0f * (S + lim + 1.0f) * PS_GUARD_K;
             st.v[ST_SELF] += 1;
-            if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) >= lim * lim * (1.0f + 1.0e-6f)) continue;   // no pair can hit
-            for (int k = 0; k < len && !hit; ++k) {
-                const int j = (int)run.y + k;
+            pass = !(fmaf(dz, dz, fmaf(dy, dy, dx * dx)) >= lim * lim * (1.0f + 1.0e-6f));
+        }
+        bool hit = false;
+        // uniform over the group
+        for (unsigned bal = __ballot_sync(gmask, pass) >> ((threadIdx.x & 31) & ~(kSelfSub - 1)); bal; bal &= bal - 1) {
+            const uint4 e = __ldg(md.sjp + jp0 + __ffs(bal) - 1);
+            const int qj = (int)(e.x >> 16);
+            const float4 bq = M.J[qj].bound;
+            const float cx = bc(qj, 0), cy = bc(qj, 1), cz = bc(qj, 2);
+            for (int r = (int)e.y + u; r < (int)e.z && !hit; r += kSelfSub) {
+                const uint2 run = __ldg(md.sruns + r);
+                const int i = run.x & 0x1ff, len = run.x >> 14, j0 = (int)run.y;
+                const float px = at(pos, i, 0), py = at(pos, i, 1), pz = at(pos, i, 2), ri = M.S[i].w;
+                const float dx = px - cx, dy = py - cy, dz = pz - cz;
+                const float S = fmaxf(fmaxf(fabsf(px), fmaxf(fabsf(py), fabsf(pz))),
+                                      fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))));
+                float lim = ri + bq.w;
+                lim += 4.0f * (S + lim + 1.0f) * PS_GUARD_K;
                 st.v[ST_SELF] += 1;
-                hit = ref_self_hit(px, py, pz, ri, at(pos, j, 0), at(pos, j, 1), at(pos, j, 2), M.S[j].w);
+                if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) >= lim * lim * (1.0f + 1.0e-6f)) continue;   // no pair can hit
+                for (int k = 0; k < len && !hit; k += 4) {   // past the end: the last sphere again
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        const int j = j0 + min(k + v, len - 1);
+                        hit |= ref_self_hit(px, py, pz, ri, at(pos, j, 0), at(pos, j, 1), at(pos, j, 2), M.S[j].w);
+                    }
+                    st.v[ST_SELF] += 4;
+                }
             }
         }
+        if (__ballot_sync(gmask, hit)) return true;
     }
-    return __ballot_sync(gmask, hit) != 0;
+    return false;
 }
 
 // Shared memory of a self-check block (kSelfThreads configuration slots): model
