@@ -52,54 +52,76 @@ __global__ void chomp_bookkeep_kernel(const float* __restrict__ theta, const flo
                        n_done);
 }
 
-// One block per (request, DoF): g = obs_grad + lambda R theta_d with the
+// One block per dg DoFs of a request: g = obs_grad + lambda R theta_d with the
 // obstacle gradient of the pinned endpoints taken as 0 (chomp.cu:100-104),
 // x = (R + 1e-8 I)^-1 g, then theta_t -= step * x_t on the interior
 // waypoints, clamped to the limits (chomp.cu:260-293). R theta (two 5-tap
-// stencils) and the banded triangular solves (thread 0) run in FP64: the
-// solve amplifies an error in g by up to 1 / lambda_min(R) (about 37 at
+// stencils) and the banded triangular solves (a thread per DoF) run in FP64:
+// the solve amplifies an error in g by up to 1 / lambda_min(R) (about 37 at
 // T = 64, dt = 0.1), so g is formed without FP32 rounding.
+//
+// The solve is a serial chain in one lane, and an FP64 instruction costs the
+// SM the same for one lane as for a warp: with a block per DoF 256 requests of
+// 64 waypoints by 7 joints took 14.7 us, with their DoFs in one warp 9.6 us.
+// Few requests keep a block per DoF, which stages less per block (update_dofs).
 __global__ void chomp_update_kernel(float* __restrict__ theta, const float* __restrict__ grad,
                                     const double* __restrict__ L, const float* __restrict__ lower,
-                                    const float* __restrict__ upper, int T, int D, float step, float lambda,
+                                    const float* __restrict__ upper, int T, int D, int dg, float step, float lambda,
                                     float dt_f, const uint8_t* __restrict__ done) {
-    extern __shared__ double shd[];   // th [T + 12], ac [T + 12], x [T], Ls [5 T]
-    const int b = blockIdx.x / D, d = blockIdx.x % D;
+    // th [T + 12][nd], ac [T + 12][nd], x [nd][S], Ls [5 T]; the odd stride S
+    // puts the chains that lanes walk side by side in different banks
+    extern __shared__ double shd[];
+    const int per = (D + dg - 1) / dg;
+    const int b = blockIdx.x / per, d0 = (blockIdx.x % per) * dg, nd = min(dg, D - d0);
     if (done[b]) return;
-    const int Np = T + 12;
+    const int Np = T + 12, S = T | 1;
     double* th = shd;
-    double* ac = th + Np;
-    double* x = ac + Np;
-    double* Ls = x + T;   // the factor, staged so that the serial solve reads shared memory
+    double* ac = th + Np * dg;
+    double* x = ac + Np * dg;
+    double* Ls = x + S * dg;   // the factor, staged so that the serial solve reads shared memory
     for (int k = threadIdx.x; k < 5 * T; k += blockDim.x) Ls[k] = L[k];
-    float* col = theta + (size_t)b * T * D + d;   // stride D
-    for (int k = threadIdx.x; k < Np; k += blockDim.x) {
-        const int t = k - 6;
-        th[k] = (t >= 0 && t < T) ? (double)col[(size_t)t * D] : 0.0;
+    float* rows = theta + (size_t)b * T * D + d0;   // [t][d], stride D
+    for (int i = threadIdx.x; i < Np * nd; i += blockDim.x) {
+        const int k = i / nd, d = i - k * nd, t = k - 6;
+        th[i] = (t >= 0 && t < T) ? (double)rows[(size_t)t * D + d] : 0.0;
     }
     __syncthreads();
     const double c1 = -1.0 / 12.0, c2 = 16.0 / 12.0, c3 = -30.0 / 12.0;
     const double dt = dt_f, inv_dt2 = 1.0 / (dt * dt);
-    for (int k = threadIdx.x; k < Np; k += blockDim.x) {
-        auto at = [&](int i) { return (i >= 0 && i < Np) ? th[i] : 0.0; };
-        ac[k] = (c1 * (at(k - 2) + at(k + 2)) + c2 * (at(k - 1) + at(k + 1)) + c3 * at(k)) * inv_dt2;
+    for (int i = threadIdx.x; i < Np * nd; i += blockDim.x) {
+        const int k = i / nd, d = i - k * nd;
+        auto at = [&](int kk) { return (kk >= 0 && kk < Np) ? th[kk * nd + d] : 0.0; };
+        ac[i] = (c1 * (at(k - 2) + at(k + 2)) + c2 * (at(k - 1) + at(k + 1)) + c3 * at(k)) * inv_dt2;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < T; t += blockDim.x) {
-        const int k = t + 6;
-        const double r = (c1 * (ac[k - 2] + ac[k + 2]) + c2 * (ac[k - 1] + ac[k + 1]) + c3 * ac[k]) * inv_dt2 * dt;
-        const double og = (t == 0 || t == T - 1) ? 0.0 : (double)grad[((size_t)b * T + t) * D + d];
-        x[t] = og + (double)lambda * r;
+    for (int i = threadIdx.x; i < T * nd; i += blockDim.x) {
+        const int t = i / nd, d = i - t * nd;
+        auto at = [&](int kk) { return ac[(t + 6 + kk) * nd + d]; };
+        const double r = (c1 * (at(-2) + at(2)) + c2 * (at(-1) + at(1)) + c3 * at(0)) * inv_dt2 * dt;
+        const double og = (t == 0 || t == T - 1) ? 0.0 : (double)grad[((size_t)b * T + t) * D + d0 + d];
+        x[d * S + t] = og + (double)lambda * r;
     }
     __syncthreads();
-    if (threadIdx.x == 0) band_solve(Ls, x, T);
+    for (int d = threadIdx.x; d < nd; d += blockDim.x) band_solve(Ls, x + (size_t)d * S, T);
     __syncthreads();
-    const float lo = lower[d], hi = upper[d];
-    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    for (int i = threadIdx.x; i < T * nd; i += blockDim.x) {
+        const int t = i / nd, d = i - t * nd;
         if (t == 0 || t == T - 1) continue;   // endpoints pinned to start and goal
-        const float v = (float)(th[t + 6] - (double)step * x[t]);
-        col[(size_t)t * D] = fmaxf(lo, fminf(hi, v));
+        const float v = (float)(th[(t + 6) * nd + d] - (double)step * x[d * S + t]);
+        rows[(size_t)t * D + d] = fmaxf(lower[d0 + d], fminf(upper[d0 + d], v));
     }
+}
+
+size_t update_smem(int T, int dg) { return sizeof(double) * ((size_t)dg * (2 * (T + 12) + (T | 1)) + 5 * (size_t)T); }
+
+// DoFs of a request that share a block: one while there are SMs for every
+// DoF's block, then as many as leave two blocks an SM, within half of an SM's
+// shared memory.
+int update_dofs(int B, int T, int D) {
+    const long long blocks = (long long)B * D;
+    int dg = (int)std::min<long long>(D, (blocks + 2 * sm_count() - 1) / (2 * sm_count()));
+    while (dg > 1 && update_smem(T, dg) > 100 * 1024) --dg;
+    return std::max(1, dg);
 }
 
 struct ChompBufs {
@@ -174,8 +196,9 @@ extern "C" int ps_chomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     const size_t bk_smem = (size_t)(2 * (T + 12) + bk_threads) * sizeof(float);
     if (bk_smem > 48 * 1024)
         PS_TRY_CUDA(allow_smem((const void*)chomp_bookkeep_kernel, bk_smem));
-    const int up_threads = std::min(T, 256);
-    const size_t up_smem = sizeof(double) * (8 * T + 24);
+    const int dg = update_dofs(B, T, D);
+    const int up_threads = std::min(T * dg, 256);
+    const size_t up_smem = update_smem(T, dg);
     if (up_smem > 48 * 1024)
         PS_TRY_CUDA(allow_smem((const void*)chomp_update_kernel, up_smem));
 
@@ -192,9 +215,9 @@ extern "C" int ps_chomp_optimize(const ps_model* m, const ps_scene_view* scene, 
                                                              P->num_iterations, P->convergence_eps, P->time_limit_ms,
                                                              o.t0, o.state, o.done, best, o.n_done);
         PS_TRY_CUDA(cudaGetLastError());
-        chomp_update_kernel<<<B * D, up_threads, up_smem, q>>>(theta, w.grad, o.band, m->dev.lower, m->dev.upper, T,
-                                                               D, P->step_size, P->smoothness_weight, P->delta_t,
-                                                               o.done);
+        chomp_update_kernel<<<B * ((D + dg - 1) / dg), up_threads, up_smem, q>>>(theta, w.grad, o.band, m->dev.lower,
+                                                                             m->dev.upper, T, D, dg, P->step_size,
+                                                                             P->smoothness_weight, P->delta_t, o.done);
         PS_TRY_CUDA(cudaGetLastError());
         return PS_OK;
     };
