@@ -44,6 +44,11 @@ def _view(scene) -> _lib.SceneView:
 
 def _dev_f32(t, shape_last=None):
     torch = _torch()
+    # what a caller passes most: nothing to convert, so no dispatcher calls (0.9 -> 0.3 us, 36 of them a mixed batch)
+    if type(t) is torch.Tensor and t.dtype is torch.float32 and t.is_cuda and t.is_contiguous():
+        if shape_last is not None and t.shape[-1] != shape_last:
+            raise ValueError(f"last dimension must be {shape_last}, got {tuple(t.shape)}")
+        return t
     if not isinstance(t, torch.Tensor):
         t = torch.as_tensor(np.asarray(t, np.float32))
     if not t.is_cuda:
@@ -432,7 +437,6 @@ def traj_cost(robot: RobotModelBuilder, scene, q, params: Optional[CostParams] =
     [B, T, n_dof] (or [B, n_dof, T] with PS_LAYOUT_BDT), one fused launch for
     cost and gradient. Returns (waypoint_cost [B, T] or None, traj_cost [B],
     grad like q or None)."""
-    torch = _torch()
     params = params or CostParams()
     q = _dev_f32(q)
     if q.dim() != 3:
@@ -443,9 +447,9 @@ def traj_cost(robot: RobotModelBuilder, scene, q, params: Optional[CostParams] =
         B, D, T = q.shape
     if D != robot.n_dof:
         raise ValueError("DoF dimension mismatch")
-    wp = torch.empty((B, T), dtype=torch.float32, device=q.device) if want_waypoint else None
-    tc = torch.empty(B, dtype=torch.float32, device=q.device)
-    g = torch.empty_like(q) if want_grad else None
+    wp = q.new_empty((B, T)) if want_waypoint else None
+    tc = q.new_empty(B)
+    g = q.new_empty(q.shape) if want_grad else None
     p = params.to_c(layout)
     v = _view(scene)
     _lib.check(_lib.load().ps_traj_cost(_model(robot), C.byref(v), q.data_ptr(), B, T, C.byref(p),
@@ -748,8 +752,8 @@ class MixedBatch:
             samples = torch.as_tensor(samples).to(device=frm.device, dtype=torch.int32).contiguous()
             if samples.shape[0] != n:
                 raise ValueError("samples must have one entry per edge")
-        valid = torch.empty(n, dtype=torch.uint8, device=frm.device)
-        cost = torch.empty(n, dtype=torch.float32, device=frm.device)
+        valid = frm.new_empty(n, dtype=torch.uint8)   # new_empty: like torch.empty, without parsing dtype and device
+        cost = frm.new_empty(n)
         _lib.check(_lib.load().ps_batch_add_edges(self.handle, frm.data_ptr(), to.data_ptr(),
                                                   samples.data_ptr() if samples is not None else None, n,
                                                   valid.data_ptr(), cost.data_ptr()))
@@ -759,14 +763,13 @@ class MixedBatch:
     def add_trajectory(self, q, want_waypoint: bool = True, want_traj: bool = True, want_grad: bool = True):
         """Queue one trajectory q [T, n_dof]; returns (waypoint_cost [T] | None,
         traj_cost [1] | None, grad [T, n_dof] | None) filled by the next launch."""
-        torch = _torch()
         q = _dev_f32(q, self.robot.n_dof)
         if q.dim() != 2:
             raise ValueError("q must be [T, n_dof]")
         T = q.shape[0]
-        wp = torch.empty(T, dtype=torch.float32, device=q.device) if want_waypoint else None
-        tc = torch.empty(1, dtype=torch.float32, device=q.device) if want_traj else None
-        g = torch.empty_like(q) if want_grad else None
+        wp = q.new_empty(T) if want_waypoint else None
+        tc = q.new_empty(1) if want_traj else None
+        g = q.new_empty(q.shape) if want_grad else None
         ptr = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
         _lib.check(_lib.load().ps_batch_add_trajectory(self.handle, q.data_ptr(), T, ptr(wp), ptr(tc), ptr(g)))
         self._keep += [q, wp, tc, g]
@@ -776,12 +779,11 @@ class MixedBatch:
         """Queue STOMP rollouts [R, n_dof, T] (the reference layout); returns
         their state costs, [R, T] or [R, n_dof, T] when broadcast_d, filled by
         the next launch (equal to ``rollout_costs`` bit for bit)."""
-        torch = _torch()
         r = _dev_f32(rollouts)
         if r.dim() != 3 or r.shape[1] != self.robot.n_dof:
             raise ValueError("rollouts must be [R, n_dof, T]")
         R, D, T = r.shape
-        out = torch.empty((R, D, T) if broadcast_d else (R, T), dtype=torch.float32, device=r.device)
+        out = r.new_empty((R, D, T) if broadcast_d else (R, T))
         _lib.check(_lib.load().ps_batch_add_rollouts(self.handle, r.data_ptr(), R, T, 1 if broadcast_d else 0,
                                                      out.data_ptr()))
         self._keep += [r, out]
