@@ -28,9 +28,8 @@ struct EdgeWs {                         // header of the persistent workspace (6
     int self_edges;                     // edges with at least one sample
     int self_next;                      // next window of the self pass
     int wp_next;                        // next waypoint group (the batch's work-queue kernel)
-    int n_long;                         // edges with more than one chunk round (the long list); without the
-                                        // list, the most rounds of any edge when long ones go by units
-    int probed, probed_hit;             // long edges probed, and those that the probe retired
+    int n_long;                         // edges with more than one chunk round (the long list)
+    unsigned long long probed;          // long edges probed, and from bit 32 up those that the probe retired
 };
 static_assert(sizeof(EdgeWs) == 64, "the workspace header is 64 B");
 
@@ -781,7 +780,7 @@ __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float*
         hdr->deadline = P.time_budget_ms > 0.0f
                             ? global_ns() + (unsigned long long)((double)P.time_budget_ms * 1.0e6) + 1ull
                             : 0ull;
-    int local_max = 0, local_ne = 0, local_units = 0;
+    int local_max = 0, local_ne = 0;
     unsigned long long local_ns = 0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x) {
         const float* a = from + (size_t)e * D;
@@ -795,7 +794,6 @@ __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float*
         done[e] = 0;
         const int rounds = ChunkOrder(G).rounds();
         local_max = max(local_max, rounds);
-        if (!lst) local_units = max(local_units, G >= kCoarseMin ? ChunkOrder(G, kCoarseUnit).rounds() : rounds);
         local_ns += (unsigned long long)(G + ((G % 16) != 0 ? 1 : 0));
         local_ne += G > 0;
         if (lst) {   // one atomic per group of converged lanes
@@ -815,10 +813,6 @@ __device__ __forceinline__ void prep_edges(const ps_edge_params& P, const float*
         local_ne += __shfl_xor_sync(kFull, local_ne, o);
     }
     if ((threadIdx.x & 31) == 0 && local_max > 0) atomicMax(&hdr->max_rounds, local_max);
-    if (!lst) {
-        local_units = __reduce_max_sync(kFull, local_units);
-        if ((threadIdx.x & 31) == 0 && local_units > 0) atomicMax(&hdr->n_long, local_units);
-    }
     if ((threadIdx.x & 31) == 0 && P.check_self && local_ns > 0) {
         atomicAdd(&hdr->self_samples, local_ns);
         atomicAdd(&hdr->self_edges, local_ne);
@@ -1032,10 +1026,8 @@ __global__ void __launch_bounds__(kProbeThreads, 4) edges_probe_kernel(ModelDev 
     if (kPrep) {   // see coarse_now
         n_long = __reduce_add_sync(kFull, n_long);
         n_hit = __reduce_add_sync(kFull, n_hit);
-        if ((threadIdx.x & 31) == 0 && n_long) {
-            atomicAdd(&hdr->probed, n_long);
-            atomicAdd(&hdr->probed_hit, n_hit);
-        }
+        if ((threadIdx.x & 31) == 0 && n_long)
+            atomicAdd(&hdr->probed, (unsigned long long)(unsigned)n_hit << 32 | (unsigned)n_long);
     }
     flush_stats(stats, st);
 }
@@ -1085,8 +1077,8 @@ int plan_probe(const ps_model* m, const ps_scene_view* sv, int mode, bool stats,
 // of them the queue took 0.65, 0.67, 0.80 and 0.88 of its time without the
 // pass, with 37, 48, 49 and 59 % 1.08, 1.36, 1.25 and 1.43.
 __device__ __forceinline__ bool coarse_now(const EdgeWs* hdr) {
-    const volatile EdgeWs* h = hdr;
-    return 10ll * h->probed_hit < 3ll * h->probed;
+    const unsigned long long v = *(const volatile unsigned long long*)&hdr->probed;
+    return 10 * (v >> 32) < 3 * (v & 0xffffffffull);
 }
 
 // Residency per variant, measured: the boxes-only fast path runs fastest
@@ -1108,7 +1100,15 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
     // round 1 would start while much of round 0 is still in flight and check
     // chunks of edges that round 0 retires, so pass 0 runs round 0 only and
     // the second launch (pass 1) the rest.
-    const int max_rounds = kMode == 3 ? *((volatile int*)&hdr->n_long) : *((volatile int*)&hdr->max_rounds);
+    int max_rounds = *((volatile int*)&hdr->max_rounds);
+    if (kMode == 3) {
+        // Edges below kCoarseMin keep their chunks (8 at most: 9 rounds). The
+        // longer ones have u units at most, in u + ceil(sqrt(u)) - 1 rounds at
+        // most: a bound instead of the maximum over the edges, whose atomics
+        // cost the preparation 2 us.
+        const int u = (max_rounds + kStride - 1) / kStride;
+        max_rounds = max(min(max_rounds, 9), u + (u <= 16 ? 3 : (u <= 81 ? 8 : u)));
+    }
     const bool split = (long long)n_edges < 8ll * gridDim.x * kWarps;
     const int r_lo = pass == 0 ? 0 : (split ? 1 : max_rounds);
     const int r_hi = pass == 0 ? (split ? min(max_rounds, 1) : max_rounds) : max_rounds;
