@@ -36,7 +36,8 @@ struct BlobHeader {          // 64 bytes
     int off_apx, off_apx_orig, bytes_core, bytes_total;
 };
 
-// One joint in DFS visit order (128 bytes).
+// One joint in DFS visit order (112 bytes: with the spheres it sets which
+// models fit in shared memory, so nothing is kept here that a kernel can derive).
 struct JointRec {
     float ft[12];            // rows 0..2 of the fixed transform, row-major
     int type, dof, parent_slot, slot;
@@ -51,10 +52,8 @@ struct JointRec {
     // |p_s - c| and near_r = near_d - r_s, the least such value (PS_NO_NEAR: no
     // exact sphere).
     float reach, near_r, near_d;
-    float link;              // length of the fixed transform's translation
-    float cen;               // |bound centre| in the joint's frame
-    int pad[2];
 };
+static_assert(sizeof(JointRec) == 112, "the largest models that a block's shared memory holds depend on it");
 #define PS_NO_NEAR 1.0e30f
 
 // Self pairs (global memory): packed (i | j << 16), reordered sphere indices.

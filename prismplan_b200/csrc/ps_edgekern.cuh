@@ -524,12 +524,13 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
             } else {
                 joint_compose<true>(jr, qi, T, T);   // rows are read before they are written
             }
+            const float link = len_up(jr.ft[3], jr.ft[7], jr.ft[11]);
             if (jr.type >= PS_X_ROT) {
-                Ao = fmaf(jr.link, fmaf(W, W, Al), Ao);
+                Ao = fmaf(link, fmaf(W, W, Al), Ao);
                 Al = fmaf(di, W, Al);
                 W += di;
             } else {   // a sliding joint: its offset is at most link + |q|
-                Ao = fmaf(jr.link + fabsf(qi) + 32.0f * di, fmaf(W, W, Al), Ao) + 2.0f * W * di;
+                Ao = fmaf(link + fabsf(qi) + 32.0f * di, fmaf(W, W, Al), Ao) + 2.0f * W * di;
             }
             if (kStats) st.v[ST_JOINTS] += 1;
         }
@@ -538,7 +539,7 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
         sphere_world(T, jr.bound.x, jr.bound.y, jr.bound.z, cx, cy, cz);
         const float nx = __shfl_sync(kFull, cx, nb) - cx, ny = __shfl_sync(kFull, cy, nb) - cy,
                     nz = __shfl_sync(kFull, cz, nb) - cz;
-        const float Ac = fmaf(jr.cen, fmaf(W, W, Al), Ao);
+        const float Ac = fmaf(len_up(jr.bound.x, jr.bound.y, jr.bound.z), fmaf(W, W, Al), Ao);
         // how far any point of the joint's spheres moves, and the ball around them
         const float dn = fmaxf(fmaf(nz, nz, fmaf(ny, ny, nx * nx)), 1.0e-30f);
         const float move = (x * dn * rsqrtf(dn) + 0.5f * (x + x * x) * Ac) * 1.001f;

@@ -435,9 +435,6 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
                 }
             }
             for (int k = abeg[p]; k < aend[p]; ++k) far(d->approx_spheres + 4 * aorder[k]);
-            const float* f = ftab + 16 * i;
-            J[p].link = (float)(std::sqrt((double)f[3] * f[3] + (double)f[7] * f[7] + (double)f[11] * f[11]) * (1.0 + 1e-6));
-            J[p].cen = (float)(std::sqrt(cx * cx + cy * cy + cz * cz) * (1.0 + 1e-6));
             J[p].reach = (float)(reach * (1.0 + 1e-6));
             J[p].near_r = (float)(near_r + std::fabs(near_r) * 1e-6);
             J[p].near_d = (float)(near_d * (1.0 + 1e-6));
