@@ -72,7 +72,9 @@ __device__ __forceinline__ bool esdf_reachable(const SceneSmem& sc, float cx, fl
 // World centre and circumscribed radius of each staged box: local = M p + t,
 // so the centre is -M^-1 t (M^-1 from its adjugate) and the box's world points
 // lie within |h| |M^-1| of it (quat_norm_err / map_stretch bound |M^-1|; a
-// box outside that bound gets an unbounded radius). Every thread of the block
+// box outside that bound gets an unbounded radius, and so does one of 1e15 m
+// and beyond, e.g. a half-space: its squares would overflow and the prefilter
+// drop it). Every thread of the block
 // calls it.
 __device__ __forceinline__ void box_spheres(const SceneSmem& sc, float4* obs) {
     for (int o = threadIdx.x; o < sc.n_obbs; o += blockDim.x) {
@@ -87,15 +89,16 @@ __device__ __forceinline__ void box_spheres(const SceneSmem& sc, float4* obs) {
         const float cx2 = b.r0.y * b.r1.z - b.r0.z * b.r1.y, cy2 = b.r0.z * b.r1.x - b.r0.x * b.r1.z,
                     cz2 = b.r0.x * b.r1.y - b.r0.y * b.r1.x;
         const float det = b.r0.x * ax + b.r0.y * ay + b.r0.z * az;
-        float4 out;
+        // never culled by the prefilter, unless a sphere is known that it can square
+        float4 out = make_float4(0.0f, 0.0f, 0.0f, 1.0e30f);
         if (lo >= 0.25f && fabsf(det) > 0.25f) {
             const float inv = 1.0f / det;
-            out.x = -(b.r0.w * ax + b.r1.w * bx + b.r2.w * cx2) * inv;
-            out.y = -(b.r0.w * ay + b.r1.w * by + b.r2.w * cy2) * inv;
-            out.z = -(b.r0.w * az + b.r1.w * bz + b.r2.w * cz2) * inv;
-            out.w = sqrtf(b.h.x * b.h.x + b.h.y * b.h.y + b.h.z * b.h.z) * rsqrtf(lo) * (1.0f + 1.0e-5f);
-        } else {
-            out = make_float4(0.0f, 0.0f, 0.0f, 1.0e30f);   // never culled by the prefilter
+            const float x = -(b.r0.w * ax + b.r1.w * bx + b.r2.w * cx2) * inv,
+                        y = -(b.r0.w * ay + b.r1.w * by + b.r2.w * cy2) * inv,
+                        z = -(b.r0.w * az + b.r1.w * bz + b.r2.w * cz2) * inv,
+                        w = sqrtf(b.h.x * b.h.x + b.h.y * b.h.y + b.h.z * b.h.z) * rsqrtf(lo) * (1.0f + 1.0e-5f);
+            if (fabsf(x) < 1.0e15f && fabsf(y) < 1.0e15f && fabsf(z) < 1.0e15f && w < 1.0e15f)
+                out = make_float4(x, y, z, w);
         }
         obs[o] = out;
     }
