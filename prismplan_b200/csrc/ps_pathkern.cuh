@@ -299,7 +299,8 @@ struct PathBlock {
 // in quarters (with kDefer they go to defer(), a thread each, instead).
 //
 // point(seg, i, a, b): DoF i of a segment's ends; sample j is a + (j / G)
-// (b - a), rounded as the edge kernels round it, and j = G + 1 is b itself.
+// (b - a), rounded as the edge kernels round it, and j = G + 1 is b itself
+// (with `ends` j = 0 is a itself, also where b - a is not finite).
 // Every thread of the block calls it after a block barrier; blk.hit holds the
 // result after the barrier inside.
 template <bool kEsdf, bool kDefer, class Point, class Stop, class Defer>
@@ -376,7 +377,7 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
             for (int i = u; i < D; i += kSub) {
                 float a, b;
                 point(x.seg, i, a, b);
-                qc[i] = j > G ? b : __fmaf_rn(tj, __fadd_rn(b, -a), a);
+                qc[i] = j > G ? b : (ends && j == 0 ? a : __fmaf_rn(tj, __fadd_rn(b, -a), a));
             }
             __syncwarp();
             bool hit = false;
