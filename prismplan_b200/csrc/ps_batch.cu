@@ -336,7 +336,8 @@ __global__ void __launch_bounds__(kW * 32, 16 / kW)
                 retired = __shfl_sync(kFull, retired, 0);
                 if (!EP.compute_clearance && retired) continue;
                 float cm = FLT_MAX;
-                const bool h = kMode ? process_chunk_fast<false, kMode == 2>(M, sc, sv, EP, from, to, ee, GG, kk, ws, st)
+                const bool h = kMode ? process_chunk_fast<false, kMode == 2>(M, sc, sv, EP.collision_margin, from, to, ee, GG,
+                                                                             32 * kk, ws, st)
                                      : process_chunk(M, sc, sv, EP, from, to, ee, GG, kk, ws,
                                                      EP.compute_clearance ? &cm : nullptr, st);
                 if (lane == 0) {
