@@ -42,7 +42,7 @@ __global__ void chomp_bookkeep_kernel(const float* __restrict__ theta, const flo
                                       float* __restrict__ best, int* __restrict__ n_done) {
     extern __shared__ float sh[];   // traj_smooth_block: 2 (T + 12) + blockDim
     const int b = blockIdx.x;
-    if (b == 0 && threadIdx.x == 0) *v.n_list = 0;
+    if (b == 0 && threadIdx.x == 0) v.lists->empty();
     if (done[b]) return;   // uniform over the block
     const float* th = theta + (size_t)b * T * D;
     const float total = traj_smooth_block([&](int t, int d) { return th[(size_t)t * D + d]; },
@@ -190,7 +190,7 @@ extern "C" int ps_chomp_optimize(const ps_model* m, const ps_scene_view* scene, 
 
     opt_band_kernel<<<1, kBandThreads, 0, s>>>(T, P->delta_t, o.band);
     opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0, o.hit_step,
-                                                  o.n_list);
+                                                  o.lists);
     PS_TRY_CUDA(cudaGetLastError());
     const int bk_threads = 128;
     const size_t bk_smem = (size_t)(2 * (T + 12) + bk_threads) * sizeof(float);

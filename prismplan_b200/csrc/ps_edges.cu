@@ -73,6 +73,7 @@ extern "C" size_t ps_edges_workspace_bytes(int n_edges) {
     return align256(sizeof(EdgeWs)) + 6 * align256(n * 4);
 }
 
+namespace ps {
 namespace {
 
 // Workspace layout: header, then per-edge G, length, retire flag,
@@ -99,21 +100,167 @@ EdgeBufs carve_workspace(void* ws, int n_edges) {
     return b;
 }
 
+// ---------------------------------------------------------------------------
+// Small edge batches: one block per edge (ps_pathkern.cuh), then all warps
+// over what the blocks left. The lists lie in the workspace's arrays: entry k
+// is edge lst[k] with G[k] samples, of which the units bad[k] (scene) and
+// clr[k] (self) are left; done[e] says that edge e of the list collides.
+// ---------------------------------------------------------------------------
+template <bool kEsdf>
+__global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md, ps_scene_view sv, ps_edge_params P,
+                                                                     const float* __restrict__ from,
+                                                                     const float* __restrict__ to,
+                                                                     const int* __restrict__ given, int n_edges,
+                                                                     uint8_t* __restrict__ valid,
+                                                                     float* __restrict__ cost,
+                                                                     float* __restrict__ clearance, EdgeBufs w) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    __shared__ PathBlock blk;
+    PathSmem ps;
+    SceneSmem sc;
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, false, ps, sc)) {   // fail closed
+        if (threadIdx.x == 0) {
+            atomicExch(&w.hdr->timed_out, 1);
+            for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
+                valid[e] = 0;
+                cost[e] = FLT_MAX;
+                if (clearance) clearance[e] = FLT_MAX;
+            }
+        }
+        return;
+    }
+    const ModelSmem M = model_view(smem);
+    const int D = M.H->n_dof;
+    const bool self = P.check_self != 0;
+    for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
+        const float* a = from + (size_t)e * D;
+        const float* b = to + (size_t)e * D;
+        const float len = edge_length(a, b, D);
+        const int G = edge_samples(P, given, e, a, b, D, len);
+        const bool start = G > 0 && (G % 16) != 0;   // the start configuration belongs to the samples
+        // at most 32 intervals (single samples when they fit the groups), and the start by itself
+        const int m = (G - 1) / kPathGroups + 1, n = G > 0 ? (G - 1) / m + 1 : 0;
+        __syncthreads();   // the previous edge's readers of blk are done
+        const int x = threadIdx.x;
+        if (x == 0) blk.hit = blk.left[0] = blk.left[1] = 0;
+        if (x < n) blk.item[x] = PathItem{0, x * m + 1, x == n - 1 ? G : (x + 1) * m, self ? 3 : 1};
+        if (x == n && start) blk.item[x] = PathItem{0, 0, 0, self ? 3 : 1};
+        path_run<kEsdf>(
+            M, md, sc, sv, ps, P.collision_margin, self, blk, n + (start ? 1 : 0), G, false,
+            [&](int, int i, float& ai, float& bi) {
+                ai = __ldg(a + i);
+                bi = __ldg(b + i);
+            },
+            []() { return false; }, [&](const PathItem& it) { path_left(blk, it, G); });
+        if (x == 0) {
+            const bool bad = blk.hit != 0;
+            valid[e] = bad ? 0 : 1;
+            cost[e] = bad ? FLT_MAX : len;
+            if (clearance) clearance[e] = FLT_MAX;
+            if (blk.left[0] | blk.left[1]) {   // free unless the list says otherwise
+                const int k = atomicAdd(&w.hdr->n_long, 1);
+                w.lst[k] = e;
+                w.G[k] = G;
+                w.bad[k] = (int)blk.left[0];
+                w.clr[k] = (int)blk.left[1];
+                w.done[e] = 0;
+                atomicMax(&w.hdr->max_rounds, rest_unit(G));
+            }
+        }
+    }
+}
+
+// The list of a tiny batch: every sample of every edge.
+__global__ void edges_list_kernel(ps_edge_params P, const float* __restrict__ from, const float* __restrict__ to,
+                                  const int* __restrict__ given, int n_edges, int D, uint8_t* __restrict__ valid,
+                                  float* __restrict__ cost, float* __restrict__ clearance, EdgeBufs w) {
+    for (int e = threadIdx.x; e < n_edges; e += blockDim.x) {
+        const float* a = from + (size_t)e * D;
+        const float* b = to + (size_t)e * D;
+        const float len = edge_length(a, b, D);
+        const int G = edge_samples(P, given, e, a, b, D, len);
+        const unsigned bits = G > 0 ? rest_bits(1, G, G) : 0u;
+        valid[e] = 1;
+        cost[e] = len;
+        if (clearance) clearance[e] = FLT_MAX;
+        w.lst[e] = e;
+        w.G[e] = max(G, 1);
+        w.bad[e] = (int)bits;
+        w.clr[e] = P.check_self ? (int)bits : 0;
+        w.done[e] = 0;
+        if (G > 0) atomicMax(&w.hdr->max_rounds, rest_unit(G));
+    }
+    if (threadIdx.x == 0) w.hdr->n_long = n_edges;
+}
+
+template <bool kEsdf>
+__global__ void __launch_bounds__(kPathThreads, 4) edges_rest_kernel(ModelDev md, ps_scene_view sv, ps_edge_params P,
+                                                                     const float* __restrict__ from,
+                                                                     const float* __restrict__ to,
+                                                                     uint8_t* __restrict__ valid,
+                                                                     float* __restrict__ cost, EdgeBufs w) {
+    const int n = w.hdr->n_long;
+    if (n == 0) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    PathSmem ps;
+    SceneSmem sc;
+    volatile int* hit = w.done;
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, true, ps, sc)) {   // fail closed
+        if (threadIdx.x == 0) atomicExch(&w.hdr->timed_out, 1);
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            valid[w.lst[k]] = 0;
+            cost[w.lst[k]] = FLT_MAX;
+        }
+        return;
+    }
+    rest_run<kEsdf>(
+        model_view(smem), md, sc, sv, ps, P.collision_margin, P.check_self != 0, from, to, n, w.hdr->max_rounds,
+        [&](int k) { return RestItem{w.lst[k], w.G[k], (unsigned)w.bad[k], (unsigned)w.clr[k]}; },
+        [&](int e) { return hit[e] != 0; },
+        [&](int e) {
+            hit[e] = 1;
+            valid[e] = 0;
+            cost[e] = FLT_MAX;
+        });
+}
+
+}  // namespace
+}  // namespace ps
+
+namespace {
+
 // Whether a batch runs one block per edge (edges_path_kernel): small ones,
-// where the queue path waits on its launches and on single warps. Measured
-// (us, queue path / block per edge; 59-sphere arm, 64 small boxes, 0.02 rad
-// steps), with the self check 27 edges 164 / 95, 1009 223 / 163, 2048 247 /
-// 241, 4096 313 / 388; without 27 109 / 39, 1009 134 / 73, but among 64 large
-// boxes at 0.01 rad 512 69 / 68 and 1009 77 / 87; 16 samples an edge among 16
-// boxes with the self check 27 85 / 27, 2048 117 / 83, 4096 131 / 140. With an ESDF layer in reach few
-// intervals are shown clear: 27 edges 237 / 184, 512 471 / 896.
-bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, const int* given, int mode,
-                int n_edges) {
+// where the queue path waits on its launches and on single warps. few: at most
+// 32 samples an edge. Measured (us, queue path / here, on scenes from an arm
+// among 16 boxes to a two-arm robot among 128, all at 0.01 rad steps unless
+// said otherwise): with the self check 64 edges 159 / 58 to 261 / 165, 1009
+// edges 242 / 131 to 541 / 385 but at 0.05 rad 323 / 327, 2048 edges 260 / 228
+// to 581 / 685; without, 64 edges 56 / 31 to 159 / 99, 200 edges 63 / 50 to
+// 208 / 115, 512 edges 119 / 90 but among large boxes 66 / 66; few samples
+// with the self check 1009 edges 95 / 52 to 227 / 194, 2048 to 269 / 334,
+// without 512 edges 40 / 33 to 138 / 83, 1009 45 / 52. With an ESDF layer in
+// reach few intervals are shown clear: 64 edges 138 / 71, with 5000 samples
+// each 156 / 133, 200 edges 156 / 148. What costs it most are edges that no
+// interval is clear of, at a box's side (the list's samples come on top of the
+// swept check): 40 / 43 for one of 1000 samples, 72 / 84 for 512 of 600.
+bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, int mode, int n_edges, bool few) {
     if (mode == 0 || !m->rigid || g_stats || P->time_budget_ms > 0.0f) return false;   // (the counters live in the queue path)
-    const bool few = !given && P->resolution <= 0.0f && P->max_joint_step <= 0.0f && P->granularity <= 32;
-    const int most = mode == 2 ? 64 : (P->check_self || few ? 2048 : 512);
+    const int most = mode == 2 ? 64 : (P->check_self ? 1024 : (few ? 512 : 256));
     return n_edges <= most && path_serves(m, scene, P->collision_margin, P->check_self != 0);
 }
+
+// Whether every sample of a batch goes on the list at once: while the device
+// holds a warp for each of the at most 32 x (1 + 4) tasks of an edge of 1024
+// samples. A block alone walks the swept check's chain of joints first: one
+// edge of the two-arm robot among 128 boxes 129 us with the self check and 84
+// without, 52 and 35 us from the list (queue path 49 and 45).
+bool tiny_batch(int n_edges) { return n_edges * 160 <= sm_count() * 4 * kPathWarps; }
 
 // memset header -> prep -> end-sample probe -> queue pass(es) -> self pass ->
 // finalize on stream s.
@@ -123,14 +270,25 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
     const int D = m->info.n_dof;
     PS_TRY_CUDA(cudaMemsetAsync(b.hdr, 0, sizeof(EdgeWs), s));   // queue heads, deadline, max rounds, timeout
     const int mode = fast_path(m, scene, P);
-    if (path_edges(m, scene, P, samples_per_edge, mode, n_edges)) {
+    // few samples an edge (fewer than a block checks without looking at intervals), as far as the call says
+    const bool few = !samples_per_edge && P->resolution <= 0.0f && P->max_joint_step <= 0.0f && P->granularity <= 32;
+    if (path_edges(m, scene, P, mode, n_edges, few)) {
         auto pk = mode == 2 ? edges_path_kernel<true> : edges_path_kernel<false>;
-        const size_t psmem = path_smem_bytes(m, scene, P->check_self != 0);
+        auto rk = mode == 2 ? edges_rest_kernel<true> : edges_rest_kernel<false>;
+        const bool self = P->check_self != 0;
+        const size_t psmem = path_smem_bytes(m, scene, self), rsmem = rest_smem_bytes(m, scene, self);
         PS_TRY_CUDA(allow_smem((const void*)pk, psmem));
+        int rgrid = 1;
+        if (int rc = rest_grid(rk, rsmem, rgrid)) return rc;
         mark_start(s);
-        pk<<<std::min(n_edges, sm_count() * 16), kPathThreads, psmem, s>>>(m->dev, *scene, *P, from, to, samples_per_edge,
-                                                                          n_edges, valid, cost, clearance,
-                                                                          &b.hdr->timed_out);
+        const bool tiny = tiny_batch(n_edges);
+        if (tiny)
+            edges_list_kernel<<<1, 32, 0, s>>>(*P, from, to, samples_per_edge, n_edges, D, valid, cost, clearance, b);
+        else
+            pk<<<std::min(n_edges, sm_count() * 16), kPathThreads, psmem, s>>>(m->dev, *scene, *P, from, to, samples_per_edge,
+                                                                          n_edges, valid, cost, clearance, b);
+        if (tiny || !few)   // few samples are settled by their block
+            rk<<<rgrid, kPathThreads, rsmem, s>>>(m->dev, *scene, *P, from, to, valid, cost, b);
         mark_stop(s);
         PS_TRY_CUDA(cudaGetLastError());
         return PS_OK;

@@ -146,13 +146,20 @@ __device__ __forceinline__ void band_solve(const double* Ls, double* x, int T) {
     band_backward(Ls, x, T);
 }
 
+// Sizes of the lists that an iteration's validity check fills (opt_refine_kernel's
+// and opt_rest_kernel's); emptied by the bookkeeping for the next one.
+struct OptLists {
+    int refine, rest, unit;   // unit: the longest rest_unit on the rest list
+    __device__ __forceinline__ void empty() { refine = rest = unit = 0; }
+};
+
 __global__ void opt_init_kernel(OptState* __restrict__ st, uint8_t* __restrict__ done, int B, int polish,
                                 int* __restrict__ n_done, unsigned long long* __restrict__ t0,
-                                int* __restrict__ hit_step, int* __restrict__ n_list) {
+                                int* __restrict__ hit_step, OptLists* __restrict__ lists) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b == 0) {
         *n_done = 0;
-        *n_list = 0;
+        lists->empty();
         *t0 = now_ns();
     }
     if (b >= B) return;
@@ -214,32 +221,34 @@ __global__ void opt_segments_kernel(const float* __restrict__ theta, int T, int 
     for (int t = threadIdx.x; t < T - 1; t += blockDim.x) G[e0 + t] = g;
 }
 
-// Validity of the iterates in one launch (opt_validity's usual path): a block
-// takes a slice of 32 consecutive segments of a request, a group each. The
-// swept check shows most segments clear, ends included; the waypoints and
-// waypoints of the others are checked, and their densified samples when they
-// are few; else the segments go on a list for opt_refine_kernel, a block each
-// (an iterate far from its goal has some 90 samples on each of 63 segments).
-// All that stops when one of the request's slices has a
-// hit: hit_step[b] = the request's step + 1 (so that nothing needs clearing
-// between iterations). Together the same points as the waypoint
-// and segment checks below (a waypoint is the start of its segment; the last
-// one belongs to the last slice), so the request's validity is the same.
-// Finished requests are skipped.
+// Validity of the iterates (opt_validity's usual path): a block takes a slice
+// of 32 consecutive segments of a request, a group each. The swept check shows
+// most segments clear, their first waypoints included; the other waypoints are
+// checked, and the densified samples too when they are few. Else a segment
+// goes on a list: of at most 32 samples, or by an ESDF layer without a self
+// check (its box of voxels, which is all that the swept check tests, has to be
+// far for an interval to be clear), for all warps (opt_rest_kernel), the
+// others for a block each first (opt_refine_kernel; an iterate far from its
+// goal has some 90 samples on each of 63 segments).
+// All that stops when one of the request's slices has a hit: hit_step[b] = the
+// request's step + 1 (so that nothing needs clearing between iterations).
+// Together the same points as the waypoint and segment checks below (a
+// waypoint is the start of its segment; the last one belongs to the last
+// slice), so the request's validity is the same. Finished requests are skipped.
 //
 // Those checks took eight launches (scene and self check of the waypoints,
 // segments, header, preparation, two queue passes, self pass, finalize) and
 // 141 us of a 256-request CHOMP iteration; this kernel takes 42 us and
-// opt_refine_kernel 36 us. With the refining inside this kernel (one launch)
-// the few requests without a colliding waypoint held it for 112 us.
+// opt_refine_kernel 36 us.
 template <bool kEsdf>
 __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md, ps_scene_view sv,
                                                                     const float* __restrict__ theta, int T,
                                                                     float check_step, float margin, int check_self,
                                                                     const uint8_t* __restrict__ done,
                                                                     const OptState* __restrict__ state,
-                                                                    int* hit_step, int2* __restrict__ list,
-                                                                    int* n_list) {
+                                                                    int* hit_step, OptLists* lists,
+                                                                    int2* __restrict__ refine,
+                                                                    RestItem* __restrict__ rest) {
     const int b = blockIdx.y;
     if (done[b]) return;   // uniform over the block
     const int now = state[b].step + 1;
@@ -252,7 +261,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md,
     __shared__ int max_seg_bits;
     PathSmem ps;
     SceneSmem sc;
-    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, ps, sc)) {   // fail closed
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, false, ps, sc)) {   // fail closed
         if (threadIdx.x == 0) *hit_at = now;
         return;
     }
@@ -278,33 +287,41 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md,
     int G = 1;   // n_sub, capped so that the cast stays defined
     if (check_step > 0.0f && max_seg > check_step)
         G = (int)fminf(ceilf(__fdiv_rn(max_seg, check_step)), 1048576.0f);
-    // the slice's segments: the waypoint, samples 1 .. G, and after the last one its end
-    const int seg0 = blockIdx.x * kPathGroups, n = min(kPathGroups, T - 1 - seg0);
-    if (threadIdx.x < n)
-        blk.stack[threadIdx.x] =
-            PathItem{seg0 + (int)threadIdx.x, 0, seg0 + (int)threadIdx.x == T - 2 ? G + 1 : G, self ? 3 : 1};
-    if (threadIdx.x == 0) blk.n_stack = n;
-    __syncthreads();
-    path_run<kEsdf, true>(
-        M, md, sc, sv, ps, margin, self, blk, G, true,
+    // the slice's segments, the waypoint and samples 1 .. G, and after the last one its end by itself
+    const int seg0 = blockIdx.x * kPathGroups, n = min(kPathGroups, T - 1 - seg0), x = threadIdx.x;
+    const bool last = seg0 + n == T - 1;
+    if (x < n) blk.item[x] = PathItem{seg0 + x, 0, G, self ? 3 : 1};
+    if (x == n && last) blk.item[x] = PathItem{T - 2, G + 1, G + 1, self ? 3 : 1};
+    path_run<kEsdf>(
+        M, md, sc, sv, ps, margin, self, blk, n + (last ? 1 : 0), G, true,
         [&](int sg, int i, float& a, float& b) {
             a = th[sg * D + i];
             b = th[(sg + 1) * D + i];
         },
         [&]() { return *hit_at == now; },
-        [&](const PathItem& x) { list[atomicAdd(n_list, 1)] = make_int2(b * (T - 1) + x.seg, G << 2 | x.what); });
+        [&](const PathItem& it) {
+            if (G <= 32 || (kEsdf && !(it.what & 2))) {
+                const unsigned bits = rest_bits(1, G, G);
+                rest[atomicAdd(&lists->rest, 1)] =
+                    RestItem{b * T + it.seg, G, it.what & 1 ? bits : 0u, it.what & 2 ? bits : 0u};
+                atomicMax(&lists->unit, rest_unit(G));
+            } else {
+                refine[atomicAdd(&lists->refine, 1)] = make_int2(b * (T - 1) + it.seg, G << 2 | it.what);
+            }
+        });
     if (threadIdx.x == 0 && blk.hit) *hit_at = now;
 }
 
-// The segments that opt_check_kernel put on the list, a block each.
+// The long segments that opt_check_kernel left, a block each.
 template <bool kEsdf>
 __global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md, ps_scene_view sv,
                                                                      const float* __restrict__ theta, int T,
                                                                      float margin, int check_self,
                                                                      const OptState* __restrict__ state,
-                                                                     int* hit_step, const int2* __restrict__ list,
-                                                                     const int* __restrict__ n_list) {
-    const int total = *n_list;
+                                                                     int* hit_step, OptLists* lists,
+                                                                     const int2* __restrict__ refine,
+                                                                     RestItem* __restrict__ rest) {
+    const int total = lists->refine;
     if ((int)blockIdx.x >= total) return;   // uniform over the block
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
@@ -313,11 +330,11 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md
     __shared__ PathBlock blk;
     PathSmem ps;
     SceneSmem sc;
-    const bool staged = path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, ps, sc);
+    const bool staged = path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, false, ps, sc);
     const ModelSmem M = model_view(smem);
     const bool self = check_self != 0;
     for (int k = blockIdx.x; k < total; k += gridDim.x) {
-        const int2 item = list[k];
+        const int2 item = refine[k];
         const int b = item.x / (T - 1), sg = item.x - b * (T - 1), G = item.y >> 2;
         const int now = state[b].step + 1;
         volatile int* hit_at = hit_step + b;
@@ -328,25 +345,53 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md
         if (__syncthreads_or(*hit_at == now)) continue;   // the request is known to collide (also: blk's readers are done)
         const float* a = theta + ((size_t)b * T + sg) * M.H->n_dof;
         const float* c = a + M.H->n_dof;
-        // samples 1 .. G, and the trajectory's end on its last segment, in up to 32 intervals
-        const int hi = sg == T - 2 ? G + 1 : G, m = (hi + kPathGroups - 1) / kPathGroups, n = (hi + m - 1) / m;
-        if (threadIdx.x == 0) {
-            blk.hit = 0;
-            blk.n_stack = n;
-        }
-        if (threadIdx.x < n)
-            blk.stack[threadIdx.x] =
-                PathItem{sg, (int)threadIdx.x * m + 1, min(((int)threadIdx.x + 1) * m, hi), item.y & 3};
-        __syncthreads();
-        path_run<kEsdf, false>(
-            M, md, sc, sv, ps, margin, self, blk, G, false,
-            [&](int, int i, float& x, float& y) {
-                x = a[i];
-                y = c[i];
+        // samples 1 .. G in up to 32 intervals (opt_check_kernel has the ends)
+        const int m = (G - 1) / kPathGroups + 1, n = (G - 1) / m + 1, x = threadIdx.x;
+        if (x == 0) blk.hit = blk.left[0] = blk.left[1] = 0;
+        if (x < n) blk.item[x] = PathItem{sg, x * m + 1, min((x + 1) * m, G), item.y & 3};
+        path_run<kEsdf>(
+            M, md, sc, sv, ps, margin, self, blk, n, G, false,
+            [&](int, int i, float& ai, float& ci) {
+                ai = a[i];
+                ci = c[i];
             },
-            [&]() { return *hit_at == now; }, [](const PathItem&) {});
-        if (threadIdx.x == 0 && blk.hit) *hit_at = now;
+            [&]() { return *hit_at == now; }, [&](const PathItem& it) { path_left(blk, it, G); });
+        if (threadIdx.x == 0) {
+            if (blk.hit) *hit_at = now;
+            if (blk.left[0] | blk.left[1]) {
+                rest[atomicAdd(&lists->rest, 1)] = RestItem{b * T + sg, G, blk.left[0], blk.left[1]};
+                atomicMax(&lists->unit, rest_unit(G));
+            }
+        }
     }
+}
+
+// The samples that those two left, all warps over all of them.
+template <bool kEsdf>
+__global__ void __launch_bounds__(kPathThreads, 4) opt_rest_kernel(ModelDev md, ps_scene_view sv,
+                                                                   const float* __restrict__ theta, int T,
+                                                                   float margin, int check_self,
+                                                                   const OptState* __restrict__ state, int* hit_step,
+                                                                   const OptLists* lists,
+                                                                   const RestItem* __restrict__ rest) {
+    const int n = lists->rest;
+    if (n == 0) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ int counters[4];
+    __shared__ float bmax;
+    PathSmem ps;
+    SceneSmem sc;
+    volatile int* hit_at = hit_step;
+    auto report = [&](int row) { hit_at[row / T] = state[row / T].step + 1; };
+    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, check_self != 0, true, ps, sc)) {   // fail closed
+        for (int k = threadIdx.x; k < n; k += blockDim.x) report(rest[k].row);
+        return;
+    }
+    const ModelSmem M = model_view(smem);
+    rest_run<kEsdf>(
+        M, md, sc, sv, ps, margin, check_self != 0, theta, theta + M.H->n_dof, n, lists->unit,
+        [&](int k) { return rest[k]; }, [&](int row) { return hit_at[row / T] == state[row / T].step + 1; }, report);
 }
 
 // What opt_bookkeep_block reads an iterate's validity from: hit_step
@@ -354,7 +399,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md
 struct OptVerdict {
     const uint8_t *seg_valid, *wp_hit;
     const int* hit_step;
-    int* n_list;   // opt_check_kernel's list, emptied for the next iteration
+    OptLists* lists;   // emptied for the next iteration
 };
 
 // Block-level part of the bookkeeping for request b (call from every thread
@@ -454,8 +499,10 @@ struct Carver {
 struct OptBufs {
     OptState* state;
     uint8_t *done, *evalid, *hit;
-    int *G, *n_done, *hit_step, *n_list;
-    int2* list;
+    int *G, *n_done, *hit_step;
+    OptLists* lists;
+    int2* refine;
+    RestItem* rest;
     unsigned long long* t0;
     float *from, *to, *ecost;
     double* band;   // 5 T, opt_band_kernel
@@ -472,8 +519,9 @@ inline void opt_carve(Carver& c, int B, int T, int D, OptBufs& o) {
     o.G = c.take<int>(4 * E);
     o.n_done = c.take<int>(sizeof(int));
     o.hit_step = c.take<int>(4 * Bq);
-    o.n_list = c.take<int>(sizeof(int));
-    o.list = c.take<int2>(8 * E);
+    o.lists = c.take<OptLists>(sizeof(OptLists));
+    o.refine = c.take<int2>(sizeof(int2) * E);
+    o.rest = c.take<RestItem>(sizeof(RestItem) * E);
     o.t0 = c.take<unsigned long long>(sizeof(unsigned long long));
     o.from = c.take<float>(4 * E * D);
     o.to = c.take<float>(4 * E * D);
@@ -491,18 +539,24 @@ inline int opt_validity(const ps_model* m, const ps_scene_view* scene, const flo
                         float collision_margin, int check_self, float check_step, const OptBufs& o, OptVerdict& v,
                         cudaStream_t q) {
     const int slices = (T - 1 + kPathGroups - 1) / kPathGroups;
-    v = OptVerdict{o.evalid, o.hit, nullptr, o.n_list};
+    v = OptVerdict{o.evalid, o.hit, nullptr, o.lists};
     if (m->rigid && !g_stats && B <= 65535 && path_serves(m, scene, collision_margin, check_self != 0)) {
-        auto k = scene->n_voxel_layers > 0 ? opt_check_kernel<true> : opt_check_kernel<false>;
-        const size_t smem = path_smem_bytes(m, scene, check_self != 0);
+        const bool esdf = scene->n_voxel_layers > 0;
+        auto k = esdf ? opt_check_kernel<true> : opt_check_kernel<false>;
+        auto k2 = esdf ? opt_refine_kernel<true> : opt_refine_kernel<false>;
+        auto k3 = esdf ? opt_rest_kernel<true> : opt_rest_kernel<false>;
+        const size_t smem = path_smem_bytes(m, scene, check_self != 0), smem3 = rest_smem_bytes(m, scene, check_self != 0);
         PS_TRY_CUDA(allow_smem((const void*)k, smem));
-        auto k2 = scene->n_voxel_layers > 0 ? opt_refine_kernel<true> : opt_refine_kernel<false>;
         PS_TRY_CUDA(allow_smem((const void*)k2, smem));
-        v = OptVerdict{nullptr, nullptr, o.hit_step, o.n_list};
+        int grid3 = 1;
+        if (int rc = rest_grid(k3, smem3, grid3)) return rc;
+        v = OptVerdict{nullptr, nullptr, o.hit_step, o.lists};
         k<<<dim3(slices, B), kPathThreads, smem, q>>>(m->dev, *scene, theta, T, check_step, collision_margin, check_self,
-                                                      o.done, o.state, o.hit_step, o.list, o.n_list);
+                                                      o.done, o.state, o.hit_step, o.lists, o.refine, o.rest);
         k2<<<(unsigned)std::min<long long>((long long)B * (T - 1), sm_count() * 4ll), kPathThreads, smem, q>>>(
-            m->dev, *scene, theta, T, collision_margin, check_self, o.state, o.hit_step, o.list, o.n_list);
+            m->dev, *scene, theta, T, collision_margin, check_self, o.state, o.hit_step, o.lists, o.refine, o.rest);
+        k3<<<grid3, kPathThreads, smem3, q>>>(m->dev, *scene, theta, T, collision_margin, check_self, o.state, o.hit_step,
+                                              o.lists, o.rest);
         PS_TRY_CUDA(cudaGetLastError());
         return PS_OK;
     }

@@ -13,15 +13,22 @@
 //      links move inside it, an interval is shown clear of every box (and out
 //      of reach of every ESDF layer) and of self collision, or not. Skipped
 //      when the samples themselves fit the groups.
-//   2. The samples of the other intervals are checked one by one, a group
-//      each (group_verdict, group_self_hit), until one hits; when there are
-//      many, only their middles, and step 1 goes over their quarters.
+//   2. The samples of the other intervals are checked, a group each
+//      (group_verdict, group_self_hit), if they are few; else their middles.
+//   3. What is left goes on a list that all warps of the device work through
+//      (rest_run), as the queue does: 32 samples a warp for the scene, 8 for
+//      the self check. A block's own work is bounded by that: a path that
+//      slides along a box has no interval that step 1 can clear, and a block
+//      alone took 0.24 ms for 600 of its samples, 3.3 ms for 20,000 (the queue
+//      40 us).
 // The verdict is the OR over the samples' verdicts, and step 1 only leaves out
 // samples that cannot hit, so the result is the queue path's.
 #pragma once
 
+#include <algorithm>
 #include <cfloat>
 
+#include "ps_chunk.cuh"
 #include "ps_group.cuh"
 #include "ps_internal.h"
 #include "ps_verdict.cuh"
@@ -30,6 +37,7 @@ namespace ps {
 namespace {
 
 constexpr int kPathThreads = 128;
+constexpr int kPathWarps = kPathThreads / 32;
 constexpr int kPathSub = kSelfSub;                       // lanes per group
 constexpr int kPathGroups = kPathThreads / kPathSub;     // intervals (or samples) at a time
 constexpr float kSweepMaxQ = 16.0f;                      // largest joint value that the swept check judges
@@ -45,7 +53,8 @@ struct PathSmem {
     int* orig;
     LayerPrep* layers;
     float4* obs;
-    float* q;        // [groups][2 D]: a group's configuration, and an interval's half width
+    float* q;        // [groups][2 D]: a group's configuration, and an interval's half width; [32 D] a warp over the list
+    uint16_t* cand;  // over the list: a warp's candidate boxes
     SelfSmem self;   // positions of the groups' configurations
 };
 
@@ -54,10 +63,23 @@ __host__ __device__ inline size_t path_tables(int n_obbs) {   // boxes, their in
     return n * sizeof(ObbPrep) + ((n + 3) & ~size_t(3)) * 4 + sizeof(LayerPrep) * PS_MAX_LAYERS + n * 16;
 }
 
-inline size_t path_smem_bytes(const ps_model* m, const ps_scene_view* sv, bool self) {
+inline size_t path_self_bytes(const ps_model* m) {   // positions of the groups' configurations
     const int nc = m->dev.bound_from_apx ? 0 : m->info.n_joints;
+    return (size_t)(m->info.n_spheres + m->info.n_approx_spheres + nc) * 3 * kPathGroups * 4;
+}
+
+inline size_t path_smem_bytes(const ps_model* m, const ps_scene_view* sv, bool self) {
     return (size_t)m->dev.bytes_core + path_tables(sv->n_obbs) + (size_t)kPathGroups * 2 * m->info.n_dof * 4 +
-           (self ? (size_t)(m->info.n_spheres + m->info.n_approx_spheres + nc) * 3 * kPathGroups * 4 : 0) + 64;
+           (self ? path_self_bytes(m) : 0) + 64;
+}
+
+// The same for the kernels over the list: a tile of 32 configurations and the
+// candidate boxes of each warp.
+__host__ __device__ inline int rest_cand(int n_obbs) { return ((n_obbs > 1 ? n_obbs : 1) + 7) & ~7; }
+
+inline size_t rest_smem_bytes(const ps_model* m, const ps_scene_view* sv, bool self) {
+    return (size_t)m->dev.bytes_core + path_tables(sv->n_obbs) + (size_t)kPathThreads * m->info.n_dof * 4 +
+           (size_t)kPathWarps * rest_cand(sv->n_obbs) * 2 + (self ? path_self_bytes(m) : 0) + 64;
 }
 
 // Models and calls these kernels serve; the rest takes the queue path. (A
@@ -65,20 +87,25 @@ inline size_t path_smem_bytes(const ps_model* m, const ps_scene_view* sv, bool s
 // which the two paths take from different bounds.)
 inline bool path_serves(const ps_model* m, const ps_scene_view* sv, float margin, bool self) {
     return m->root_slot_only && m->info.approx_shares_chain && !sv->sphere_obb_acm_mask && !sv->sphere_acm_mask &&
-           m->min_radius + margin >= 0.0f && path_smem_bytes(m, sv, self) <= smem_optin() / 2;
+           m->min_radius + margin >= 0.0f && path_smem_bytes(m, sv, self) <= smem_optin() / 2 &&
+           rest_smem_bytes(m, sv, self) <= smem_optin() / 2;
 }
 
-__device__ __forceinline__ PathSmem path_carve(unsigned char* smem, const ModelDev& md, const ps_scene_view& sv) {
+// rest: the layout of rest_smem_bytes, else path_smem_bytes'.
+__device__ __forceinline__ PathSmem path_carve(unsigned char* smem, const ModelDev& md, const ps_scene_view& sv,
+                                               bool rest) {
     const BlobHeader* H = reinterpret_cast<const BlobHeader*>(md.blob);
-    const int nob = max(sv.n_obbs, 1);
+    const int nob = max(sv.n_obbs, 1), D = H->n_dof;
     PathSmem s;
     s.obbs = reinterpret_cast<ObbPrep*>(smem + md.bytes_core);
     s.orig = reinterpret_cast<int*>(s.obbs + nob);
     s.layers = reinterpret_cast<LayerPrep*>(s.orig + ((nob + 3) & ~3));
     s.obs = reinterpret_cast<float4*>(s.layers + PS_MAX_LAYERS);
     s.q = reinterpret_cast<float*>(s.obs + nob);
-    s.self = carve_self<kPathGroups>(reinterpret_cast<unsigned char*>(s.q + kPathGroups * 2 * H->n_dof), H->n_spheres,
-                                     H->n_approx, H->n_joints, md.bound_from_apx != 0);
+    s.cand = reinterpret_cast<uint16_t*>(s.q + kPathThreads * D);
+    unsigned char* end = rest ? reinterpret_cast<unsigned char*>(s.cand + kPathWarps * rest_cand(nob))
+                              : reinterpret_cast<unsigned char*>(s.q + kPathGroups * 2 * D);
+    s.self = carve_self<kPathGroups>(end, H->n_spheres, H->n_approx, H->n_joints, md.bound_from_apx != 0);
     return s;
 }
 
@@ -281,32 +308,30 @@ __device__ __forceinline__ unsigned path_sweep(const ModelSmem& M, const ModelDe
 struct PathItem {
     int seg, lo, hi, what;
 };
-constexpr int kPathBatch = 4 * kPathGroups;   // intervals swept before the samples of those left
-constexpr int kPathStack = 512;
+constexpr int kPathMost = kPathGroups + 1;   // intervals of a path: one per group, and a sample by itself
 struct PathBlock {
-    int hit;          // a sample collides
-    int n_stack;      // intervals still to sweep
-    int n_list;       // intervals of this pass that the swept check left
-    int n_samples;    // samples they hold (saturated)
-    PathItem list[kPathBatch], stack[kPathStack];
+    int hit;              // a sample collides
+    int n_list;           // intervals that the swept check left
+    int n_samples;        // samples they hold (saturated)
+    unsigned left[2];     // units of the path that go on the list: scene, self (path_left)
+    PathItem item[kPathMost], list[kPathMost];
 };
 
-// Works through the intervals on blk.stack, up to 128 at a time from the top, until
-// one sample hits, stop() says that the answer no longer matters, or nothing
-// is left: the swept check (skipped for single samples), then for the
-// intervals that it leaves every sample if they are few, else the middle ones
-// (on the first pass the first ones, when `ends`) and the intervals once more
-// in quarters (with kDefer they go to defer(), a thread each, instead).
+// Works through the n intervals blk.item: the swept check (skipped for single
+// samples), then for the intervals that it leaves every sample if they are
+// few, else one of each (the first one when `ends`, else the middle one), and
+// with no hit among those the intervals go to defer(), a thread each. Stops
+// early once a sample hits or stop() says that the answer no longer matters.
 //
 // point(seg, i, a, b): DoF i of a segment's ends; sample j is a + (j / G)
 // (b - a), rounded as the edge kernels round it, and j = G + 1 is b itself
 // (with `ends` j = 0 is a itself, also where b - a is not finite).
-// Every thread of the block calls it after a block barrier; blk.hit holds the
-// result after the barrier inside.
-template <bool kEsdf, bool kDefer, class Point, class Stop, class Defer>
+// Every thread of the block calls it after a block barrier; blk.hit and what
+// defer() wrote are there after the barrier inside.
+template <bool kEsdf, class Point, class Stop, class Defer>
 __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
                                          const ps_scene_view& sv, const PathSmem& ps, float margin, bool self,
-                                         PathBlock& blk, int G, bool ends, Point&& point, Stop&& stop,
+                                         PathBlock& blk, int n, int G, bool ends, Point&& point, Stop&& stop,
                                          Defer&& defer) {
     constexpr int kSub = kPathSub;
     const int D = M.H->n_dof;
@@ -317,104 +342,180 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
     volatile int* hit_flag = &blk.hit;
     LaneStats st;
     st.zero();
-    for (bool begin = true;; begin = false) {
-        const int ns = blk.n_stack, nc = min(ns, kPathBatch);
-        if (nc == 0) break;   // uniform
-        __syncthreads();      // n_stack's and the last pass' readers are done
-        if (threadIdx.x == 0) {
-            blk.n_stack = ns - nc;
-            blk.n_list = blk.n_samples = 0;
-        }
-        __syncthreads();
-        // ---- swept check of the top intervals, a group each ----
-        for (int k0 = 0; k0 < nc; k0 += kPathGroups) {
-            const PathItem it = blk.stack[ns - 1 - min(k0 + slot, nc - 1)];   // a group past the end repeats the last one
-            const bool single = it.lo == it.hi;
-            unsigned bits = (unsigned)it.what;
-            if (!__all_sync(kGrpFull, single)) {   // uniform
-                const int lo = min(it.lo, G), hi = min(it.hi, G);
-                const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
-                            th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
-                bool ok = !single;   // a single sample is checked itself
-                __syncwarp();
-                for (int i = 0; i < D; ++i) {
-                    float a, b;
-                    point(it.seg, i, a, b);
-                    ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
-                    if ((i & (kSub - 1)) == u) {
-                        qc[i] = fmaf(tm, b - a, a);
-                        dq[i] = th * (b - a);
-                    }
-                }
-                __syncwarp();
-                bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
-            }
-            if (u == 0 && k0 + slot < nc && bits) {   // in any order
-                const int k = atomicAdd(&blk.n_list, 1);
-                blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
-                atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
-            }
-        }
-        __syncthreads();
-        const int n = blk.n_list;
-        const bool all = blk.n_samples <= 2 * kPathGroups || blk.n_stack + 4 * n > kPathStack;
-        int per = 1;
-        if (all)
-            for (int k = 0; k < n; ++k) per = max(per, blk.list[k].hi - blk.list[k].lo + 1);
-        // ---- samples: task t is sample t / n of interval t % n, so that every
-        //      interval is looked at before any is finished ----
-        const long long total = (long long)per * n;
-        for (long long t0 = first; t0 < total; t0 += kPathGroups) {
-            if (__any_sync(kGrpFull, *hit_flag != 0 || stop())) break;   // one decision for the warp
-            const long long t = min(t0 + (slot - first), total - 1);
-            const PathItem x = blk.list[(int)(t % n)];
-            const int s = (int)(t / n), cnt = x.hi - x.lo + 1;
-            const bool on = t0 + (slot - first) < total && s < cnt;
-            if (!__any_sync(kGrpFull, on)) continue;   // uniform
-            const int j = x.lo + (begin && ends ? s : (s + cnt / 2) % cnt);   // from the middle on
-            const float tj = __fdiv_rn((float)j, (float)G);
+    if (threadIdx.x == 0) blk.n_list = blk.n_samples = 0;
+    __syncthreads();
+    // ---- swept check, a group per interval ----
+    for (int k0 = 0; k0 < n; k0 += kPathGroups) {
+        const PathItem it = blk.item[min(k0 + slot, n - 1)];   // a group past the end repeats the last one
+        const bool single = it.lo == it.hi;
+        unsigned bits = (unsigned)it.what;
+        if (!__all_sync(kGrpFull, single)) {   // uniform
+            const int lo = min(it.lo, G), hi = min(it.hi, G);
+            const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
+                        th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
+            bool ok = !single;   // a single sample is checked itself
             __syncwarp();
-            for (int i = u; i < D; i += kSub) {
+            for (int i = 0; i < D; ++i) {
                 float a, b;
-                point(x.seg, i, a, b);
-                qc[i] = j > G ? b : (ends && j == 0 ? a : __fmaf_rn(tj, __fadd_rn(b, -a), a));
+                point(it.seg, i, a, b);
+                ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
+                if ((i & (kSub - 1)) == u) {
+                    qc[i] = fmaf(tm, b - a, a);
+                    dq[i] = th * (b - a);
+                }
             }
             __syncwarp();
-            bool hit = false;
-            if (__any_sync(kGrpFull, on && (x.what & 1))) {   // uniform
-                bool h;
-                float clr;
-                group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
-                hit = on && (x.what & 1) && h;
-            }
-            if (self && on && (x.what & 2) && !hit)   // uniform over the group
-                hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
-            if (hit && u == 0) *hit_flag = 1;
-            __syncwarp();
+            bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
         }
-        __syncthreads();
-        if (__syncthreads_or(*hit_flag != 0 || stop())) break;   // one decision for the block
-        if (!all && threadIdx.x < n) {
-            const PathItem x = blk.list[threadIdx.x];
-            const long long cnt = x.hi - x.lo + 1;
-            if (kDefer) defer(x);
-            for (int k = 0; k < 4 && cnt > 1 && !kDefer; ++k) {
-                const int lo = x.lo + (int)(cnt * k / 4), hi = x.lo + (int)(cnt * (k + 1) / 4) - 1;
-                if (lo <= hi) blk.stack[atomicAdd(&blk.n_stack, 1)] = PathItem{x.seg, lo, hi, x.what};
-            }
+        if (u == 0 && k0 + slot < n && bits) {   // in any order
+            const int k = atomicAdd(&blk.n_list, 1);
+            blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
+            atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
         }
-        __syncthreads();
     }
     __syncthreads();
+    const int nl = blk.n_list;
+    const bool all = blk.n_samples <= 2 * kPathGroups;
+    int per = nl > 0 ? 1 : 0;
+    if (all)
+        for (int k = 0; k < nl; ++k) per = max(per, blk.list[k].hi - blk.list[k].lo + 1);
+    // ---- samples: task t is sample t / nl of interval t % nl, so that every
+    //      interval is looked at before any is finished ----
+    const int total = per * nl;
+    for (int t0 = first; t0 < total; t0 += kPathGroups) {
+        if (__any_sync(kGrpFull, *hit_flag != 0 || stop())) break;   // one decision for the warp
+        const int t = min(t0 + (slot - first), total - 1);
+        const PathItem x = blk.list[t % nl];
+        const int s = t / nl, cnt = x.hi - x.lo + 1;
+        const bool on = t0 + (slot - first) < total && s < cnt;
+        if (!__any_sync(kGrpFull, on)) continue;   // uniform
+        const int j = x.lo + (ends ? s : (s + cnt / 2) % cnt);   // from the middle on
+        const float tj = __fdiv_rn((float)j, (float)G);
+        __syncwarp();
+        for (int i = u; i < D; i += kSub) {
+            float a, b;
+            point(x.seg, i, a, b);
+            qc[i] = j > G ? b : (ends && j == 0 ? a : __fmaf_rn(tj, __fadd_rn(b, -a), a));
+        }
+        __syncwarp();
+        bool hit = false;
+        if (__any_sync(kGrpFull, on && (x.what & 1))) {   // uniform
+            bool h;
+            float clr;
+            group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
+            hit = on && (x.what & 1) && h;
+        }
+        if (self && on && (x.what & 2) && !hit)   // uniform over the group
+            hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
+        if (hit && u == 0) *hit_flag = 1;
+        __syncwarp();
+    }
+    if (!__syncthreads_or(*hit_flag != 0 || stop()) && !all && threadIdx.x < nl && blk.list[threadIdx.x].lo < blk.list[threadIdx.x].hi)
+        defer(blk.list[threadIdx.x]);   // one decision for the block
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// The list: paths whose samples are left, and which
+// ---------------------------------------------------------------------------
+// A path's samples 1 .. G in up to 32 units of rest_unit(G) samples, a whole
+// number of warps' worth; bit u of `scene` / `self`: unit u is to be checked.
+struct RestItem {
+    int row, G;   // the path's ends are rows `row` of from and to
+    unsigned scene, self;
+};
+constexpr int kRestSelf = 32 / kSelfSub;   // samples a warp checks for self collision at a time
+
+__device__ __forceinline__ int rest_unit(int G) { return 32 * ((G - 1) / 1024 + 1); }
+
+// The units that samples lo .. hi lie in.
+__device__ __forceinline__ unsigned rest_bits(int lo, int hi, int G) {
+    const int unit = rest_unit(G);
+    return (0xffffffffu >> (31 - (min(hi, G) - 1) / unit)) & (0xffffffffu << ((max(lo, 1) - 1) / unit));
+}
+
+// Marks an interval's units in blk.left.
+__device__ __forceinline__ void path_left(PathBlock& blk, const PathItem& x, int G) {
+    const unsigned bits = rest_bits(x.lo, x.hi, G);
+    if (x.what & 1) atomicOr(&blk.left[0], bits);
+    if (x.what & 2) atomicOr(&blk.left[1], bits);
+}
+
+// Blocks that work through a list: all that fit at once.
+template <class K>
+inline int rest_grid(K k, size_t smem, int& grid) {
+    PS_TRY_CUDA(allow_smem((const void*)k, smem));
+    int per_sm = 0;
+    PS_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPathThreads, smem));
+    grid = sm_count() * std::max(per_sm, 1);
+    return PS_OK;
+}
+
+// Checks what n paths have left, get(k) the k-th of them (unit: the longest
+// rest_unit among them): every warp of the grid takes 32 samples for the scene
+// or 8 for the self check at a time, consecutive ones on consecutive blocks.
+// known(row): the path is known to collide; report(row): a sample of it does.
+template <bool kEsdf, class Get, class Known, class Report>
+__device__ __forceinline__ void rest_run(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
+                                         const ps_scene_view& sv, const PathSmem& ps, float margin, bool self,
+                                         const float* __restrict__ from, const float* __restrict__ to, int n, int unit,
+                                         Get&& get, Known&& known, Report&& report) {
+    const int D = M.H->n_dof;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, u = lane & (kSelfSub - 1);
+    const WarpScratch ws{ps.q + warp * 32 * D, ps.cand + warp * rest_cand(sv.n_obbs), ps.obs};
+    LaneStats st;
+    st.zero();
+    const int per_scene = unit / 32, per_self = self ? unit / kRestSelf : 0;   // tasks a unit
+    const long long scene = 32ll * n * per_scene, total = scene + 32ll * n * per_self;
+    const long long warps = (long long)gridDim.x * kPathWarps, me = (long long)warp * gridDim.x + blockIdx.x;
+    for (long long base = me; base < total; base += 32 * warps) {
+        const long long v = base + lane * warps;   // the lanes look at 32 tasks of this warp
+        RestItem x{};
+        int j0 = 0;
+        bool live = false;
+        if (v < total) {
+            // task w is part k of unit b of path w % n: the paths' first units
+            // first, which most have, so that the warps share them evenly
+            const long long w = v < scene ? v : v - scene, r = w / n;
+            x = get((int)(w - r * n));
+            const int un = rest_unit(x.G), b = (int)(r & 31), k = (int)(r >> 5) * (v < scene ? 32 : kRestSelf);
+            j0 = b * un + k;
+            // the start configuration (see process_chunk) follows the last sample
+            const int last = x.G + (v >= scene && x.G % 16 != 0 ? 1 : 0);
+            live = k < un && j0 < last && (((v < scene ? x.scene : x.self) >> b) & 1u);
+        }
+        for (unsigned todo = __ballot_sync(kFull, live); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const int row = __shfl_sync(kFull, x.row, src), G = __shfl_sync(kFull, x.G, src),
+                      j = __shfl_sync(kFull, j0, src);
+            if (__any_sync(kFull, known(row))) continue;   // one decision for the warp
+            bool hit;
+            if (base + src * warps < scene) {   // uniform
+                hit = process_chunk_fast<false, kEsdf>(M, sc, sv, margin, from, to, row, G, j, ws, st);
+            } else {
+                const int raw = j + 1 + lane / kSelfSub;   // past the end: the last one
+                const float t = __fdiv_rn((float)(raw == G + 1 && G % 16 != 0 ? 0 : min(raw, G)), (float)G);
+                float* qc = ws.q + (lane / kSelfSub) * D;
+                for (int i = u; i < D; i += kSelfSub) {
+                    const float a = __ldg(from + (size_t)row * D + i), b = __ldg(to + (size_t)row * D + i);
+                    qc[i] = __fmaf_rn(t, __fadd_rn(b, -a), a);
+                }
+                __syncwarp();
+                hit = __any_sync(kFull, group_self_hit<kPathGroups>(M, md, qc, ps.self, threadIdx.x / kSelfSub, u, st));
+            }
+            if (hit && lane == 0) report(row);
+            __syncwarp();
+        }
+    }
 }
 
 // Stages the model and the scene. False: the staging gave up (uniform).
 __device__ __forceinline__ bool path_stage(const ModelDev& md, const ps_scene_view& sv, unsigned char* smem,
-                                           uint64_t* mbar, int* counters, float* bmax, bool self, PathSmem& ps,
+                                           uint64_t* mbar, int* counters, float* bmax, bool self, bool rest, PathSmem& ps,
                                            SceneSmem& sc) {
     if (!stage_model(md, smem, mbar)) return false;
     if (self) warm_self_tables<true>(md, reinterpret_cast<const BlobHeader*>(smem)->n_joints);
-    ps = path_carve(smem, md, sv);
+    ps = path_carve(smem, md, sv, rest);
     stage_scene(sv, ps.obbs, ps.orig, ps.layers, counters, bmax, sc);
     box_spheres(sc, ps.obs);
     __syncthreads();
@@ -448,75 +549,6 @@ __device__ __forceinline__ float edge_length(const float* a, const float* b, int
         len2 = __fmaf_rn(d, d, len2);
     }
     return sqrtf(len2);
-}
-
-// ---------------------------------------------------------------------------
-// Small edge batches: one block per edge
-// ---------------------------------------------------------------------------
-template <bool kEsdf>
-__global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md, ps_scene_view sv, ps_edge_params P,
-                                                                     const float* __restrict__ from,
-                                                                     const float* __restrict__ to,
-                                                                     const int* __restrict__ given, int n_edges,
-                                                                     uint8_t* __restrict__ valid,
-                                                                     float* __restrict__ cost,
-                                                                     float* __restrict__ clearance, int* timed_out) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ int counters[4];
-    __shared__ float bmax;
-    __shared__ PathBlock blk;
-    PathSmem ps;
-    SceneSmem sc;
-    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, ps, sc)) {   // fail closed
-        if (threadIdx.x == 0) {
-            atomicExch(timed_out, 1);
-            for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
-                valid[e] = 0;
-                cost[e] = FLT_MAX;
-                if (clearance) clearance[e] = FLT_MAX;
-            }
-        }
-        return;
-    }
-    const ModelSmem M = model_view(smem);
-    const int D = M.H->n_dof;
-    const bool self = P.check_self != 0;
-    const float margin = P.collision_margin;
-    for (int e = blockIdx.x; e < n_edges; e += gridDim.x) {
-        const float* a = from + (size_t)e * D;
-        const float* b = to + (size_t)e * D;
-        const float len = edge_length(a, b, D);
-        const int G = edge_samples(P, given, e, a, b, D, len);
-        const bool start = G > 0 && (G % 16) != 0;   // the start configuration belongs to the samples
-        // at most 32 intervals (33 with the start by itself); single samples when they fit the groups
-        const int m = max(1, (G + kPathGroups - 1) / kPathGroups);
-        const int n = G > 0 ? (G + m - 1) / m : 0;
-        __syncthreads();   // the previous edge's readers of blk are done
-        if (threadIdx.x == 0) {
-            blk.hit = 0;
-            blk.n_stack = n + (start && m == 1 ? 1 : 0);
-        }
-        if (threadIdx.x <= n && G > 0) {
-            const int x = threadIdx.x;   // x = n: the start configuration
-            blk.stack[x] = PathItem{0, x == n || (x == 0 && start && m > 1) ? 0 : x * m + 1,
-                                    x == n ? 0 : min((x + 1) * m, G), self ? 3 : 1};
-        }
-        __syncthreads();
-        path_run<kEsdf, false>(
-            M, md, sc, sv, ps, margin, self, blk, G, false,
-            [&](int, int i, float& ai, float& bi) {
-                ai = __ldg(a + i);
-                bi = __ldg(b + i);
-            },
-            []() { return false; }, [](const PathItem&) {});
-        if (threadIdx.x == 0) {
-            const bool bad = blk.hit != 0;
-            valid[e] = bad ? 0 : 1;
-            cost[e] = bad ? FLT_MAX : len;
-            if (clearance) clearance[e] = FLT_MAX;
-        }
-    }
 }
 
 }  // namespace

@@ -413,7 +413,7 @@ __global__ void stomp_bookkeep_kernel(const float* __restrict__ theta, const flo
                                       float* __restrict__ best, int* __restrict__ n_done) {
     extern __shared__ float sh[];   // traj_smooth_block: 2 (T + 12) + blockDim
     const int b = blockIdx.x;
-    if (b == 0 && threadIdx.x == 0) *v.n_list = 0;
+    if (b == 0 && threadIdx.x == 0) v.lists->empty();
     if (done[b]) return;
     const float* th = theta + (size_t)b * T * D;
     const float total = traj_smooth_block([&](int t, int d) { return th[(size_t)t * D + d]; },
@@ -550,7 +550,7 @@ extern "C" int ps_stomp_optimize(const ps_model* m, const ps_scene_view* scene, 
     stomp_setup_kernel<<<1, 256, setup_shared ? setup_smem : 0, s>>>(T, o.band, w.scratch, w.colscale, w.amp,
                                                                      P->noise_scale, setup_shared);
     opt_init_kernel<<<(B + 127) / 128, 128, 0, s>>>(o.state, o.done, B, P->num_iterations_after_valid, o.n_done, o.t0, o.hit_step,
-                                                  o.n_list);
+                                                  o.lists);
     PS_TRY_CUDA(cudaGetLastError());
 
     // rollouts per block of the rollouts kernel: up to 8, within 96 KiB of
