@@ -230,8 +230,10 @@ typedef struct ps_edge_params {
                                planners' own device deadline is the model
                                (pRRTC.cu:1595-1602). 0: no limit. The plain
                                path ignores it. No reference field.          */
-    /* Launch shape of the persistent paths; 0 = automatic, and
-       ps_tune_edges picks them. No reference fields. */
+    /* Launch shape of the work queue; 0 = automatic, and ps_tune_edges
+       picks them. With all three 0 small batches run one block per edge
+       instead; a field set to anything else asks for the queue. No
+       reference fields. */
     int   probe;            /* end-sample probe: 0 automatic (on with at least
                                8 warps of edges per SM, boxes-only scenes),
                                1 on (boxes-only scenes), 2 off              */
@@ -255,8 +257,11 @@ size_t ps_edges_workspace_bytes(int n_edges);
 
 /* Persistent work-queue path: edges are cut into warp-sized sample chunks,
    ordered chunk-major and pulled from a global queue by a persistent grid;
-   an edge found in collision retires its remaining chunks. All launches are
-   capture-safe. workspace: device, >= ps_edges_workspace_bytes(n_edges). */
+   an edge found in collision retires its remaining chunks. Small batches (up
+   to 256 edges, 512 of at most 32 samples, 1024 with the self check, 64 with
+   ESDF layers; no masks, clearance, time budget or shape fields) run one block
+   per edge and share what those leave among all warps: same results. All
+   launches are capture-safe. workspace: device, >= ps_edges_workspace_bytes(n_edges). */
 int ps_check_edges(const ps_model* model, const ps_scene_view* scene,
                    const float* from, const float* to,
                    const int* samples_per_edge, int n_edges,

@@ -251,6 +251,7 @@ namespace {
 // swept check): 40 / 43 for one of 1000 samples, 72 / 84 for 512 of 600.
 bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, int mode, int n_edges, bool few) {
     if (mode == 0 || !m->rigid || g_stats || P->time_budget_ms > 0.0f) return false;   // (the counters live in the queue path)
+    if (P->probe || P->queue_blocks_per_sm || P->grab) return false;   // the caller asks for a shape of the queue
     const int most = mode == 2 ? 64 : (P->check_self ? 1024 : (few ? 512 : 256));
     return n_edges <= most && path_serves(m, scene, P->collision_margin, P->check_self != 0);
 }
@@ -490,7 +491,8 @@ extern "C" int ps_tune_edges(const ps_model* m, const ps_scene_view* scene, cons
     p.probe = p.queue_blocks_per_sm = p.grab = 0;
     float def_ms = 0.0f;
     if (int rc = time_calls(run, s, 5, def_ms)) return rc;
-    // candidates: probe on/off (on only where the probe exists), the queue's
+    // candidates: the default (for small batches one block per edge), and the
+    // queue with the probe on/off (on only where the probe exists), the queue's
     // residency from all that fit down by two, three grab sizes
     const int mode = fast_path(m, scene, P);
     int per_sm = 0;
