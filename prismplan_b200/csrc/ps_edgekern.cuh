@@ -241,7 +241,9 @@ constexpr float kCoarseMaxQ = 16.0f;
 template <bool kStats>
 __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, const ps_edge_params& P,
                                    const float* __restrict__ from, const float* __restrict__ to, int e, int G,
-                                   int unit, WarpScratch ws, LaneStats& st) {
+                                   int unit, WarpScratch ws, LaneStats& st_out) {
+    LaneStats st;   // lanes past the end repeat a node: their work is not credited
+    st.zero();
     const int lane = threadIdx.x & 31;
     const int D = M.H->n_dof, NJ = M.H->n_joints;
     const int j0 = unit * kCoarseUnit;
@@ -261,7 +263,7 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
     }
     if (!ok) return valid;   // uniform
     __syncwarp();
-    if (kStats && lane < nv) st.v[ST_SAMPLES] += 1;
+    if (kStats) st.v[ST_SAMPLES] += 1;
     // spacings from the node to the farthest sample it stands for
     const bool start = unit == 0 && node == 0 && (G % 16) != 0;
     const float x = start ? 0.5f * (kStride + 1) / kStride : 0.5f * (kStride - 1) / kStride;
@@ -363,8 +365,10 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
                         sphere_world(T, sp.x, sp.y, sp.z, px[i], py[i], pz[i]);
                         lim[i] = (fabsf(sp.w) + am + move + turn + g) * sc.Mscale;
                     }
+                    int met = 0;
 #pragma unroll 1
                     for (unsigned m = mask; m && !fail; m &= m - 1) {
+                        if (kStats) ++met;
                         const ObbPrep& o = sc.obbs[ws.cand[c0 + __ffs(m) - 1]];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
@@ -373,14 +377,17 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
                         }
                     }
                     if (kStats) {
-                        st.v[ST_SPHERES] += 4;
-                        st.v[ST_PAIRS] += 4 * __popc(mask);
+                        const int ns = min(4, jr.sph_end - k);
+                        st.v[ST_SPHERES] += ns;
+                        st.v[ST_PAIRS] += ns * met;
                     }
                 }
             }
         }
         if ((__ballot_sync(kFull, fail) & valid) == valid) break;   // uniform
     }
+    if (kStats && lane < nv)
+        for (int k = 0; k < ST_COUNT; ++k) st_out.v[k] += st.v[k];
     return __ballot_sync(kFull, fail) & valid;
 }
 

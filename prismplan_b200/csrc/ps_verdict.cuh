@@ -673,7 +673,7 @@ __device__ bool group_self_hit(const ModelSmem& M, const ModelDev& md, const flo
             need |= ref_self_hit(at(apos, i, 0), at(apos, i, 1), at(apos, i, 2), M.A[i].w, at(apos, j, 0),
                                  at(apos, j, 1), at(apos, j, 2), M.A[j].w);
         }
-        st.v[ST_SELF] += 4;
+        st.v[ST_SELF] += min(4, (na - k0 + kSelfSub - 1) / kSelfSub);   // the last pair again is no pair
     }
     if (!__ballot_sync(gmask, need)) return false;
     // joint pairs (a, q), nearest in DFS order first, one per lane: a pair
@@ -719,7 +719,7 @@ __device__ bool group_self_hit(const ModelSmem& M, const ModelDev& md, const flo
                         const int j = j0 + min(k + v, len - 1);
                         hit |= ref_self_hit(px, py, pz, ri, at(pos, j, 0), at(pos, j, 1), at(pos, j, 2), M.S[j].w);
                     }
-                    st.v[ST_SELF] += 4;
+                    st.v[ST_SELF] += min(4, len - k);
                 }
             }
         }
