@@ -80,6 +80,8 @@ struct ModelDev {
                                    // sliding joint k: its motion is the same everywhere), sliding joints between
                                    // them out by at most slide_max
     float slide_max;
+    const float2* lengths;         // device [n_joints], DFS positions: lengths of the fixed transform's translation and
+                                   // of the bound centre, never below them
     int* status;                   // device error latch
     int bytes_core;
     int stage_polls;               // polls of the staging wait before a kernel gives up

@@ -239,7 +239,7 @@ constexpr float kCoarseMaxQ = 16.0f;
 // shown free. Lane 0 of unit 0 also stands for the start configuration when
 // G % 16 != 0. Every lane of the warp calls it.
 template <bool kStats>
-__device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, const ps_edge_params& P,
+__device__ unsigned process_coarse(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc, const ps_edge_params& P,
                                    const float* __restrict__ from, const float* __restrict__ to, int e, int G,
                                    int unit, WarpScratch ws, LaneStats& st_out) {
     LaneStats st;   // lanes past the end repeat a node: their work is not credited
@@ -288,7 +288,7 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
             } else {
                 joint_compose<true>(jr, qi, T, T);   // rows are read before they are written
             }
-            const float link = len_up(jr.ft[3], jr.ft[7], jr.ft[11]);
+            const float link = __ldg(md.lengths + p).x;
             if (jr.type >= PS_X_ROT) {
                 Ao = fmaf(link, fmaf(W, W, Al), Ao);
                 Al = fmaf(di, W, Al);
@@ -303,7 +303,7 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
         sphere_world(T, jr.bound.x, jr.bound.y, jr.bound.z, cx, cy, cz);
         const float nx = __shfl_sync(kFull, cx, nb) - cx, ny = __shfl_sync(kFull, cy, nb) - cy,
                     nz = __shfl_sync(kFull, cz, nb) - cz;
-        const float Ac = fmaf(len_up(jr.bound.x, jr.bound.y, jr.bound.z), fmaf(W, W, Al), Ao);
+        const float Ac = fmaf(__ldg(md.lengths + p).y, fmaf(W, W, Al), Ao);
         // how far any point of the joint's spheres moves, and the ball around them
         const float dn = fmaxf(fmaf(nz, nz, fmaf(ny, ny, nx * nx)), 1.0e-30f);
         const float move = (x * dn * rsqrtf(dn) + 0.5f * (x + x * x) * Ac) * 1.001f;
@@ -394,7 +394,7 @@ __device__ unsigned process_coarse(const ModelSmem& M, const SceneSmem& sc, cons
 // A work unit of an edge: whether any of its samples collides. A unit of more
 // than one chunk is first passed coarsely.
 template <bool kStats>
-__device__ __forceinline__ bool process_unit(const ModelSmem& M, const SceneSmem& sc, const ps_scene_view& sv,
+__device__ __forceinline__ bool process_unit(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc, const ps_scene_view& sv,
                                              const ps_edge_params& P, const float* __restrict__ from,
                                              const float* __restrict__ to, int e, int G, int unit, WarpScratch ws,
                                              LaneStats& st) {
@@ -405,7 +405,7 @@ __device__ __forceinline__ bool process_unit(const ModelSmem& M, const SceneSmem
     bool last = false;      // the start configuration, which rides with the edge's last chunk
     if (unit < 0) {   // ~unit of a long edge; else a chunk
         unit = ~unit;
-        left = process_coarse<kStats>(M, sc, P, from, to, e, G, unit, ws, st);
+        left = process_coarse<kStats>(M, md, sc, P, from, to, e, G, unit, ws, st);
         if (!left) return false;
         first = unit * kStride;
         chunks = 0;
@@ -981,7 +981,7 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
             retired = __shfl_sync(kFull, retired, 0);
             if (!P.compute_clearance && retired) continue;   // retired meanwhile
             float cm = FLT_MAX;
-            const bool h = kMode == 3 ? process_unit<kStats>(M, sc, sv, P, from, to, ee, GG, kk, ws, st)
+            const bool h = kMode == 3 ? process_unit<kStats>(M, md, sc, sv, P, from, to, ee, GG, kk, ws, st)
                            : kMode  ? process_chunk_fast<kStats, kMode == 2>(M, sc, sv, P.collision_margin, from, to, ee, GG,
                                                                             32 * kk, ws, st)
                                     : process_chunk(M, sc, sv, P, from, to, ee, GG, kk, ws,

@@ -345,6 +345,8 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     off += align16(sizeof(float) * nd);
     const size_t off_lever = off;
     off += align16(sizeof(float) * nj * nj);
+    const size_t off_lengths = off;
+    off += align16(sizeof(float2) * nj);
     const size_t off_status = off;
     off += 16;
     const size_t total = align16(off);
@@ -463,6 +465,16 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     std::memcpy(host.data() + off_lower, d->joint_lower, sizeof(float) * nd);
     std::memcpy(host.data() + off_upper, d->joint_upper, sizeof(float) * nd);
 
+    {
+        const JointRec* J = reinterpret_cast<const JointRec*>(host.data() + h.off_joints);
+        float2* L = reinterpret_cast<float2*>(host.data() + off_lengths);
+        auto up = [](float x, float y, float z) {
+            return (float)(std::sqrt((double)x * x + (double)y * y + (double)z * z) * (1.0 + 1e-6));
+        };
+        for (int p = 0; p < nj; ++p)
+            L[p] = make_float2(up(J[p].ft[3], J[p].ft[7], J[p].ft[11]), up(J[p].bound.x, J[p].bound.y, J[p].bound.z));
+    }
+
     // levers (ModelDev::lever), for rigid transforms
     float slide_max = 1.0f;
     {
@@ -516,6 +528,7 @@ extern "C" int ps_model_create(const ps_model_desc* d, ps_model** out) {
     m->dev.upper = reinterpret_cast<const float*>(base + off_upper);
     m->dev.lever = reinterpret_cast<const float*>(base + off_lever);
     m->dev.slide_max = slide_max;
+    m->dev.lengths = reinterpret_cast<const float2*>(base + off_lengths);
     m->dev.status = reinterpret_cast<int*>(base + off_status);
     m->dev.bytes_core = (int)core;
     m->dev.stage_polls = PS_STAGE_POLLS;
