@@ -122,7 +122,7 @@ size_t waypoint_smem_bytes(const ps_model* m, const ps_scene_view* sv, int warps
 // waypoints fill [0, n_wp) of the packed rows, rollout waypoints
 // [cap - n_roll, cap); a warp takes its waypoints from one range, so rollout
 // warps run without the adjoint.
-template <int kWarps>
+template <int kWarps, bool kEsdf>
 __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) batch_waypoint_kernel(ModelDev md, ps_scene_view sv,
                                                                                  ps_cost_params P,
                                                                                  const Counts* __restrict__ cnt,
@@ -174,13 +174,13 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) batch_waypoint_kerne
         __syncwarp();
         st.zero();
         if (traj) {
-            const float v = lane_cost<true, false>(M, md, sc, sv, P, cb, ws, st);
+            const float v = lane_cost<true, false, kEsdf>(M, md, sc, sv, P, cb, ws, st);
             if (k < hi) {
                 if (u == 0) wp_cost[k] = v;
                 lane_write_grad(M, cb, ws, grad + (size_t)k * D, 1);
             }
         } else {
-            const float v = lane_cost<false, false>(M, md, sc, sv, P, cb, ws, st);
+            const float v = lane_cost<false, false, kEsdf>(M, md, sc, sv, P, cb, ws, st);
             if (k < hi && u == 0) wp_cost[k] = v;
         }
     }
@@ -365,13 +365,13 @@ __global__ void __launch_bounds__(kW * 32, 16 / kW)
             for (int d = u; d < D; d += kCostSub) lane_put_q(ws, slot, d, q[(size_t)kc * D + d]);
             __syncwarp();
             if (traj) {
-                const float v = lane_cost<true, false>(M, md, sc, sv, CP, cb, ws, st);
+                const float v = lane_cost<true, false, kMode != 1>(M, md, sc, sv, CP, cb, ws, st);
                 if (k < hi) {
                     if (u == 0) wp_cost[k] = v;
                     lane_write_grad(M, cb, ws, grad + (size_t)k * D, 1);
                 }
             } else {
-                const float v = lane_cost<false, false>(M, md, sc, sv, CP, cb, ws, st);
+                const float v = lane_cost<false, false, kMode != 1>(M, md, sc, sv, CP, cb, ws, st);
                 if (k < hi && u == 0) wp_cost[k] = v;
             }
         }
@@ -493,8 +493,9 @@ WorkKernel pick_work_kernel(int mode, int threads) {
 using WaypointKernel = void (*)(ModelDev, ps_scene_view, ps_cost_params, const Counts*, const float*, float*, float*,
                                 int);
 
-WaypointKernel pick_waypoint_kernel(int threads) {
-    return threads == 128 ? batch_waypoint_kernel<4> : batch_waypoint_kernel<8>;
+WaypointKernel pick_waypoint_kernel(int threads, bool esdf) {
+    if (esdf) return threads == 128 ? batch_waypoint_kernel<4, true> : batch_waypoint_kernel<8, true>;
+    return threads == 128 ? batch_waypoint_kernel<4, false> : batch_waypoint_kernel<8, false>;
 }
 
 // Everything that is not a stream operation happens before the capture.
@@ -530,7 +531,7 @@ int plan_launch(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep, 
     if (b->lim.max_waypoints > 0) {
         const int tt = b->traj_threads;
         L.wsmem = waypoint_smem_bytes(m, sv, tt / 32);
-        L.wk = pick_waypoint_kernel(tt);
+        L.wk = pick_waypoint_kernel(tt, sv->n_voxel_layers > 0);
         int per_sm = 0;
         PS_TRY_CUDA(allow_smem((const void*)L.wk, L.wsmem));
         PS_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, L.wk, tt, L.wsmem));
@@ -545,7 +546,7 @@ int plan_launch(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep, 
         L.slices_t = request_slices(L.req_grid_t);
     }
     if (b->layout == 1) {   // one work-queue kernel for edge chunks and waypoint groups
-        const int mode = b->lim.max_edges > 0 ? L.mode : 1;
+        const int mode = b->lim.max_edges > 0 ? L.mode : (sv->n_voxel_layers > 0 ? 2 : 1);   // 1: no ESDF layers
         const int kt = b->work_threads;
         L.work = pick_work_kernel(mode, kt);
         L.ksmem = work_smem_bytes(m, sv, kt / 32, std::min(b->work_cost_warps, kt / 32));

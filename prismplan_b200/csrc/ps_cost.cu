@@ -37,7 +37,7 @@ size_t cost_block_smem(const ps_model* m, const ps_scene_view* sv, bool grad) {
 // NULL): rows b with skip[b] != 0 need no output and get none; a warp whose
 // rows are all skipped does nothing. A waypoint gets the same bits whichever
 // rows share its warp.
-template <bool kGrad, bool kStats>
+template <bool kGrad, bool kStats, bool kEsdf>
 __global__ void __launch_bounds__(kLaneCostWarps * 32, 2) waypoint_cost_kernel(
     ModelDev md, ps_scene_view sv, const float* __restrict__ q, int n_rows, int T, ps_cost_params P,
     float* __restrict__ wp_cost, int broadcast_d, float* __restrict__ traj_acc, float* __restrict__ grad,
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kLaneCostWarps * 32, 2) waypoint_cost_kernel(
         __syncwarp();
         LaneStats ls;
         ls.zero();
-        const float cost = lane_cost<kGrad, kStats>(M, md, sc, sv, P, cb, ws, ls);
+        const float cost = lane_cost<kGrad, kStats, kEsdf>(M, md, sc, sv, P, cb, ws, ls);
         if (!live) continue;
         if (kStats) {
             if (u == 0) ls.v[ST_SAMPLES] += 1;
@@ -118,6 +118,13 @@ __global__ void __launch_bounds__(kLaneCostWarps * 32, 2) waypoint_cost_kernel(
                             bdt ? T : 1);
     }
     if (kStats) flush_stats(stats, st);
+}
+
+template <bool kGrad>
+auto pick_cost(const ps_scene_view* scene) {
+    if (scene->n_voxel_layers > 0)
+        return g_stats ? waypoint_cost_kernel<kGrad, true, true> : waypoint_cost_kernel<kGrad, false, true>;
+    return g_stats ? waypoint_cost_kernel<kGrad, true, false> : waypoint_cost_kernel<kGrad, false, false>;
 }
 
 // Per trajectory: smoothness cost and its gradient added to grad (see
@@ -183,7 +190,7 @@ int ps::traj_cost_launch(const ps_model* m, const ps_scene_view* scene, const fl
     if (atomic_traj) PS_TRY_CUDA(cudaMemsetAsync(traj_cost, 0, sizeof(float) * B, s));
     if (grad) {
         const size_t smem = cost_block_smem(m, scene, true);
-        auto k = g_stats ? waypoint_cost_kernel<true, true> : waypoint_cost_kernel<true, false>;
+        auto k = pick_cost<true>(scene);
         const int grid = cost_grid(k, smem, total);
         if (grid < 0) return PS_EINVAL;
         mark_start(s);
@@ -192,7 +199,7 @@ int ps::traj_cost_launch(const ps_model* m, const ps_scene_view* scene, const fl
         mark_stop(s);
     } else {
         const size_t smem = cost_block_smem(m, scene, false);
-        auto k = g_stats ? waypoint_cost_kernel<false, true> : waypoint_cost_kernel<false, false>;
+        auto k = pick_cost<false>(scene);
         const int grid = cost_grid(k, smem, total);
         if (grid < 0) return PS_EINVAL;
         mark_start(s);
@@ -231,7 +238,7 @@ extern "C" int ps_rollout_costs(const ps_model* m, const ps_scene_view* scene, c
     cudaStream_t s = (cudaStream_t)stream;
     const long long total = (long long)n_rows * T;
     const size_t smem = cost_block_smem(m, scene, false);
-    auto k = g_stats ? waypoint_cost_kernel<false, true> : waypoint_cost_kernel<false, false>;
+    auto k = pick_cost<false>(scene);
     const int grid = cost_grid(k, smem, total);
     if (grid < 0) return PS_EINVAL;
     mark_start(s);

@@ -242,8 +242,12 @@ __device__ __forceinline__ void lane_key_masked(const SceneSmem& sc, const uint1
 
 // Hinge terms of one sphere (box key already found): adds the OBB and ESDF
 // hinges to the lane's partial sums and, with kGrad, returns the force on the
-// sphere in (gx, gy, gz).
-template <bool kGrad, bool kStats>
+// sphere in (gx, gy, gz). kEsdf: the scene may have ESDF layers. Their lookups,
+// a cell's eight loads in flight together in each of four copies, cost the
+// sphere loop registers and code where there are none: 131,072 waypoints of a
+// 59-sphere arm among 96 boxes took 272 us with the loads one by one, 298 with
+// them together, 211 without lookups.
+template <bool kGrad, bool kStats, bool kEsdf>
 __device__ __forceinline__ void lane_sphere_terms(const ModelSmem& M, const SceneSmem& sc, const ps_scene_view& sv,
                                                   const ps_cost_params& P, int k, float px, float py, float pz,
                                                   float r, bool have_key, float key, int arg, float& obb_part,
@@ -264,7 +268,7 @@ __device__ __forceinline__ void lane_sphere_terms(const ModelSmem& M, const Scen
             }
         }
     }
-    if (sc.n_layers) {
+    if (kEsdf && sc.n_layers) {
         const int so = M.SO[k];
         const uint8_t* eacm = sv.sphere_acm_mask ? sv.sphere_acm_mask + (size_t)so * sv.n_voxel_layers : nullptr;
         if (sv.esdf_mode == PS_ESDF_TRILINEAR) {
@@ -308,7 +312,7 @@ __device__ __forceinline__ void lane_sphere_terms(const ModelSmem& M, const Scen
 // Cost of the lane group's waypoint (its configuration in ws.q) and, with
 // kGrad, the per-joint gradient in ws.dq. Every lane of the warp calls it; the
 // result is the same on the kCostSub lanes of a group.
-template <bool kGrad, bool kStats>
+template <bool kGrad, bool kStats, bool kEsdf>
 __device__ float lane_cost(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc, const ps_scene_view& sv,
                            const ps_cost_params& P, const CostBlock& cb, const LaneScratch& ws, LaneStats& st) {
     const float4* __restrict__ obs = cb.obs;
@@ -433,7 +437,7 @@ __device__ float lane_cost(const ModelSmem& M, const ModelDev& md, const SceneSm
                 ws.pos[(kk[i] * 3 + 1) * kCostSlots + slot] = py[i];
                 ws.pos[(kk[i] * 3 + 2) * kCostSlots + slot] = pz[i];
                 float gx, gy, gz;
-                lane_sphere_terms<kGrad, kStats>(M, sc, sv, P, kk[i], px[i], py[i], pz[i], rr[i], ncand > 0, key[i],
+                lane_sphere_terms<kGrad, kStats, kEsdf>(M, sc, sv, P, kk[i], px[i], py[i], pz[i], rr[i], ncand > 0, key[i],
                                                  arg[i], obb_part, esdf_part, gx, gy, gz, st);
                 if (kGrad) {
                     Fx += gx;
