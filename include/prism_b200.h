@@ -513,16 +513,17 @@ int ps_batch_add_rollouts(ps_batch* batch, const float* rollouts, int n_rows, in
 int ps_batch_launch(ps_batch* batch, const ps_scene_view* scene,
                     const ps_edge_params* params, const ps_cost_params* cost,
                     void* stream);
-/* Autotuner: times every candidate split of the SMs between the edge and the
-   trajectory branch, every trajectory block width and tile size on the
-   batch's current requests, keeps the fastest for later launches and
-   reports it (out may be NULL). Synchronous; launches the batch several
-   times. */
 /* Use this launch shape from the next launch on (for example one that
    ps_batch_tune returned earlier); best_ms and traj_tile are ignored.
    Shares in (0, 1], thread counts 128 or 256, layout 0 or 1,
    work_cost_warps 1 .. work_threads / 32. */
 int ps_batch_set_shape(ps_batch* batch, const ps_batch_tuning* shape);
+/* Autotuner: times every shape (the two branches by their shares of the SMs
+   and block width, the work-queue kernel by threads and warps that also take
+   waypoints) on the batch's current requests, the median of a few launches
+   each, the fastest three once more over more launches, keeps the fastest for
+   later launches and reports it (out may be NULL). Synchronous; launches the
+   batch some 140 times. */
 int ps_batch_tune(ps_batch* batch, const ps_scene_view* scene,
                   const ps_edge_params* params, const ps_cost_params* cost,
                   ps_batch_tuning* out);

@@ -909,15 +909,45 @@ extern "C" int ps_batch_set_shape(ps_batch* b, const ps_batch_tuning* shape) {
     return PS_OK;   // the next launch captures a graph for the new shape
 }
 
+// Median of a shape's timed launches.
+static float tune_median(std::vector<float>& ms) {
+    std::sort(ms.begin(), ms.end());
+    return ms[ms.size() / 2];
+}
+
 extern "C" int ps_batch_tune(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep,
                              const ps_cost_params* cp, ps_batch_tuning* out) {
     PS_NVTX("ps_batch_tune");
     clear_error();
     if (!b) return set_error(PS_EINVAL, "NULL batch");
-    const float edge_shares[] = {0.5f, 0.75f, 1.0f};
-    const float traj_shares[] = {0.25f, 0.5f, 1.0f};
-    const int widths[] = {128, 256};
-    const int tiles[] = {1};
+    // every shape: the work-queue kernel by threads per block and warps that also
+    // take waypoint groups (layout 1); the two branches by SM shares and block
+    // width (layout 0)
+    std::vector<ps_batch_tuning> cand;
+    const ps_batch_tuning keep{b->edge_share, b->traj_share, b->traj_threads, b->traj_tile, 0.0f,
+                               b->layout,     b->work_threads, b->work_cost_warps};
+    const bool edges = b->lim.max_edges > 0, trajs = b->lim.max_waypoints > 0;
+    const int work_shapes[][2] = {{256, 8}, {256, 4}, {256, 2}, {128, 4}, {128, 2}};
+    for (const auto& ws : work_shapes) {
+        if (!trajs && ws[1] != ws[0] / 32) continue;   // no waypoints: one shape per width
+        ps_batch_tuning t = keep;
+        t.layout = 1;
+        t.work_threads = ws[0];
+        t.work_cost_warps = ws[1];
+        cand.push_back(t);
+    }
+    for (float es : {0.5f, 0.75f, 1.0f})
+        for (float ts : {0.25f, 0.5f, 1.0f})
+            for (int w : {128, 256}) {
+                if ((!edges && es != 1.0f) || (!trajs && (ts != 0.5f || w != 256))) continue;
+                ps_batch_tuning t = keep;
+                t.layout = 0;
+                t.edge_share = es;
+                t.traj_share = ts;
+                t.traj_threads = w;
+                t.traj_tile = 1;
+                cand.push_back(t);
+            }
     cudaStream_t s = nullptr;
     cudaEvent_t a = nullptr, z = nullptr;
     PS_TRY_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -927,105 +957,50 @@ extern "C" int ps_batch_tune(ps_batch* b, const ps_scene_view* sv, const ps_edge
         cudaStreamDestroy(s);
         return cuda_error(le, "tuning events");
     }
-    const float keep_e = b->edge_share, keep_t = b->traj_share;
-    const int keep_w = b->traj_threads, keep_tile = b->traj_tile, keep_l = b->layout, keep_k = b->work_threads,
-              keep_c = b->work_cost_warps;
-    float best = 3.0e38f, best_e = keep_e, best_t = keep_t;
-    int best_w = keep_w, best_tile = keep_tile, best_l = keep_l, best_k = keep_k, best_c = keep_c;
-    int rc = PS_OK;
-    const bool edges = b->lim.max_edges > 0, trajs = b->lim.max_waypoints > 0;
-    auto time_now = [&](float& ms_min) {   // capture + warm-up, then the best of 3 launches
+    auto use = [&](const ps_batch_tuning& t) {
+        b->edge_share = t.edge_share;
+        b->traj_share = t.traj_share;
+        b->traj_threads = t.traj_threads;
+        b->traj_tile = t.traj_tile;
+        b->layout = t.layout;
+        b->work_threads = t.work_threads;
+        b->work_cost_warps = t.work_cost_warps;
+    };
+    // capture and warm-up, then the median of `reps` launches
+    auto time_now = [&](ps_batch_tuning& t, int reps) {
+        use(t);
         int r = ps_batch_launch(b, sv, ep, cp, s);
-        ms_min = 3.0e38f;
-        for (int k = 0; k < 3 && r == PS_OK; ++k) {
+        std::vector<float> ms;
+        for (int k = 0; k < reps && r == PS_OK; ++k) {
             cudaEventRecord(a, s);
             r = ps_batch_launch(b, sv, ep, cp, s);
             cudaEventRecord(z, s);
             if (cudaEventSynchronize(z) != cudaSuccess) r = cuda_error(cudaGetLastError(), "tuning run");
-            float ms = 0.0f;
-            cudaEventElapsedTime(&ms, a, z);
-            ms_min = std::min(ms_min, ms);
+            float v = 0.0f;
+            cudaEventElapsedTime(&v, a, z);
+            ms.push_back(v);
         }
+        if (r == PS_OK) t.best_ms = tune_median(ms);
         return r;
     };
-    // layout 1: one work-queue kernel; (threads per block, warps that also
-    // take waypoint groups)
-    const int work_shapes[][2] = {{256, 8}, {256, 4}, {256, 2}, {128, 4}, {128, 2}};
-    b->layout = 1;
-    for (const auto& ws : work_shapes) {
-        if (!trajs && ws[1] != ws[0] / 32) continue;   // no waypoints: one shape per width
-        b->work_threads = ws[0];
-        b->work_cost_warps = ws[1];
-        float ms_min = 0.0f;
-        rc = time_now(ms_min);
-        if (rc) break;
-        if (ms_min < best) {
-            best = ms_min;
-            best_l = 1;
-            best_k = ws[0];
-            best_c = ws[1];
-        }
-    }
-    b->layout = 0;
-    for (float es : edge_shares) {
-        if (rc) break;
-        if (!edges && es != 1.0f) continue;
-        for (float ts : traj_shares) {
-            for (int w : widths) {
-                for (int tl : tiles) {
-                    if (!trajs && (ts != 0.5f || w != 256 || tl != 1)) continue;
-                    b->edge_share = es;
-                    b->traj_share = ts;
-                    b->traj_threads = w;
-                    b->traj_tile = tl;
-                    float ms_min = 0.0f;
-                    rc = time_now(ms_min);
-                    if (rc) break;
-                    if (ms_min < best) {
-                        best = ms_min;
-                        best_l = 0;
-                        best_e = es;
-                        best_t = ts;
-                        best_w = w;
-                        best_tile = tl;
-                    }
-                }
-                if (rc) break;
-            }
-            if (rc) break;
-        }
-        if (rc) break;
-    }
+    // The fastest three are timed once more, longer: the best of 23 shapes by
+    // its shortest of three launches was once in six tunings one whose launches
+    // were lucky (0.412 ms by them, 0.463 in use, the right one 0.416).
+    int rc = PS_OK;
+    for (auto& t : cand)
+        if (rc == PS_OK) rc = time_now(t, 3);
+    const auto faster = [](const ps_batch_tuning& x, const ps_batch_tuning& y) { return x.best_ms < y.best_ms; };
+    std::stable_sort(cand.begin(), cand.end(), faster);
+    cand.resize(std::min<size_t>(cand.size(), 3));
+    for (auto& t : cand)
+        if (rc == PS_OK) rc = time_now(t, 15);
     cudaStreamSynchronize(s);
     cudaEventDestroy(a);
     cudaEventDestroy(z);
     cudaStreamDestroy(s);
-    if (rc) {
-        b->edge_share = keep_e;
-        b->traj_share = keep_t;
-        b->traj_threads = keep_w;
-        b->traj_tile = keep_tile;
-        b->layout = keep_l;
-        b->work_threads = keep_k;
-        b->work_cost_warps = keep_c;
-        return rc;
-    }
-    b->edge_share = best_e;
-    b->traj_share = best_t;
-    b->traj_threads = best_w;
-    b->traj_tile = best_tile;
-    b->layout = best_l;
-    b->work_threads = best_k;
-    b->work_cost_warps = best_c;
-    if (out) {
-        out->edge_share = best_e;
-        out->traj_share = best_t;
-        out->traj_threads = best_w;
-        out->traj_tile = best_tile;
-        out->best_ms = best;
-        out->layout = best_l;
-        out->work_threads = best_k;
-        out->work_cost_warps = best_c;
-    }
+    const ps_batch_tuning best = rc ? keep : *std::min_element(cand.begin(), cand.end(), faster);
+    use(best);
+    if (rc) return rc;
+    if (out) *out = best;
     return PS_OK;
 }
