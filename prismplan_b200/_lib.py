@@ -302,7 +302,9 @@ def stream_handle(stream) -> int | None:
     import torch
 
     if stream is None:
-        if torch.cuda.is_initialized():   # the handle itself, without a Stream object around it (3.5 -> 0.6 us)
-            return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) or None
+        # the handle itself, without a Stream object around it (3.5 -> 0.6 us), where this torch can tell it
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None and torch.cuda.is_initialized():
+            return raw(torch.cuda.current_device()) or None
         stream = torch.cuda.current_stream()
     return int(stream.cuda_stream) or None
