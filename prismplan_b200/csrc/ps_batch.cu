@@ -465,7 +465,7 @@ namespace {
 struct LaunchPlan {
     int mode = 0;
     void (*qk)(ModelDev, ps_scene_view, ps_edge_params, const float*, const float*, int, EdgeWs*, const int*, int*,
-               int*, int*, unsigned long long*, int, const int*, const int*, bool) = nullptr;
+               int*, int*, unsigned long long*, int, const int*, const int*, bool, EdgeOut) = nullptr;
     void (*wk)(ModelDev, ps_scene_view, ps_cost_params, const Counts*, const float*, float*, float*, int) = nullptr;
     void (*work)(ModelDev, ps_scene_view, ps_edge_params, ps_cost_params, const Counts*, const float*, const float*,
                  EdgeWs*, const int*, int*, int*, int*, const float*, float*, float*, int, int, int) = nullptr;
@@ -592,8 +592,8 @@ void record_work_graph(ps_batch* b, const ps_scene_view* sv, const ps_edge_param
             edges_self_kernel<<<L.sgrid, kSelfThreads, L.ssmem, s0>>>(m->dev, *ep, b->d_from, b->d_to, b->d_given,
                                                                       b->lim.max_edges, b->d_G, b->d_bad, nullptr,
                                                                       nullptr, b->d_hdr, nullptr, n_dev);
-        edges_finalize_kernel<<<L.pgrid, 256, 0, s0>>>(b->lim.max_edges, *ep, b->d_bad, b->d_len, b->d_clr, b->d_done,
-                                                       b->d_G, b->d_hdr, b->d_valid, b->d_cost, nullptr, n_dev);
+        edges_finalize_kernel<<<L.pgrid, 256, 0, s0>>>(b->lim.max_edges, *ep, b->d_bad, b->d_clr, b->d_done, b->d_G, b->d_hdr,
+                                                       EdgeOut{b->d_valid, b->d_cost, nullptr, b->d_len}, n_dev);
         batch_scatter_edges<<<L.req_grid_e, 128, 0, s0>>>(b->d_ereq, b->d_cnt, b->d_valid, b->d_cost);
     }
     if (trajs)
@@ -630,16 +630,16 @@ void record_graph(ps_batch* b, const ps_scene_view* sv, const ps_edge_params* ep
                                                                           b->d_bad, nullptr, n_dev, PrepArgs{});
         L.qk<<<L.qgrid, kEdgeThreads, L.qsmem, s0>>>(m->dev, *sv, *ep, b->d_from, b->d_to, b->lim.max_edges, b->d_hdr,
                                                     b->d_G, b->d_bad, b->d_clr, b->d_done, nullptr, 0, n_dev, nullptr,
-                                                    false);
+                                                    false, EdgeOut{});
         L.qk<<<L.qgrid, kEdgeThreads, L.qsmem, s0>>>(m->dev, *sv, *ep, b->d_from, b->d_to, b->lim.max_edges, b->d_hdr,
                                                     b->d_G, b->d_bad, b->d_clr, b->d_done, nullptr, 1, n_dev, nullptr,
-                                                    false);
+                                                    false, EdgeOut{});
         if (ep->check_self)
             edges_self_kernel<<<L.sgrid, kSelfThreads, L.ssmem, s0>>>(m->dev, *ep, b->d_from, b->d_to, b->d_given,
                                                                       b->lim.max_edges, b->d_G, b->d_bad, nullptr,
                                                                       nullptr, b->d_hdr, nullptr, n_dev);
-        edges_finalize_kernel<<<L.pgrid, 256, 0, s0>>>(b->lim.max_edges, *ep, b->d_bad, b->d_len, b->d_clr, b->d_done,
-                                                       b->d_G, b->d_hdr, b->d_valid, b->d_cost, nullptr, n_dev);
+        edges_finalize_kernel<<<L.pgrid, 256, 0, s0>>>(b->lim.max_edges, *ep, b->d_bad, b->d_clr, b->d_done, b->d_G, b->d_hdr,
+                                                       EdgeOut{b->d_valid, b->d_cost, nullptr, b->d_len}, n_dev);
         batch_scatter_edges<<<L.req_grid_e, 128, 0, s0>>>(b->d_ereq, b->d_cnt, b->d_valid, b->d_cost);
     }
     if (b->lim.max_waypoints > 0) {   // trajectory branch on s1

@@ -840,8 +840,6 @@ int plan_probe(const ps_model* m, const ps_scene_view* sv, int mode, bool stats,
     return PS_OK;
 }
 
-// kMode: 0 generic, 1 boxes only, 2 boxes and ESDF layers, 3 boxes only with
-// the coarse pass over long edges.
 // Whether the long edges of a batch that may be passed coarsely (coarse_path)
 // are. The pass costs an edge that collides more than chunks do, so it depends
 // on how many long edges the end-sample probe retired: with 11, 16, 23 and 27 %
@@ -852,6 +850,34 @@ __device__ __forceinline__ bool coarse_now(const EdgeWs* hdr) {
     return 10 * (v >> 32) < 3 * (v & 0xffffffffull);
 }
 
+// Results of a batch: the caller's arrays, and the edges' lengths.
+struct EdgeOut {
+    uint8_t* valid;
+    float* cost;
+    float* clearance;   // may be NULL
+    const float* len;
+};
+
+// After a timeout an edge that is neither retired nor complete comes back
+// invalid (cost FLT_MAX): not shown free. Its clearance is the min over the
+// samples that were checked. With check_self an edge is free only when the
+// self pass marked it so (bad == 2). The grid shares the edges.
+__device__ __forceinline__ void finalize_edges(int n_edges, const ps_edge_params& P, const int* __restrict__ bad,
+                                               const int* __restrict__ clr, const int* __restrict__ done,
+                                               const int* __restrict__ Gs, const EdgeWs* hdr, const EdgeOut& out) {
+    const bool timed_out = hdr->timed_out != 0;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x) {
+        const int bv = bad[e];
+        const bool b = (P.check_self ? bv != 2 : bv != 0) || (timed_out && done[e] < ChunkOrder(Gs[e]).nc);
+        out.valid[e] = b ? 0 : 1;
+        out.cost[e] = b ? FLT_MAX : out.len[e];
+        if (out.clearance) out.clearance[e] = P.compute_clearance ? unordered_float(clr[e]) : FLT_MAX;
+    }
+}
+
+// The queue. kMode: 0 generic, 1 boxes only, 2 boxes and ESDF layers, 3 boxes
+// only with the coarse pass over long edges.
+//
 // Residency per variant, measured: the boxes-only fast path runs fastest
 // with 5 blocks per SM (room for 96 registers), the ESDF variant with 6.
 template <int kMode, bool kStats>
@@ -862,10 +888,17 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
                                                                   int* clr, int* done, unsigned long long* stats,
                                                                   int pass, const int* n_dev = nullptr,
                                                                   const int* __restrict__ lst = nullptr,
-                                                                  bool either = false) {
+                                                                  bool either = false, EdgeOut out = EdgeOut{}) {
     if (n_dev) n_edges = *n_dev;
-    // either: a launch of mode 1 and one of mode 3, of which one runs
-    if (either && (kMode == 3) != coarse_now(hdr)) return;
+    // either: a launch of mode 1 and one of mode 3 behind it, of which one runs
+    // the queue. The other one writes the results (out, unless the self pass
+    // has yet to come): mode 3 what mode 1 found; mode 1 what the probe found,
+    // to which mode 3 adds its hits. A launch with nothing to do and the
+    // finalize kernel cost 2.4 us each and a gap.
+    if (either && (kMode == 3) != coarse_now(hdr)) {
+        if (out.valid) finalize_edges(n_edges, P, bad, clr, done, Gs, hdr, out);
+        return;
+    }
     // Rounds of this launch. With many edges per resident warp (>= 8) one
     // launch (pass 0) runs every round and pass 1 returns at once. With fewer,
     // round 1 would start while much of round 0 is still in flight and check
@@ -901,6 +934,11 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
         // fail closed: finalize reports every edge that is neither retired
         // nor complete as invalid, and the status query PS_ETIMEOUT
         if (threadIdx.x == 0) atomicExch(&hdr->timed_out, 1);
+        if (kMode == 3 && out.valid)   // the results are there already
+            for (int e = threadIdx.x; e < n_edges; e += blockDim.x) {
+                out.valid[e] = 0;
+                out.cost[e] = FLT_MAX;
+            }
         return;
     }
     const ModelSmem M = model_view(smem);
@@ -988,6 +1026,10 @@ __global__ void __launch_bounds__(kEdgeThreads, kMode & 1 ? 5 : (kMode ? 6 : 3))
                                                     P.compute_clearance ? &cm : nullptr, st);
             if (lane == 0) {
                 if (h) vbad[ee] = 1;
+                if (kMode == 3 && h && out.valid) {
+                    out.valid[ee] = 0;
+                    out.cost[ee] = FLT_MAX;
+                }
                 if (P.compute_clearance) atomicMin(clr + ee, ordered_float(cm));
                 if (deadline) atomicAdd(done + ee, 1);   // completed chunks, read only after a timeout
             }
@@ -1135,24 +1177,12 @@ __global__ void __launch_bounds__(kSelfThreads, 6) edges_self_kernel(ModelDev md
     flush_stats(stats, st);
 }
 
-// After a timeout an edge that is neither retired nor complete comes back
-// invalid (cost FLT_MAX): not shown free. Its clearance is the min over the
-// samples that were checked. With check_self an edge is free only when the
-// self pass marked it so (bad == 2).
 __global__ void edges_finalize_kernel(int n_edges, const ps_edge_params P, const int* __restrict__ bad,
-                                      const float* __restrict__ len, const int* __restrict__ clr,
-                                      const int* __restrict__ done, const int* __restrict__ Gs, const EdgeWs* hdr,
-                                      uint8_t* __restrict__ valid, float* __restrict__ cost,
-                                      float* __restrict__ clearance, const int* n_dev = nullptr) {
+                                      const int* __restrict__ clr, const int* __restrict__ done,
+                                      const int* __restrict__ Gs, const EdgeWs* hdr, EdgeOut out,
+                                      const int* n_dev = nullptr) {
     if (n_dev) n_edges = *n_dev;
-    const bool timed_out = hdr->timed_out != 0;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x) {
-        const int bv = bad[e];
-        const bool b = (P.check_self ? bv != 2 : bv != 0) || (timed_out && done[e] < ChunkOrder(Gs[e]).nc);
-        valid[e] = b ? 0 : 1;
-        cost[e] = b ? FLT_MAX : len[e];
-        if (clearance) clearance[e] = P.compute_clearance ? unordered_float(clr[e]) : FLT_MAX;
-    }
+    finalize_edges(n_edges, P, bad, clr, done, Gs, hdr, out);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }

@@ -326,22 +326,25 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
         probe.kp<<<probe.grid, kProbeThreads, probe.smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G,
                                                                 b.bad, g_stats, nullptr,
                                                                 PrepArgs{samples_per_edge, b.len, b.clr, b.done, lst});
+    const EdgeOut out{valid, cost, clearance, b.len};
+    const EdgeOut early = coarse && !P->check_self ? out : EdgeOut{};   // written by the queue's launches
     qk<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
-                                         g_stats, 0, nullptr, lst, coarse);
+                                         g_stats, 0, nullptr, lst, coarse, early);
     if (coarse)   // one pass (not split); the probe's counts say which of the two runs
         qk3<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
-                                              g_stats, 0, nullptr, lst, true);
+                                              g_stats, 0, nullptr, lst, true, early);
     if (split)
         qk<<<qgrid, kEdgeThreads, smem, s>>>(m->dev, *scene, *P, from, to, n_edges, b.hdr, b.G, b.bad, b.clr, b.done,
-                                             g_stats, 1, nullptr, lst, false);
+                                             g_stats, 1, nullptr, lst, false, EdgeOut{});
     mark_stop(s);
     PS_TRY_CUDA(cudaGetLastError());
     if (int rc = launch_edges_self(m, P, from, to, samples_per_edge, n_edges, b.G, b.bad, nullptr, nullptr, b.hdr,
                                    nullptr, s))
         return rc;
-    const int fgrid = std::max(1, std::min((n_edges + 255) / 256, sm_count() * 4));
-    edges_finalize_kernel<<<fgrid, 256, 0, s>>>(n_edges, *P, b.bad, b.len, b.clr, b.done, b.G, b.hdr, valid, cost,
-                                                clearance);
+    if (!early.valid) {
+        const int fgrid = std::max(1, std::min((n_edges + 255) / 256, sm_count() * 4));
+        edges_finalize_kernel<<<fgrid, 256, 0, s>>>(n_edges, *P, b.bad, b.clr, b.done, b.G, b.hdr, out);
+    }
     PS_TRY_CUDA(cudaGetLastError());
     return PS_OK;
 }
