@@ -151,3 +151,42 @@ def test_fine_steps_in_a_solve(golden, robot, boxes, esdf, self_check, T, step):
     r, m = (api.chomp_solve(b, sc, starts, goals, s) for sc in (plain, masked))
     for name in ("solved", "iterations", "cost", "path", "theta"):
         assert torch.equal(getattr(r, name), getattr(m, name)), name
+
+
+@pytest.mark.parametrize("n,self_check", [(10, True), (100, False), (300, True)])
+def test_captured_calls(golden, n, self_check):
+    """A captured call replayed on other edges, and two streams with a workspace each."""
+    import torch
+
+    from prismplan_b200 import api
+
+    asset, b = _robot(golden, "panda")
+    scene, _ = _ceiling(b, asset, gap=0.02, needle=0.3)
+    params = api.EdgeEvalParams(max_joint_step=0.01, check_self=self_check)
+    batches = []
+    for seed in range(3):
+        frm, to, _ = workloads.edge_batch(np.random.default_rng(seed), asset, n)
+        batches.append((torch.from_numpy(frm).cuda(), torch.from_numpy(to).cuda()))
+    want = [api.check_edges(b, scene, f, t, params=params, persistent=False)[:2] for f, t in batches]
+    f, t = (x.clone() for x in batches[0])
+    ws = api.edges_workspace(n)
+    api.check_edges(b, scene, f, t, params=params, workspace=ws)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        got = api.check_edges(b, scene, f, t, params=params, workspace=ws)
+    for (a, c), w in zip(batches, want):
+        f.copy_(a)
+        t.copy_(c)
+        g.replay()
+        assert torch.equal(got[0], w[0]) and torch.equal(got[1], w[1])
+    streams, out = [torch.cuda.Stream() for _ in batches], []
+    spaces = [api.edges_workspace(n) for _ in batches]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for s, (a, c), w in zip(streams, batches, spaces):
+            with torch.cuda.stream(s):
+                out.append(api.check_edges(b, scene, a, c, params=params, workspace=w))
+    torch.cuda.synchronize()
+    for k, o in enumerate(out):
+        assert torch.equal(o[0], want[k % 3][0]) and torch.equal(o[1], want[k % 3][1])
