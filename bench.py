@@ -264,9 +264,10 @@ def run_ours(args):
     del graph
     # Kernels per step: the preparation, or the end-sample probe whose launch
     # also prepares (when the tuned shape, or automatic with at least 8 warps
-    # of edges per SM, runs it); queue pass 0; finalize; and a second queue
-    # pass when the edges are fewer than 8 per resident warp (the tuned queue
-    # residency, or 5 blocks of 4 warps per SM for this kernel variant)
+    # of edges per SM, runs it); queue pass 0; finalize (or the second of the
+    # queue's two launches, which does that too); and a second queue pass when
+    # the edges are fewer than 8 per resident warp (the tuned queue residency,
+    # or 5 blocks of 4 warps per SM for this kernel variant)
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     qres = tuning["queue_blocks_per_sm"] or 5
     launches_per_step = 3 + (1 if E < 8 * sms * qres * 4 else 0)

@@ -164,7 +164,9 @@ typedef struct ps_scene_view {
 } ps_scene_view;
 
 /* =========================================================================
- * Batched configuration check (config-major, one lane per configuration).
+ * Batched configuration check (1, 4 or 16 lanes per configuration, by the
+ * batch size; one lane with masks, several FK slots, an approximate chain of
+ * its own, or clearance from ESDF layers).
  * Replaces pRRTC::check_collision_scene + check_collision_scene_kernel
  * (cpp/src/planning/pRRTC.cu:2337-2423) and prrtc.check_collision_scene
  * (cpp/src/python/bindings.cpp:493-532). The verdict is the two-phase one of

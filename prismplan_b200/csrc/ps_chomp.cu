@@ -15,9 +15,11 @@
 //   * R theta is the 5-tap stencil pair and A^-1 = (R + 1e-8 I)^-1 is applied
 //     as a banded Cholesky solve (bandwidth 4) in FP64, factored once per call
 //     on the device;
-//   * validity checks every segment with the persistent edge kernel (samples
-//     j / n_sub, n_sub = ceil(max segment length / collision_check_step)) and
-//     every waypoint with the configuration kernel, both with the self check;
+//   * validity checks every waypoint and every segment (samples j / n_sub,
+//     n_sub = ceil(max segment length / collision_check_step)), with the self
+//     check, in three launches (opt_check_kernel and the two behind it); models
+//     and scenes that those do not serve go through the configuration kernel and
+//     the persistent edge kernel;
 //   * the bookkeeping (best valid snapshot, polish budget, two-step convergence
 //     streak, iteration count) runs per request on the device, and a finished
 //     request is skipped by every later kernel.

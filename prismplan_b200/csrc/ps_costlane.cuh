@@ -246,7 +246,7 @@ __device__ __forceinline__ void lane_key_masked(const SceneSmem& sc, const uint1
 // a cell's eight loads in flight together in each of four copies, cost the
 // sphere loop registers and code where there are none: 131,072 waypoints of a
 // 59-sphere arm among 96 boxes took 272 us with the loads one by one, 298 with
-// them together, 211 without lookups.
+// them together, 213 without lookups.
 template <bool kGrad, bool kStats, bool kEsdf>
 __device__ __forceinline__ void lane_sphere_terms(const ModelSmem& M, const SceneSmem& sc, const ps_scene_view& sv,
                                                   const ps_cost_params& P, int k, float px, float py, float pz,
@@ -530,7 +530,9 @@ __device__ float lane_cost(const ModelSmem& M, const ModelDev& md, const SceneSm
                     float tb = cl + ri + 2.0e-6f * (fabsf(cl) + ri);
                     // four at a time, one branch for all: with a test and a branch each, a
                     // sphere's loads waited for the one before (16,384 waypoints with
-                    // gradient 43.0 us, now 41.3; 16 x 50 rollouts of 51 waypoints 28.0, now 25.7)
+                    // gradient 42.1 us, now 40.3; 131,072 among 96 boxes 246, now 213; 16 x 30
+                    // rollouts of 51 waypoints 26.9, now 24.6; with one sphere a link, where a
+                    // run is one pair, 131,072 waypoints 152, now 158)
                     for (int m = 0; m < len; m += 4) {   // past the end: the last sphere again
                         float d2[4], rj[4];
                         bool hit = false;

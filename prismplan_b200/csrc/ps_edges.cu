@@ -105,6 +105,11 @@ EdgeBufs carve_workspace(void* ws, int n_edges) {
 // over what the blocks left. The lists lie in the workspace's arrays: entry k
 // is edge lst[k] with G[k] samples, of which the units bad[k] (scene) and
 // clr[k] (self) are left; done[e] says that edge e of the list collides.
+//
+// Bound by latency: 4-lane groups walk one chain of joints each. 1009 edges of
+// 1 to 300 samples with self check among 64 boxes: 106 us a block each and 31
+// us for the list (a call 163 us when a block finished its edge, 127 now); 27
+// edges of 16 samples 21 us.
 // ---------------------------------------------------------------------------
 template <bool kEsdf>
 __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md, ps_scene_view sv, ps_edge_params P,
