@@ -260,9 +260,9 @@ size_t ps_edges_workspace_bytes(int n_edges);
 /* Persistent work-queue path: edges are cut into warp-sized sample chunks,
    ordered chunk-major and pulled from a global queue by a persistent grid;
    an edge found in collision retires its remaining chunks. Small batches (up
-   to 256 edges, 512 of at most 32 samples, 1024 with the self check, 64 with
-   ESDF layers; no masks, clearance, time budget or shape fields) run one block
-   per edge and share what those leave among all warps: same results. All
+   to 512 edges, 2048 with the self check or of 16 samples, 64 with ESDF
+   layers; no masks, clearance, time budget or shape fields) run one block per
+   edge and share what those leave among all warps: same results. All
    launches are capture-safe. workspace: device, >= ps_edges_workspace_bytes(n_edges). */
 int ps_check_edges(const ps_model* model, const ps_scene_view* scene,
                    const float* from, const float* to,

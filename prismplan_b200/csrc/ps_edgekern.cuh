@@ -1185,6 +1185,24 @@ __global__ void edges_finalize_kernel(int n_edges, const ps_edge_params P, const
     finalize_edges(n_edges, P, bad, clr, done, Gs, hdr, out);
 }
 
+// Launches a kernel that may start before the one in front of it in the stream
+// has ended; it waits for that one with cudaGridDependencySynchronize.
+template <class... Params, class... Args>
+int launch_dependent(void (*k)(Params...), int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    PS_TRY_CUDA(cudaLaunchKernelEx(&c, k, Params(args)...));
+    return PS_OK;
+}
+
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Launches the self pass when params ask for it (a no-op otherwise). The grid

@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md
     __shared__ PathBlock blk;
     PathSmem ps;
     SceneSmem sc;
+    cudaTriggerProgrammaticLaunchCompletion();   // edges_rest_kernel may stage its tables meanwhile
     if (!path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, false, ps, sc)) {   // fail closed
         if (threadIdx.x == 0) {
             atomicExch(&w.hdr->timed_out, 1);
@@ -146,15 +147,16 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md
         const float len = edge_length(a, b, D);
         const int G = edge_samples(P, given, e, a, b, D, len);
         const bool start = G > 0 && (G % 16) != 0;   // the start configuration belongs to the samples
-        // at most 32 intervals (single samples when they fit the groups), and the start by itself
+        // at most 32 intervals, the start in the first one, or single samples (33 with the start) when they fit the groups
         const int m = (G - 1) / kPathGroups + 1, n = G > 0 ? (G - 1) / m + 1 : 0;
         __syncthreads();   // the previous edge's readers of blk are done
         const int x = threadIdx.x;
         if (x == 0) blk.hit = blk.left[0] = blk.left[1] = 0;
-        if (x < n) blk.item[x] = PathItem{0, x * m + 1, x == n - 1 ? G : (x + 1) * m, self ? 3 : 1};
-        if (x == n && start) blk.item[x] = PathItem{0, 0, 0, self ? 3 : 1};
+        const bool apart = start && m == 1;
+        if (x < n) blk.item[x] = PathItem{0, x == 0 && start && !apart ? 0 : x * m + 1, x == n - 1 ? G : (x + 1) * m, self ? 3 : 1};
+        if (x == n && apart) blk.item[x] = PathItem{0, 0, 0, self ? 3 : 1};
         path_run<kEsdf>(
-            M, md, sc, sv, ps, P.collision_margin, self, blk, n + (start ? 1 : 0), G, false,
+            M, md, sc, sv, ps, P.collision_margin, self, blk, n + (apart ? 1 : 0), G, false, 1,
             [&](int, int i, float& ai, float& bi) {
                 ai = __ldg(a + i);
                 bi = __ldg(b + i);
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md
 __global__ void edges_list_kernel(ps_edge_params P, const float* __restrict__ from, const float* __restrict__ to,
                                   const int* __restrict__ given, int n_edges, int D, uint8_t* __restrict__ valid,
                                   float* __restrict__ cost, float* __restrict__ clearance, EdgeBufs w) {
+    cudaTriggerProgrammaticLaunchCompletion();
     for (int e = threadIdx.x; e < n_edges; e += blockDim.x) {
         const float* a = from + (size_t)e * D;
         const float* b = to + (size_t)e * D;
@@ -207,8 +210,6 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_rest_kernel(ModelDev md
                                                                      const float* __restrict__ to,
                                                                      uint8_t* __restrict__ valid,
                                                                      float* __restrict__ cost, EdgeBufs w) {
-    const int n = w.hdr->n_long;
-    if (n == 0) return;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ int counters[4];
@@ -216,7 +217,11 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_rest_kernel(ModelDev md
     PathSmem ps;
     SceneSmem sc;
     volatile int* hit = w.done;
-    if (!path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, true, ps, sc)) {   // fail closed
+    const bool staged = path_stage(md, sv, smem, &mbar, counters, &bmax, P.check_self != 0, true, ps, sc);
+    cudaGridDependencySynchronize();   // the kernel in front has written the list
+    const int n = w.hdr->n_long;
+    if (n == 0) return;
+    if (!staged) {   // fail closed
         if (threadIdx.x == 0) atomicExch(&w.hdr->timed_out, 1);
         for (int k = threadIdx.x; k < n; k += blockDim.x) {
             valid[w.lst[k]] = 0;
@@ -242,31 +247,38 @@ namespace {
 
 // Whether a batch runs one block per edge (edges_path_kernel): small ones,
 // where the queue path waits on its launches and on single warps. few: at most
-// 32 samples an edge. Measured (us, queue path / here, on scenes from an arm
-// among 16 boxes to a two-arm robot among 128, all at 0.01 rad steps unless
-// said otherwise): with the self check 64 edges 159 / 58 to 261 / 165, 1009
-// edges 242 / 131 to 541 / 385 but at 0.05 rad 323 / 327, 2048 edges 260 / 228
-// to 581 / 685; without, 64 edges 56 / 31 to 159 / 99, 200 edges 63 / 50 to
-// 208 / 115, 512 edges 119 / 90 but among large boxes 66 / 66; few samples
-// with the self check 1009 edges 95 / 52 to 227 / 194, 2048 to 269 / 334,
-// without 512 edges 40 / 33 to 138 / 83, 1009 45 / 52. With an ESDF layer in
-// reach few intervals are shown clear: 64 edges 138 / 71, with 5000 samples
-// each 156 / 133, 200 edges 156 / 148. What costs it most are edges that no
-// interval is clear of, at a box's side (the list's samples come on top of the
-// swept check): 40 / 43 for one of 1000 samples, 72 / 84 for 512 of 600.
-bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, int mode, int n_edges, bool few) {
+// 32 samples an edge (0: not known to be). Measured over three robots among 16
+// to 128 boxes (us, queue path / here; the most and the least it gains): with
+// the self check 64 edges 538 / 139 and 79 / 67, 1024 edges 1356 / 313 and 303 /
+// 279, 2048 edges 685 / 308 and, where most collide, 158 / 253; without, 64
+// edges 210 / 99 and 57 / 54, 400 edges 222 / 85 and 69 / 70, 1024 edges 256 /
+// 123 but 263 / 309; 16 samples an edge 2048 edges 183 / 113 and 58 / 67, 32
+// samples 1009 edges 118 / 91 and 45 / 52, 2048 edges 48 / 89. With an ESDF
+// layer in reach 64 edges 195 / 166 and 474 / 217. What costs most here are
+// edges that no interval is clear of, at a box's side (the list's samples come
+// on top of the swept check): 39 / 43 for one of 600 samples, 72 / 84 for 512.
+bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, int mode, int n_edges, int few) {
     if (mode == 0 || !m->rigid || g_stats || P->time_budget_ms > 0.0f) return false;   // (the counters live in the queue path)
     if (P->probe || P->queue_blocks_per_sm || P->grab) return false;   // the caller asks for a shape of the queue
-    const int most = mode == 2 ? 64 : (P->check_self ? 1024 : (few ? 512 : 256));
+    const int most = mode == 2 ? 64 : (P->check_self ? 2048 : (few ? std::min(2048, 32768 / few) : 512));
     return n_edges <= most && path_serves(m, scene, P->collision_margin, P->check_self != 0);
 }
 
-// Whether every sample of a batch goes on the list at once: while the device
-// holds a warp for each of the at most 32 x (1 + 4) tasks of an edge of 1024
-// samples. A block alone walks the swept check's chain of joints first: one
-// edge of the two-arm robot among 128 boxes 129 us with the self check and 84
-// without, 52 and 35 us from the list (queue path 49 and 45).
-bool tiny_batch(int n_edges) { return n_edges * 160 <= sm_count() * 4 * kPathWarps; }
+// Whether every sample of a tiny batch goes on the list at once. A block walks
+// the swept check's chain of joints first, and then its list is another
+// launch; with a warp of the device for each of an edge's tasks (up to 32 for
+// the scene and 128 for the self check with 1024 samples) that is slower: with
+// the self check (us, a block per edge / the list) 4 edges 61 / 43 to 151 / 115,
+// 12 edges 39 / 33 to 162 / 72 (two-arm robot among 128 boxes, 172 by the
+// queue). Without it fewer warps share the chunks: 1 edge of a 7-joint arm among
+// 16 boxes 28 / 29, 4 edges among 64 38 / 29 and of a two-arm robot among 40
+// 68 / 41, but 12 edges 27 / 33, and among many boxes for many joints the
+// chunks' own candidates cost more (1 edge of the two-arm robot among 80 72 /
+// 105, among 128 90 / 143).
+bool tiny_batch(const ps_model* m, const ps_scene_view* sv, bool self, int n_edges) {
+    if (self) return n_edges * 160 <= sm_count() * 4 * kPathWarps;
+    return n_edges <= 4 && m->info.n_joints * sv->n_obbs <= 1000;
+}
 
 // memset header -> prep -> end-sample probe -> queue pass(es) -> self pass ->
 // finalize on stream s.
@@ -276,8 +288,9 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
     const int D = m->info.n_dof;
     PS_TRY_CUDA(cudaMemsetAsync(b.hdr, 0, sizeof(EdgeWs), s));   // queue heads, deadline, max rounds, timeout
     const int mode = fast_path(m, scene, P);
-    // few samples an edge (fewer than a block checks without looking at intervals), as far as the call says
-    const bool few = !samples_per_edge && P->resolution <= 0.0f && P->max_joint_step <= 0.0f && P->granularity <= 32;
+    // few samples an edge (no more than a block checks without looking at intervals), as far as the call says
+    const bool fixed = !samples_per_edge && P->resolution <= 0.0f && P->max_joint_step <= 0.0f && P->granularity <= 32;
+    const int few = fixed ? std::max(P->granularity, 1) : 0;
     if (path_edges(m, scene, P, mode, n_edges, few)) {
         auto pk = mode == 2 ? edges_path_kernel<true> : edges_path_kernel<false>;
         auto rk = mode == 2 ? edges_rest_kernel<true> : edges_rest_kernel<false>;
@@ -287,14 +300,15 @@ int run_persistent(const ps_model* m, const ps_scene_view* scene, const float* f
         int rgrid = 1;
         if (int rc = rest_grid(rk, rsmem, rgrid)) return rc;
         mark_start(s);
-        const bool tiny = tiny_batch(n_edges);
+        const bool tiny = !few && tiny_batch(m, scene, self, n_edges);
         if (tiny)
             edges_list_kernel<<<1, 32, 0, s>>>(*P, from, to, samples_per_edge, n_edges, D, valid, cost, clearance, b);
         else
             pk<<<std::min(n_edges, sm_count() * 16), kPathThreads, psmem, s>>>(m->dev, *scene, *P, from, to, samples_per_edge,
                                                                           n_edges, valid, cost, clearance, b);
-        if (tiny || !few)   // few samples are settled by their block
-            rk<<<rgrid, kPathThreads, rsmem, s>>>(m->dev, *scene, *P, from, to, valid, cost, b);
+        if (!few)   // few samples are settled by their block
+            if (int rc = launch_dependent(rk, rgrid, kPathThreads, rsmem, s, m->dev, *scene, *P, from, to, valid, cost, b))
+                return rc;
         mark_stop(s);
         PS_TRY_CUDA(cudaGetLastError());
         return PS_OK;

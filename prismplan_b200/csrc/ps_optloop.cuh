@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md,
     if (x < n) blk.item[x] = PathItem{seg0 + x, 0, G, self ? 3 : 1};
     if (x == n && last) blk.item[x] = PathItem{T - 2, G + 1, G + 1, self ? 3 : 1};
     path_run<kEsdf>(
-        M, md, sc, sv, ps, margin, self, blk, n + (last ? 1 : 0), G, true,
+        M, md, sc, sv, ps, margin, self, blk, n + (last ? 1 : 0), G, true, 0,
         [&](int sg, int i, float& a, float& b) {
             a = th[sg * D + i];
             b = th[(sg + 1) * D + i];
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_refine_kernel(ModelDev md
         if (x == 0) blk.hit = blk.left[0] = blk.left[1] = 0;
         if (x < n) blk.item[x] = PathItem{sg, x * m + 1, min((x + 1) * m, G), item.y & 3};
         path_run<kEsdf>(
-            M, md, sc, sv, ps, margin, self, blk, n, G, false,
+            M, md, sc, sv, ps, margin, self, blk, n, G, false, 1,
             [&](int, int i, float& ai, float& ci) {
                 ai = a[i];
                 ci = c[i];

@@ -308,7 +308,8 @@ __device__ __forceinline__ unsigned path_sweep(const ModelSmem& M, const ModelDe
 struct PathItem {
     int seg, lo, hi, what;
 };
-constexpr int kPathMost = kPathGroups + 1;   // intervals of a path: one per group, and a sample by itself
+constexpr int kPathQuarter = 16;             // most intervals that a block starts over with in quarters
+constexpr int kPathMost = 4 * kPathQuarter;  // intervals of a pass (33 on the first one)
 struct PathBlock {
     int hit;              // a sample collides
     int n_list;           // intervals that the swept check left
@@ -319,9 +320,12 @@ struct PathBlock {
 
 // Works through the n intervals blk.item: the swept check (skipped for single
 // samples), then for the intervals that it leaves every sample if they are
-// few, else one of each (the first one when `ends`, else the middle one), and
-// with no hit among those the intervals go to defer(), a thread each. Stops
-// early once a sample hits or stop() says that the answer no longer matters.
+// few, else one of each (the first one when `ends`, else the middle one). With
+// no hit among those, half of them or fewer start over in quarters, `again` times
+// at most (an edge near something on a part of its way: 400 edges without self
+// check 273 -> 199 us among 128 boxes, where nothing is left after one more
+// pass), and else they go to defer(), a thread each. Stops early once a sample hits or stop() says that
+// the answer no longer matters.
 //
 // point(seg, i, a, b): DoF i of a segment's ends; sample j is a + (j / G)
 // (b - a), rounded as the edge kernels round it, and j = G + 1 is b itself
@@ -331,7 +335,7 @@ struct PathBlock {
 template <bool kEsdf, class Point, class Stop, class Defer>
 __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md, const SceneSmem& sc,
                                          const ps_scene_view& sv, const PathSmem& ps, float margin, bool self,
-                                         PathBlock& blk, int n, int G, bool ends, Point&& point, Stop&& stop,
+                                         PathBlock& blk, int n, int G, bool ends, int again, Point&& point, Stop&& stop,
                                          Defer&& defer) {
     constexpr int kSub = kPathSub;
     const int D = M.H->n_dof;
@@ -342,76 +346,90 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
     volatile int* hit_flag = &blk.hit;
     LaneStats st;
     st.zero();
-    if (threadIdx.x == 0) blk.n_list = blk.n_samples = 0;
-    __syncthreads();
-    // ---- swept check, a group per interval ----
-    for (int k0 = 0; k0 < n; k0 += kPathGroups) {
-        const PathItem it = blk.item[min(k0 + slot, n - 1)];   // a group past the end repeats the last one
-        const bool single = it.lo == it.hi;
-        unsigned bits = (unsigned)it.what;
-        if (!__all_sync(kGrpFull, single)) {   // uniform
-            const int lo = min(it.lo, G), hi = min(it.hi, G);
-            const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
-                        th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
-            bool ok = !single;   // a single sample is checked itself
-            __syncwarp();
-            for (int i = 0; i < D; ++i) {
-                float a, b;
-                point(it.seg, i, a, b);
-                ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
-                if ((i & (kSub - 1)) == u) {
-                    qc[i] = fmaf(tm, b - a, a);
-                    dq[i] = th * (b - a);
+    for (;; --again) {
+        if (threadIdx.x == 0) blk.n_list = blk.n_samples = 0;
+        __syncthreads();
+        // ---- swept check, a group per interval ----
+        for (int k0 = 0; k0 < n; k0 += kPathGroups) {
+            const PathItem it = blk.item[min(k0 + slot, n - 1)];   // a group past the end repeats the last one
+            const bool single = it.lo == it.hi;
+            unsigned bits = (unsigned)it.what;
+            if (!__all_sync(kGrpFull, single)) {   // uniform
+                const int lo = min(it.lo, G), hi = min(it.hi, G);
+                const float tm = __fdiv_rn((float)lo + (float)hi, 2.0f * (float)G),
+                            th = __fdiv_rn((float)hi - (float)lo, 2.0f * (float)G);
+                bool ok = !single;   // a single sample is checked itself
+                __syncwarp();
+                for (int i = 0; i < D; ++i) {
+                    float a, b;
+                    point(it.seg, i, a, b);
+                    ok = ok && fabsf(a) <= kSweepMaxQ && fabsf(b) <= kSweepMaxQ;
+                    if ((i & (kSub - 1)) == u) {
+                        qc[i] = fmaf(tm, b - a, a);
+                        dq[i] = th * (b - a);
+                    }
                 }
+                __syncwarp();
+                bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
+            }
+            if (u == 0 && k0 + slot < n && bits) {   // in any order
+                const int k = atomicAdd(&blk.n_list, 1);
+                blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
+                atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
+            }
+        }
+        __syncthreads();
+        const int nl = blk.n_list;
+        const bool all = blk.n_samples <= 2 * kPathGroups;
+        int per = nl > 0 ? 1 : 0;
+        if (all)
+            for (int k = 0; k < nl; ++k) per = max(per, blk.list[k].hi - blk.list[k].lo + 1);
+        // ---- samples: task t is sample t / nl of interval t % nl, so that every
+        //      interval is looked at before any is finished ----
+        const int total = per * nl;
+        for (int t0 = first; t0 < total; t0 += kPathGroups) {
+            if (__any_sync(kGrpFull, *hit_flag != 0 || stop())) break;   // one decision for the warp
+            const int t = min(t0 + (slot - first), total - 1);
+            const PathItem x = blk.list[t % nl];
+            const int s = t / nl, cnt = x.hi - x.lo + 1;
+            const bool on = t0 + (slot - first) < total && s < cnt;
+            if (!__any_sync(kGrpFull, on)) continue;   // uniform
+            const int j = x.lo + (ends ? s : (s + cnt / 2) % cnt);   // from the middle on
+            const float tj = __fdiv_rn((float)j, (float)G);
+            __syncwarp();
+            for (int i = u; i < D; i += kSub) {
+                float a, b;
+                point(x.seg, i, a, b);
+                qc[i] = j > G ? b : (ends && j == 0 ? a : __fmaf_rn(tj, __fadd_rn(b, -a), a));
             }
             __syncwarp();
-            bits &= path_sweep<kEsdf>(M, md, sc, ps.obs, qc, dq, margin, ok, self, ps.self, slot);
+            bool hit = false;
+            if (__any_sync(kGrpFull, on && (x.what & 1))) {   // uniform
+                bool h;
+                float clr;
+                group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
+                hit = on && (x.what & 1) && h;
+            }
+            if (self && on && (x.what & 2) && !hit)   // uniform over the group
+                hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
+            if (hit && u == 0) *hit_flag = 1;
+            __syncwarp();
         }
-        if (u == 0 && k0 + slot < n && bits) {   // in any order
-            const int k = atomicAdd(&blk.n_list, 1);
-            blk.list[k] = PathItem{it.seg, it.lo, it.hi, (int)bits};
-            atomicAdd(&blk.n_samples, min(it.hi - it.lo + 1, 1 << 20));
+        if (__syncthreads_or(*hit_flag != 0 || stop()) || all) break;   // one decision for the block
+        const bool quarter = again > 0 && nl <= kPathQuarter;
+        if (threadIdx.x < nl) {
+            const PathItem x = blk.list[threadIdx.x];
+            const int cnt = x.hi - x.lo + 1;
+            if (!quarter && cnt > 1) defer(x);
+            for (int k = 0; k < 4 && quarter; ++k) {   // an empty quarter, and a sample by itself, which is done: nothing
+                const int lo = x.lo + (int)((long long)cnt * k / 4), hi = x.lo + (int)((long long)cnt * (k + 1) / 4) - 1;
+                blk.item[4 * threadIdx.x + k] = PathItem{x.seg, lo, max(lo, hi), lo <= hi && cnt > 1 ? x.what : 0};
+            }
         }
+        if (!quarter) break;
+        n = 4 * nl;
+        __syncthreads();
     }
-    __syncthreads();
-    const int nl = blk.n_list;
-    const bool all = blk.n_samples <= 2 * kPathGroups;
-    int per = nl > 0 ? 1 : 0;
-    if (all)
-        for (int k = 0; k < nl; ++k) per = max(per, blk.list[k].hi - blk.list[k].lo + 1);
-    // ---- samples: task t is sample t / nl of interval t % nl, so that every
-    //      interval is looked at before any is finished ----
-    const int total = per * nl;
-    for (int t0 = first; t0 < total; t0 += kPathGroups) {
-        if (__any_sync(kGrpFull, *hit_flag != 0 || stop())) break;   // one decision for the warp
-        const int t = min(t0 + (slot - first), total - 1);
-        const PathItem x = blk.list[t % nl];
-        const int s = t / nl, cnt = x.hi - x.lo + 1;
-        const bool on = t0 + (slot - first) < total && s < cnt;
-        if (!__any_sync(kGrpFull, on)) continue;   // uniform
-        const int j = x.lo + (ends ? s : (s + cnt / 2) % cnt);   // from the middle on
-        const float tj = __fdiv_rn((float)j, (float)G);
-        __syncwarp();
-        for (int i = u; i < D; i += kSub) {
-            float a, b;
-            point(x.seg, i, a, b);
-            qc[i] = j > G ? b : (ends && j == 0 ? a : __fmaf_rn(tj, __fadd_rn(b, -a), a));
-        }
-        __syncwarp();
-        bool hit = false;
-        if (__any_sync(kGrpFull, on && (x.what & 1))) {   // uniform
-            bool h;
-            float clr;
-            group_verdict<kSub, false, kEsdf, false>(M, sc, sv, ps.obs, qc, margin, false, h, clr, st);
-            hit = on && (x.what & 1) && h;
-        }
-        if (self && on && (x.what & 2) && !hit)   // uniform over the group
-            hit = group_self_hit<kPathGroups>(M, md, qc, ps.self, slot, u, st);
-        if (hit && u == 0) *hit_flag = 1;
-        __syncwarp();
-    }
-    if (!__syncthreads_or(*hit_flag != 0 || stop()) && !all && threadIdx.x < nl && blk.list[threadIdx.x].lo < blk.list[threadIdx.x].hi)
-        defer(blk.list[threadIdx.x]);   // one decision for the block
     __syncthreads();
 }
 
@@ -434,9 +452,10 @@ __device__ __forceinline__ unsigned rest_bits(int lo, int hi, int G) {
     return (0xffffffffu >> (31 - (min(hi, G) - 1) / unit)) & (0xffffffffu << ((max(lo, 1) - 1) / unit));
 }
 
-// Marks an interval's units in blk.left.
+// Marks an interval's units in blk.left (the start configuration, sample 0,
+// goes with the last one: rest_run checks it behind sample G).
 __device__ __forceinline__ void path_left(PathBlock& blk, const PathItem& x, int G) {
-    const unsigned bits = rest_bits(x.lo, x.hi, G);
+    const unsigned bits = rest_bits(x.lo, x.hi, G) | (x.lo == 0 ? rest_bits(G, G, G) : 0u);
     if (x.what & 1) atomicOr(&blk.left[0], bits);
     if (x.what & 2) atomicOr(&blk.left[1], bits);
 }
