@@ -289,13 +289,12 @@ __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md,
     int G = 1;   // n_sub, capped so that the cast stays defined
     if (check_step > 0.0f && max_seg > check_step)
         G = (int)fminf(ceilf(__fdiv_rn(max_seg, check_step)), 1048576.0f);
-    // the slice's segments, the waypoint and samples 1 .. G, and after the last one its end by itself
+    // the slice's segments, the waypoint and samples 1 .. G, and on the last one its end
     const int seg0 = blockIdx.x * kPathGroups, n = min(kPathGroups, T - 1 - seg0), x = threadIdx.x;
     const bool last = seg0 + n == T - 1;
-    if (x < n) blk.item[x] = PathItem{seg0 + x, 0, G, self ? 3 : 1};
-    if (x == n && last) blk.item[x] = PathItem{T - 2, G + 1, G + 1, self ? 3 : 1};
+    if (x < n) blk.item[x] = PathItem{seg0 + x, 0, last && x == n - 1 ? G + 1 : G, self ? 3 : 1};
     path_run<kEsdf>(
-        M, md, sc, sv, ps, margin, self, blk, n + (last ? 1 : 0), G, true, 0,
+        M, md, sc, sv, ps, margin, self, blk, n, G, true, 0,
         [&](int sg, int i, float& a, float& b) {
             a = th[sg * D + i];
             b = th[(sg + 1) * D + i];

@@ -324,8 +324,8 @@ struct PathBlock {
 // no hit among those, half of them or fewer start over in quarters, `again` times
 // at most (an edge near something on a part of its way: 400 edges without self
 // check 273 -> 199 us among 128 boxes, where nothing is left after one more
-// pass), and else they go to defer(), a thread each. Stops early once a sample hits or stop() says that
-// the answer no longer matters.
+// pass), and else they go to defer(), a thread each. Stops early once a sample
+// hits or stop() says that the answer no longer matters.
 //
 // point(seg, i, a, b): DoF i of a segment's ends; sample j is a + (j / G)
 // (b - a), rounded as the edge kernels round it, and j = G + 1 is b itself
@@ -381,9 +381,10 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
         __syncthreads();
         const int nl = blk.n_list;
         const bool all = blk.n_samples <= 2 * kPathGroups;
-        int per = nl > 0 ? 1 : 0;
-        if (all)
-            for (int k = 0; k < nl; ++k) per = max(per, blk.list[k].hi - blk.list[k].lo + 1);
+        // samples of an interval that are checked now: all, or one and sample G + 1 (defer() takes no more than G)
+        auto count = [&](const PathItem& x) { return all ? x.hi - x.lo + 1 : (x.lo <= G && x.hi > G ? 2 : 1); };
+        int per = 0;
+        for (int k = 0; k < nl; ++k) per = max(per, count(blk.list[k]));
         // ---- samples: task t is sample t / nl of interval t % nl, so that every
         //      interval is looked at before any is finished ----
         const int total = per * nl;
@@ -392,9 +393,9 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
             const int t = min(t0 + (slot - first), total - 1);
             const PathItem x = blk.list[t % nl];
             const int s = t / nl, cnt = x.hi - x.lo + 1;
-            const bool on = t0 + (slot - first) < total && s < cnt;
+            const bool on = t0 + (slot - first) < total && s < count(x);
             if (!__any_sync(kGrpFull, on)) continue;   // uniform
-            const int j = x.lo + (ends ? s : (s + cnt / 2) % cnt);   // from the middle on
+            const int j = s == 1 && !all ? x.hi : x.lo + (ends ? s : (s + cnt / 2) % cnt);   // from the middle on
             const float tj = __fdiv_rn((float)j, (float)G);
             __syncwarp();
             for (int i = u; i < D; i += kSub) {
@@ -418,7 +419,8 @@ __device__ __forceinline__ void path_run(const ModelSmem& M, const ModelDev& md,
         if (__syncthreads_or(*hit_flag != 0 || stop()) || all) break;   // one decision for the block
         const bool quarter = again > 0 && nl <= kPathQuarter;
         if (threadIdx.x < nl) {
-            const PathItem x = blk.list[threadIdx.x];
+            PathItem x = blk.list[threadIdx.x];
+            x.hi = max(min(x.hi, G), x.lo);
             const int cnt = x.hi - x.lo + 1;
             if (!quarter && cnt > 1) defer(x);
             for (int k = 0; k < 4 && quarter; ++k) {   // an empty quarter, and a sample by itself, which is done: nothing

@@ -1,5 +1,5 @@
-"""A waypoint is checked whatever its neighbours hold: seeds whose second
-waypoint is not finite, against the separate waypoint and segment checks
+"""A waypoint is checked whatever its neighbours hold: seeds whose second or
+last but one waypoint is not finite, against the separate waypoint and segment checks
 (all-ones allowed-collision masks select those)."""
 import numpy as np
 import pytest
@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("value", [np.nan, np.inf])
 @pytest.mark.parametrize("T", [3, 40])
-def test_start_beside_a_bad_waypoint(golden, value, T):
+@pytest.mark.parametrize("at", [0, -1])
+def test_end_beside_a_bad_waypoint(golden, value, T, at):
     import torch
 
     from prismplan_b200 import api
@@ -28,8 +29,8 @@ def test_start_beside_a_bad_waypoint(golden, value, T):
     q = workloads.uniform_configs(rng, asset, 4000)
     hit = api.check_configs(b, plain, torch.from_numpy(q).cuda())[0].cpu().numpy() == 1
     theta = np.repeat(q[~hit][:4, None], T, 1)
-    theta[:2, 0] = q[hit][:2]          # two requests start in collision
-    theta[[0, 2], 1, 0] = value        # of each kind one with a bad second waypoint
+    theta[:2, at] = q[hit][:2]                            # two requests start (or end) in collision
+    theta[[0, 2], 1 if at == 0 else T - 2, 0] = value     # of each kind one with a bad waypoint beside it
     s = api.ChompSettings(num_timesteps=T, num_iterations=1, check_self=False, time_limit_ms=0.0)
     r, m = (api.chomp_optimize(b, scene, torch.from_numpy(theta).cuda(), s) for scene in (plain, masked))
     assert torch.equal(r.solved, m.solved)
