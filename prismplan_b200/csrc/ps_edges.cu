@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md
         if (x < n) blk.item[x] = PathItem{0, x == 0 && start && !apart ? 0 : x * m + 1, x == n - 1 ? G : (x + 1) * m, self ? 3 : 1};
         if (x == n && apart) blk.item[x] = PathItem{0, 0, 0, self ? 3 : 1};
         path_run<kEsdf>(
-            M, md, sc, sv, ps, P.collision_margin, self, blk, n + (apart ? 1 : 0), G, false, 1,
+            M, md, sc, sv, ps, P.collision_margin, self, blk, n + (apart ? 1 : 0), G, false, self ? 0 : 1,
             [&](int, int i, float& ai, float& bi) {
                 ai = __ldg(a + i);
                 bi = __ldg(b + i);
