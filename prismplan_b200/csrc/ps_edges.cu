@@ -107,9 +107,9 @@ EdgeBufs carve_workspace(void* ws, int n_edges) {
 // clr[k] (self) are left; done[e] says that edge e of the list collides.
 //
 // Bound by latency: 4-lane groups walk one chain of joints each. 1009 edges of
-// 1 to 300 samples with self check among 64 boxes: 106 us a block each and 31
-// us for the list (a call 163 us when a block finished its edge, 127 now); 27
-// edges of 16 samples 21 us.
+// 1 to 300 samples with self check among 64 boxes: 104 us a block each, the
+// list 50 us after them (a call 174 us when a block finished its edge, 158
+// now; over six scenes 167 and 142); 27 edges of 16 samples 20 us.
 // ---------------------------------------------------------------------------
 template <bool kEsdf>
 __global__ void __launch_bounds__(kPathThreads, 4) edges_path_kernel(ModelDev md, ps_scene_view sv, ps_edge_params P,
@@ -256,7 +256,7 @@ namespace {
 // samples 1009 edges 118 / 91 and 45 / 52, 2048 edges 48 / 89. With an ESDF
 // layer in reach 64 edges 195 / 166 and 474 / 217. What costs most here are
 // edges that no interval is clear of, at a box's side (the list's samples come
-// on top of the swept check): 39 / 43 for one of 600 samples, 72 / 84 for 512.
+// on top of the swept check): 512 of 600 samples 72 / 76, 256 of 5000 167 / 177.
 bool path_edges(const ps_model* m, const ps_scene_view* scene, const ps_edge_params* P, int mode, int n_edges, int few) {
     if (mode == 0 || !m->rigid || g_stats || P->time_budget_ms > 0.0f) return false;   // (the counters live in the queue path)
     if (P->probe || P->queue_blocks_per_sm || P->grab) return false;   // the caller asks for a shape of the queue

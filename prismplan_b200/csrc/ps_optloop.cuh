@@ -238,9 +238,9 @@ __global__ void opt_segments_kernel(const float* __restrict__ theta, int T, int 
 //
 // Those checks took eight launches (scene and self check of the waypoints,
 // segments, header, preparation, two queue passes, self pass, finalize) and
-// 141 us of a 256-request CHOMP iteration; this kernel takes 42 us,
-// opt_refine_kernel 29 us and opt_rest_kernel 5 us. With the segments' samples
-// finished in their own blocks refining took 36 us there, and by an ESDF layer
+// 141 us of a 256-request CHOMP iteration; this kernel takes 40 us,
+// opt_refine_kernel 21 us and opt_rest_kernel 4 us. With the segments' samples
+// finished in their own blocks refining took 28 us there, and by an ESDF layer
 // 510 us an iteration (64 requests of 200 waypoints; now 144 us on the list).
 template <bool kEsdf>
 __global__ void __launch_bounds__(kPathThreads, 4) opt_check_kernel(ModelDev md, ps_scene_view sv,
